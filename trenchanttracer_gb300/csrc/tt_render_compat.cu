@@ -21,6 +21,7 @@
 #include "tt_device.h"
 #include "tt_refmath.cuh"
 #include "tt_reorder.h"
+#include "tt_wide.cuh"
 
 namespace tt {
 
@@ -323,7 +324,8 @@ __device__ V3 radiance(const CompatArgs &a, curandState *rs, RRay ray, uint32_t 
     for (int bounce = 0; bounce < 10; bounce++) {
         const float4 r0 = make_float4(ray.o.x, ray.o.y, ray.o.z, ray.d.x);
         const float4 r1 = make_float4(ray.d.y, ray.d.z, ray.tmin, ray.tmax);
-        const TraceResult tr = traverse<true>(a.bvh, r0, r1, err);
+        WideStackOf<0, 1, true> stack;
+        const TraceResult tr = traverse_wide<true>(stack, a.bvh, r0, r1, err);
         RHit hit;
         hit.distance = tr.t;
         hit.index = -1;

@@ -1,29 +1,27 @@
 // Ray-cast kernels (closest-hit / any-hit) and the device half of the compact BVH.
 //
-// All kernels are persistent grids sized to fill every SM of the GB300 with resident blocks.
+// All kernels are persistent grids sized to fill every SM of the GB300 with resident blocks. They
+// traverse the four-wide form of the tree (tt_wide.cuh), each warp as a small queue of its own
+// (trace_queue), except where noted.
 // Kernel shapes (tt_dbvh_set_variant; tt_dbvh_autotune times them and keeps the fastest):
-//   TT_VARIANT_WARP       each warp claims 32 consecutive rays (lane i traces ray base+i, as a
-//                         one-ray-per-thread launch would) and traces them with the per-ray
-//                         semantics; the whole traversal stack is in local memory.
+//   TT_VARIANT_WARP       the whole traversal stack is in local memory.
 //   TT_VARIANT_WARP_SH16  as WARP, the lowest 16 stack entries in shared memory (the rest, rarely
 //   TT_VARIANT_WARP_SH32  touched, in local memory), so stack traffic does not evict BVH nodes
 //                         from L1; SH32 keeps 32 entries.
-//   TT_VARIANT_DYNAMIC    every lane claims a new ray (one warp-aggregated atomic per claim
-//                         round: ballot + popc + one atomicAdd) as soon as it finishes one.
-//   TT_VARIANT_WARP_VOTE  as WARP, but a lane that has postponed a leaf keeps visiting inner
-//                         nodes until a warp vote says every active lane holds one, as the
-//                         reference kernel does (IntersectKernel.cuh:180-203). Which lanes are
+//   TT_VARIANT_DYNAMIC    the two-wide tree; every lane claims a new ray (one warp-aggregated atomic
+//                         per claim round: ballot + popc + one atomicAdd) as soon as it finishes one.
+//   TT_VARIANT_WARP_VOTE  the two-wide tree, 32 rays per warp; a lane that has postponed a leaf keeps
+//                         visiting inner nodes until a warp vote says every active lane holds one, as
+//                         the reference kernel does (IntersectKernel.cuh:180-203). Which lanes are
 //                         active at the vote depends on how the warp re-converges, so in float
 //                         corner cases (a leaf box whose entry rounds above a nearly equal hit
 //                         distance) the result can depend on the other rays of the warp.
-//   TT_VARIANT_SORTED     WARP_SH16 over the rays in the order of a counting sort by origin
-//                         cell and direction cell (tt_reorder.cu), or in their own order when a
-//                         sample finds them coherent; each hit still goes to its own ray's slot.
-//                         Compiled for 10 resident blocks per SM (48 registers, 8 bytes spilled;
-//                         without that bound it takes 61 registers and 8 blocks fit).
-//   TT_VARIANT_SH16_OCC,  WARP_SH16 and SORTED compiled for 12 resident blocks per SM (40
-//   TT_VARIANT_SORTED_OCC registers and a few spilled values), trading spills for more warps to
-//                         hide the node-fetch latency.
+//   TT_VARIANT_SORTED     with 8 shared stack entries, over the rays in the order of a counting sort
+//                         by origin cell and direction cell (tt_reorder.cu), or in their own order
+//                         when a sample finds them coherent; each hit still goes to its own ray's
+//                         slot.
+//   TT_VARIANT_SH16_OCC,  WARP_SH16 and SORTED (16 entries) compiled for 12 resident blocks per SM (40
+//   TT_VARIANT_SORTED_OCC registers and spilled values), trading spills for more warps.
 // All but WARP_VOTE return the per-ray result of the reference's algorithm, bit for bit.
 #include <cuda_runtime.h>
 
@@ -36,7 +34,7 @@
 
 #include "tt_internal.h"
 #include "tt_reorder.h"
-#include "tt_traverse.cuh"
+#include "tt_wide.cuh"
 
 namespace tt {
 
@@ -50,26 +48,33 @@ enum TraceVariant : int {
     VARIANT_SORTED = 5,
     VARIANT_SH16_OCC = 6,
     VARIANT_SORTED_OCC = 7,
-    NUM_VARIANTS = 8
+    NUM_VARIANTS = 8,
+    VARIANT_TWO_WIDE = 8,  // internal: the two-wide tree, for trees without a four-wide form
+    kNumKernels = 9
 };
+constexpr int64_t kMaxLaunchRays = (int64_t)1 << 30;
 constexpr int kOccBlocks = 12;  // resident blocks per SM the *_OCC variants are compiled for
-// resident blocks per SM the default (ordered) variant is compiled for: 48 registers, 8 bytes
-// spilled; against 8 blocks at 61 registers it traces the terrain sets 4 % faster (9: 2 %)
-constexpr int kSortedBlocks = 10;
+// resident blocks per SM and shared stack entries of the default (ordered) variant: 64 registers, no
+// spills. 4M camera rays / 4M bounces on the 2,097,152-triangle terrain: 0.49 / 0.86 ms; 7 blocks
+// 0.51 / 0.89, 9 blocks 0.55 / 0.92, 10 blocks 0.55 / 0.94 (kWideInner 16); 4 entries 0.51 / 0.90, 12
+// entries 0.49 / 0.86
+constexpr int kSortedBlocks = 8;
+constexpr int kSortedStack = 8;
 // the node array's top levels laid out first at upload (bytes), and the default L2 persisting
 // window of the trace launches over them
 constexpr size_t kL2TopRegion = 16ull << 20;
 constexpr size_t kL2WindowDefault = 8ull << 20;
 
 struct DeviceBVH {
-    BvhView view;
+    BvhView view{};
     void *base = nullptr;          // one allocation holding all five arrays
+    void *wide = nullptr;          // the four-wide form: nodes, then triangle pairs
     size_t bytes = 0;
     uint32_t num_nodes = 0, num_verts = 0;
     unsigned long long *scratch = nullptr;  // [0] work counter, [1] error word (low 32 bits)
     int device = 0;
     int num_sms = 0;
-    int blocks_per_sm[NUM_VARIANTS] = {1, 1, 1, 1, 1, 1, 1, 1};
+    int blocks_per_sm[kNumKernels] = {1, 1, 1, 1, 1, 1, 1, 1, 1};
     int variant = VARIANT_SORTED;
     // L2 access-policy window over the node array for the trace launches (0 bytes: none), set up
     // at the first trace launch (the persisting set-aside shrinks the L2 left to other work, so a
@@ -111,8 +116,8 @@ struct TraceArgs {
     const unsigned long long *order_state;
 };
 
-template <bool kExt>
-__device__ __forceinline__ void store_hit(const TraceArgs &a, void *hits, int64_t i, const TravState &s) {
+template <bool kExt, class Hit>
+__device__ __forceinline__ void store_hit(const TraceArgs &a, void *hits, int64_t i, const Hit &s) {
     int id = -1;
     if (s.addr >= 0) id = __ldg(a.bvh.tri_idx + s.addr);
     if (!kExt) {
@@ -134,16 +139,43 @@ __device__ __forceinline__ void store_hit(const TraceArgs &a, void *hits, int64_
     }
 }
 
-// Warp-batched: each warp claims 32 consecutive rays (kPerm: 32 consecutive slots of the sorted
-// ray copy, when the ordering built one). kSh stack entries live in shared memory.
-template <bool kClosest, bool kExt, bool kSpec, int kSh, bool kPerm = false, int kMinBlocks = 1>
-__global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_warp_kernel(TraceArgs a) {
+// The four-wide tree (kPerm: over the slots of the sorted ray copy, when the ordering built one). kSh
+// stack entries live in shared memory.
+template <bool kClosest, bool kExt, int kSh, bool kPerm, int kMinBlocks>
+__global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(TraceArgs a) {
+    __shared__ typename WideEntry<kClosest>::type sh_stack[(kSh > 0 ? kSh : 1) * kTraceBlock];
+    const int lane = threadIdx.x & 31;
+    uint32_t err = 0;
+    WideStackOf<kSh, kTraceBlock, kClosest> stack;
+    stack.sh = sh_stack + threadIdx.x;
+    const bool use_perm = kPerm && order_built(a.order_state);
+    // sorted: rays and hits by sorted slot (contiguous); else by ray
+    const float4 *rays = use_perm ? a.sorted : a.rays;
+    void *hits = use_perm ? a.sorted_hits : a.hits;
+    trace_queue<kClosest, kWideInner>(
+        stack, a.bvh, (unsigned)a.n, err,
+        [&](int count) {
+            unsigned b = 0;
+            if (lane == 0) b = (unsigned)atomicAdd(a.counter, (unsigned long long)count);
+            return __shfl_sync(0xffffffffu, b, 0);
+        },
+        [&](unsigned i, float4 &r0, float4 &r1) {
+            r0 = __ldg(rays + 2 * (size_t)i);
+            r1 = __ldg(rays + 2 * (size_t)i + 1);
+        },
+        [&](unsigned, unsigned i, const TraceResult &tr) { store_hit<kExt>(a, hits, i, tr); });
+    if (err) atomicOr(a.err, err);
+}
+
+// The two-wide tree: each warp claims 32 consecutive rays. kSpec: with the reference's warp vote.
+template <bool kClosest, bool kExt, bool kSpec, int kSh, bool kPerm = false>
+__global__ void __launch_bounds__(kTraceBlock) trace_warp_kernel(TraceArgs a) {
     __shared__ int sh_stack[(kSh > 0 ? kSh : 1) * kTraceBlock];
     const int lane = threadIdx.x & 31;
     uint32_t err = 0;
     TravStack<kSh, kTraceBlock> stack;
     stack.sh = sh_stack + threadIdx.x;
-    const bool use_perm = kPerm && order_built(a.order_state);
+    const bool use_perm = kPerm && a.order_state && order_built(a.order_state);
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(a.counter, 32ull);
@@ -213,13 +245,14 @@ __global__ void __launch_bounds__(kTraceBlock) trace_dynamic_kernel(TraceArgs a)
 template <bool kClosest, bool kExt>
 static const void *kernel_for(int variant) {
     switch (variant) {
-        case VARIANT_WARP: return (const void *)trace_warp_kernel<kClosest, kExt, false, 0>;
-        case VARIANT_WARP_SH16: return (const void *)trace_warp_kernel<kClosest, kExt, false, 16>;
-        case VARIANT_WARP_SH32: return (const void *)trace_warp_kernel<kClosest, kExt, false, 32>;
+        case VARIANT_WARP: return (const void *)trace_wide_kernel<kClosest, kExt, 0, false, 1>;
+        case VARIANT_WARP_SH16: return (const void *)trace_wide_kernel<kClosest, kExt, 16, false, 1>;
+        case VARIANT_WARP_SH32: return (const void *)trace_wide_kernel<kClosest, kExt, 32, false, 1>;
         case VARIANT_DYNAMIC: return (const void *)trace_dynamic_kernel<kClosest, kExt, 16>;
-        case VARIANT_SORTED: return (const void *)trace_warp_kernel<kClosest, kExt, false, 16, true, kSortedBlocks>;
-        case VARIANT_SH16_OCC: return (const void *)trace_warp_kernel<kClosest, kExt, false, 16, false, kOccBlocks>;
-        case VARIANT_SORTED_OCC: return (const void *)trace_warp_kernel<kClosest, kExt, false, 16, true, kOccBlocks>;
+        case VARIANT_SORTED: return (const void *)trace_wide_kernel<kClosest, kExt, kSortedStack, true, kSortedBlocks>;
+        case VARIANT_SH16_OCC: return (const void *)trace_wide_kernel<kClosest, kExt, 16, false, kOccBlocks>;
+        case VARIANT_SORTED_OCC: return (const void *)trace_wide_kernel<kClosest, kExt, 16, true, kOccBlocks>;
+        case VARIANT_TWO_WIDE: return (const void *)trace_warp_kernel<kClosest, kExt, false, 16, true>;
         default: return (const void *)trace_warp_kernel<kClosest, kExt, true, 0>;
     }
 }
@@ -234,58 +267,42 @@ static tt_status cuda_fail(cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return cuda_fail(e_, #call); \
     } while (0)
 
-// The device's node order: the top levels of the tree first (breadth first from the root, until
-// they fill top_bytes), then every other inner node in the file's depth-first order. Child order,
-// node contents and leaf addresses are unchanged, only inner-child addresses are renumbered, so a
-// traversal visits the same nodes and leaves in the same order and returns the same hits. The
-// L2 persisting window of the trace launches then covers a prefix of the array that is exactly
-// the tree's top levels (the file's depth-first order scatters them over the whole array).
-// Returns false, leaving `out` empty, for an array whose child addresses do not form a tree.
-static bool top_first_nodes(const std::vector<I4> &nodes, size_t top_bytes, std::vector<I4> &out, size_t &top_out) {
-    const size_t count = nodes.size() / 4;
-    out.clear();
-    top_out = 0;
-    if (count == 0 || nodes.size() % 4) return false;
-    std::vector<int64_t> new_index(count, -1), order;
-    order.reserve(count);
-    const size_t top_nodes = std::max<size_t>(1, top_bytes / 64);
-    // breadth first, level by level, while the placed nodes fit in top_bytes
-    new_index[0] = 0;
-    order.push_back(0);
-    for (size_t head = 0; head < order.size() && order.size() < top_nodes; head++) {
-        const I4 &c = nodes[4 * (size_t)order[head] + 3];
-        for (int32_t addr : {c.x, c.y}) {
-            if (addr < 0) continue;  // a leaf
-            if (addr % 4 || (size_t)addr / 4 >= count) return false;
-            const size_t k = (size_t)addr / 4;
-            if (new_index[k] >= 0) return false;  // not a tree
-            if (order.size() >= top_nodes) break;
-            new_index[k] = (int64_t)order.size();
-            order.push_back((int64_t)k);
-        }
+// The leaves' triangles as pairs (tt_wide.h), one leaf per thread.
+__global__ void __launch_bounds__(256) k_wide_pairs(const uint2 *leaves, uint32_t n, const float4 *verts, char *pairs) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 l = leaves[i];
+        wide_fill_pairs(verts, l.x, reinterpret_cast<float *>(pairs + (size_t)l.y * kWidePairBytes));
     }
-    top_out = 64 * order.size();
-    for (size_t k = 0; k < count; k++)
-        if (new_index[k] < 0) {
-            new_index[k] = (int64_t)order.size();
-            order.push_back((int64_t)k);
-        }
-    out.resize(nodes.size());
-    for (size_t j = 0; j < count; j++) {
-        const size_t k = (size_t)order[j];
-        for (int q = 0; q < 4; q++) out[4 * j + q] = nodes[4 * k + q];
-        I4 &c = out[4 * j + 3];
-        for (int32_t *addr : {&c.x, &c.y}) {
-            if (*addr < 0) continue;
-            if (*addr % 4 || (size_t)*addr / 4 >= count) {
-                out.clear();
-                top_out = 0;
-                return false;
-            }
-            *addr = (int32_t)(4 * new_index[(size_t)*addr / 4]);
-        }
+}
+
+// The four-wide form of the tree beside the compact arrays, which must already be on the device.
+static tt_status upload_wide(const CompactBVH &b, DeviceBVH &d) {
+    WideBVH w;
+    if (!build_wide(b, kL2TopRegion, w)) return TT_OK;
+    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t nb = 4 * w.nodes.size(), pb = kWidePairBytes * w.pairs, lb = 4 * w.leaves.size();
+    cudaError_t e = cudaMalloc(&d.wide, align(nb) + align(pb));
+    if (e != cudaSuccess) return fail(TT_ERR_OOM, std::string("cudaMalloc BVH: ") + cudaGetErrorString(e));
+    void *leaves = nullptr;
+    e = cudaMalloc(&leaves, lb);
+    if (e != cudaSuccess) return fail(TT_ERR_OOM, std::string("cudaMalloc BVH: ") + cudaGetErrorString(e));
+    char *nodes = static_cast<char *>(d.wide), *pairs = nodes + align(nb);
+    e = cudaMemcpy(nodes, w.nodes.data(), nb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(leaves, w.leaves.data(), lb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        const uint32_t n = (uint32_t)(w.leaves.size() / 2);
+        k_wide_pairs<<<std::min<uint32_t>((n + 255) / 256, 8u * (uint32_t)d.num_sms), 256>>>(
+            static_cast<const uint2 *>(leaves), n, d.view.verts, pairs);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     }
-    return true;
+    cudaFree(leaves);
+    if (e != cudaSuccess) return cuda_fail(e, "four-wide BVH");
+    d.view.wide_nodes = nodes;
+    d.view.wide_pairs = pairs;
+    d.view.wide_flags = w.flags;
+    d.l2_top_bytes = std::min(w.top_bytes, nb);
+    return TT_OK;
 }
 
 static tt_status upload(const CompactBVH &b, DeviceBVH &d) {
@@ -293,7 +310,7 @@ static tt_status upload(const CompactBVH &b, DeviceBVH &d) {
     TT_CUDA(cudaGetDevice(&dev));
     d.device = dev;
     TT_CUDA(cudaDeviceGetAttribute(&d.num_sms, cudaDevAttrMultiProcessorCount, dev));
-    for (int v = 0; v < NUM_VARIANTS; v++) {
+    for (int v = 0; v < kNumKernels; v++) {
         int bps = 0;
         TT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel_for<true, false>(v), kTraceBlock, 0));
         d.blocks_per_sm[v] = bps > 0 ? bps : 1;
@@ -306,17 +323,7 @@ static tt_status upload(const CompactBVH &b, DeviceBVH &d) {
     if (e != cudaSuccess) return fail(TT_ERR_OOM, std::string("cudaMalloc BVH: ") + cudaGetErrorString(e));
     char *p = static_cast<char *>(d.base);
     d.view.nodes = reinterpret_cast<const float4 *>(p);
-    {
-        std::vector<I4> reordered;
-        size_t top = 0;
-        if (top_first_nodes(b.nodes, kL2TopRegion, reordered, top)) {
-            TT_CUDA(cudaMemcpy(p, reordered.data(), nb, cudaMemcpyHostToDevice));
-            d.l2_top_bytes = top;
-        } else {
-            TT_CUDA(cudaMemcpy(p, b.nodes.data(), nb, cudaMemcpyHostToDevice));
-            d.l2_top_bytes = nb;  // file order: only the whole array is a window over the top levels
-        }
-    }
+    TT_CUDA(cudaMemcpy(p, b.nodes.data(), nb, cudaMemcpyHostToDevice));
     p += align(nb);
     d.view.verts = reinterpret_cast<const float4 *>(p);
     TT_CUDA(cudaMemcpy(p, b.vertices.data(), vb, cudaMemcpyHostToDevice));
@@ -348,11 +355,12 @@ static tt_status upload(const CompactBVH &b, DeviceBVH &d) {
     e = cudaMalloc(&d.scratch, 256);
     if (e != cudaSuccess) return fail(TT_ERR_OOM, std::string("cudaMalloc scratch: ") + cudaGetErrorString(e));
     TT_CUDA(cudaMemset(d.scratch, 0, 256));
-    return TT_OK;
+    return upload_wide(b, d);
 }
 
 static void release(DeviceBVH &d) {
     if (d.base) cudaFree(d.base);
+    if (d.wide) cudaFree(d.wide);
     if (d.scratch) cudaFree(d.scratch);
     if (d.d_stage) cudaFree(d.d_stage);
     for (int i = 0; i < 4; i++)
@@ -378,9 +386,9 @@ static cudaError_t launch_variant(const DeviceBVH &d, int variant, unsigned bloc
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    if (d.l2_window_bytes) {
+    if (d.l2_window_bytes && variant != VARIANT_TWO_WIDE && variant != VARIANT_WARP_VOTE && variant != VARIANT_DYNAMIC) {
         attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
-        attr[0].val.accessPolicyWindow.base_ptr = const_cast<float4 *>(d.view.nodes);
+        attr[0].val.accessPolicyWindow.base_ptr = const_cast<char *>(d.view.wide_nodes);
         attr[0].val.accessPolicyWindow.num_bytes = d.l2_window_bytes;
         attr[0].val.accessPolicyWindow.hitRatio = d.l2_hit_ratio;
         attr[0].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
@@ -400,7 +408,7 @@ static void setup_l2_window(DeviceBVH &d) {
     if (cudaDeviceGetAttribute(&max_persist, cudaDevAttrMaxPersistingL2CacheSize, d.device) == cudaSuccess &&
         cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, d.device) == cudaSuccess &&
         max_persist > 0 && max_window > 0) {
-        const size_t nb = std::min(std::min((size_t)16 * (size_t)d.num_nodes, d.l2_top_bytes), d.l2_window_want);
+        const size_t nb = std::min(d.l2_top_bytes, d.l2_window_want);
         size_t cur = 0;
         cudaDeviceGetLimit(&cur, cudaLimitPersistingL2CacheSize);
         const size_t want = std::min(nb, (size_t)max_persist);
@@ -420,6 +428,14 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     if (!d_rays || !d_hits) return fail(TT_ERR_INVALID, "null ray or hit buffer");
     if ((reinterpret_cast<uintptr_t>(d_rays) & 15) || (reinterpret_cast<uintptr_t>(d_hits) & 7))
         return fail(TT_ERR_INVALID, "ray buffer must be 16-byte aligned and hit buffer 8-byte aligned");
+    // the kernels count rays in 32 bits: a longer set is traced in parts, one after the other
+    for (; n > kMaxLaunchRays; n -= kMaxLaunchRays) {
+        const tt_status st =
+            launch_trace(d, d_rays, kMaxLaunchRays, d_hits, closest, ext, stream, counter_slot, unordered);
+        if (st != TT_OK) return st;
+        d_rays = static_cast<const char *>(d_rays) + 32 * kMaxLaunchRays;
+        d_hits = static_cast<char *>(d_hits) + (ext ? sizeof(tt_hit_ext) : sizeof(tt_hit)) * kMaxLaunchRays;
+    }
     if (!d.l2_setup) setup_l2_window(const_cast<DeviceBVH &>(d));
     TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
     TraceArgs a;
@@ -435,10 +451,12 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     OrderOut order{};
     int variant = d.variant;
     const bool sorted = variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC;
-    // slots are int; too few rays cannot pay for the ordering
-    if (sorted && (unordered || n >= ((int64_t)1 << 31) || n < kOrderMinRays))
+    // too few rays cannot pay for the ordering
+    if (sorted && (unordered || n < kOrderMinRays))
         variant = variant == VARIANT_SORTED_OCC ? VARIANT_SH16_OCC : VARIANT_WARP_SH16;
-    if (variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC) {
+    const bool order_rays = variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC;
+    if (!d.view.wide_nodes && variant != VARIANT_DYNAMIC && variant != VARIANT_WARP_VOTE) variant = VARIANT_TWO_WIDE;
+    if (order_rays) {
         // one scratch per work-counter slot, so the pipeline streams never share one
         const int k = counter_slot == 0 ? 0 : 1 + (counter_slot - kScratchPipe) % 3;
         const size_t need = reorder_scratch_bytes(n);
@@ -527,7 +545,7 @@ static tt_status noalloc_setup(NoAllocDevice &out) {
         TT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         // one launch size for closest and any hit: the kernels claim rays from a counter, so the
         // grid only needs to fill the SMs, and the closest-hit build has the larger register count
-        TT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel_for<true, false>(VARIANT_WARP_SH16),
+        TT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel_for<true, false>(VARIANT_TWO_WIDE),
                                                               kTraceBlock, 0));
         d.num_sms = sms;
         d.blocks_per_sm = bps > 0 ? bps : 1;
@@ -780,8 +798,8 @@ tt_status tt_trace_host_noalloc(const void *d_nodes, const void *d_vertices, con
     d.view.mat_idx = nullptr;
     d.scratch = reinterpret_cast<unsigned long long *>(nd.scratch);
     d.num_sms = nd.num_sms;
-    d.variant = VARIANT_WARP_SH16;
-    d.blocks_per_sm[VARIANT_WARP_SH16] = nd.blocks_per_sm;
+    d.variant = VARIANT_WARP_SH16;  // traced two-wide: the caller's arrays have no four-wide form
+    d.blocks_per_sm[VARIANT_TWO_WIDE] = nd.blocks_per_sm;
     d.l2_setup = true;  // no L2 window: the call changes no limit of the context
     cudaStream_t s = (cudaStream_t)stream;
     char *dr = reinterpret_cast<char *>(nd.scratch) + kNoAllocHeader;

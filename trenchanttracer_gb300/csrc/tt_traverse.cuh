@@ -44,6 +44,10 @@ struct BvhView {
     const float4 *__restrict__ norms;
     const int32_t *__restrict__ tri_idx;
     const uint32_t *__restrict__ mat_idx;
+    // the four-wide form (tt_wide.h); wide_nodes == nullptr: the tree has none
+    const char *__restrict__ wide_nodes;
+    const char *__restrict__ wide_pairs;
+    uint32_t wide_flags;
 };
 
 __device__ __forceinline__ float4 ldg4(const float4 *p) { return __ldg(p); }
