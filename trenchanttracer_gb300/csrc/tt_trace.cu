@@ -35,6 +35,7 @@
 #include "tt_internal.h"
 #include "tt_reorder.h"
 #include "tt_wide.cuh"
+#include "tt_wide_build.h"
 
 namespace tt {
 
@@ -267,44 +268,6 @@ static tt_status cuda_fail(cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return cuda_fail(e_, #call); \
     } while (0)
 
-// The leaves' triangles as pairs (tt_wide.h), one leaf per thread.
-__global__ void __launch_bounds__(256) k_wide_pairs(const uint2 *leaves, uint32_t n, const float4 *verts, char *pairs) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint2 l = leaves[i];
-        wide_fill_pairs(verts, l.x, reinterpret_cast<float *>(pairs + (size_t)l.y * kWidePairBytes));
-    }
-}
-
-// The four-wide form of the tree beside the compact arrays, which must already be on the device.
-static tt_status upload_wide(const CompactBVH &b, DeviceBVH &d) {
-    WideBVH w;
-    if (!build_wide(b, kL2TopRegion, w)) return TT_OK;
-    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t nb = 4 * w.nodes.size(), pb = kWidePairBytes * w.pairs, lb = 4 * w.leaves.size();
-    cudaError_t e = cudaMalloc(&d.wide, align(nb) + align(pb));
-    if (e != cudaSuccess) return fail(TT_ERR_OOM, std::string("cudaMalloc BVH: ") + cudaGetErrorString(e));
-    void *leaves = nullptr;
-    e = cudaMalloc(&leaves, lb);
-    if (e != cudaSuccess) return fail(TT_ERR_OOM, std::string("cudaMalloc BVH: ") + cudaGetErrorString(e));
-    char *nodes = static_cast<char *>(d.wide), *pairs = nodes + align(nb);
-    e = cudaMemcpy(nodes, w.nodes.data(), nb, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(leaves, w.leaves.data(), lb, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) {
-        const uint32_t n = (uint32_t)(w.leaves.size() / 2);
-        k_wide_pairs<<<std::min<uint32_t>((n + 255) / 256, 8u * (uint32_t)d.num_sms), 256>>>(
-            static_cast<const uint2 *>(leaves), n, d.view.verts, pairs);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    }
-    cudaFree(leaves);
-    if (e != cudaSuccess) return cuda_fail(e, "four-wide BVH");
-    d.view.wide_nodes = nodes;
-    d.view.wide_pairs = pairs;
-    d.view.wide_flags = w.flags;
-    d.l2_top_bytes = std::min(w.top_bytes, nb);
-    return TT_OK;
-}
-
 static tt_status upload(const CompactBVH &b, DeviceBVH &d) {
     int dev = 0;
     TT_CUDA(cudaGetDevice(&dev));
@@ -355,7 +318,14 @@ static tt_status upload(const CompactBVH &b, DeviceBVH &d) {
     e = cudaMalloc(&d.scratch, 256);
     if (e != cudaSuccess) return fail(TT_ERR_OOM, std::string("cudaMalloc scratch: ") + cudaGetErrorString(e));
     TT_CUDA(cudaMemset(d.scratch, 0, 256));
-    return upload_wide(b, d);
+    WideBVH w;
+    TT_CUDA(build_wide(d.view, d.num_nodes, d.num_verts, kL2TopRegion, d.num_sms, w));
+    d.wide = w.base;
+    d.view.wide_nodes = w.nodes;
+    d.view.wide_pairs = w.pairs;
+    d.view.wide_flags = w.flags;
+    d.l2_top_bytes = w.top_bytes;
+    return TT_OK;
 }
 
 static void release(DeviceBVH &d) {

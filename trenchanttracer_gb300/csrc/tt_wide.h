@@ -1,5 +1,5 @@
 // The four-wide form of the compact SBVH that the device traverses (tt_wide.cuh), made from the
-// reference's two-wide arrays at upload (tt_wide.cpp). Host and device code share the layout.
+// reference's two-wide arrays at upload (tt_wide_build.cu).
 //
 // Node: 224 bytes, seven 32-byte sectors. Four slots in two groups, (0, 1) for the left child of a
 // two-wide inner node A and (2, 3) for its right child. A group holds either A's child itself in
@@ -26,9 +26,7 @@
 // determinant is 0, so it is never accepted).
 #pragma once
 
-#include <cstddef>
 #include <cstdint>
-#include <vector>
 
 namespace tt {
 
@@ -48,20 +46,5 @@ constexpr uint32_t kWideNegZero = 1u;  // some box plane is -0.0
 constexpr float kWideCoordMax = 68719476736.0f;   // 2^36: |vertex|, |box plane|, |ray origin|
 constexpr float kWideDirMax = 1073741824.0f;      // 2^30: |ray direction component|
 constexpr float kWidePlaneMin = 7.703719777548943e-34f;  // 2^-110: |box plane| unless zero
-
-struct CompactBVH;
-
-struct WideBVH {
-    std::vector<uint32_t> nodes;  // kWideNodeBytes / 4 words per node, root first
-    std::vector<uint32_t> leaves; // per leaf: its float4 slot in the vertex array, its first pair
-    size_t pairs = 0;
-    size_t top_bytes = 0;         // the top levels laid out first, breadth first
-    uint32_t flags = 0;
-};
-
-// False when the tree must stay two-wide: not a tree, no inner node, a box or vertex outside the
-// bounds above, an inverted box, a child's box that sticks out of its parent's, or a stack need
-// above kWideStack.
-bool build_wide(const CompactBVH &b, size_t top_bytes, WideBVH &out);
 
 }  // namespace tt
