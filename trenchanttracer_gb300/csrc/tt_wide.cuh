@@ -102,9 +102,10 @@ __device__ __forceinline__ f32x2 neg2(f32x2 v) {
     unpack2(v, a, b);
     return pack2(-a, -b);
 }
-// a.y*b.z - a.z*b.y and a.x*b.x + a.y*b.y + a.z*b.z of two triangles, contracted as cross_c and dot_c
-__device__ __forceinline__ f32x2 cross2(f32x2 ay, f32x2 bz, f32x2 az, f32x2 by) {
-    return fma2(ay, bz, neg2(mul2(az, by)));
+// a.y*b.z - a.z*b.y and a.x*b.x + a.y*b.y + a.z*b.z of two triangles, contracted as cross_c and dot_c;
+// naz = -a.z (negating a factor negates the product)
+__device__ __forceinline__ f32x2 cross2(f32x2 ay, f32x2 bz, f32x2 naz, f32x2 by) {
+    return fma2(ay, bz, mul2(naz, by));
 }
 __device__ __forceinline__ f32x2 dot2(f32x2 ax, f32x2 ay, f32x2 az, f32x2 bx, f32x2 by, f32x2 bz) {
     return fma2(az, bz, fma2(ax, bx, mul2(ay, by)));
@@ -220,7 +221,7 @@ __device__ __noinline__ TraceResult traverse_two_wide(const BvhView &bvh, float4
     return traverse<kClosest>(bvh, r0, r1, err);
 }
 
-// One triangle of a pair whose cheap tests did not refuse it: the rest of trav_leaf_phase's test.
+// The rest of trav_leaf_phase's test, for a triangle whose cheap tests did not refuse it.
 __device__ __forceinline__ bool accept_triangle(float det, float un, float vn, float tn, float tmin, float tcur,
                                                 float &u, float &v, float &t) {
     const float inv_det = __frcp_rn(det);
@@ -228,13 +229,6 @@ __device__ __forceinline__ bool accept_triangle(float det, float un, float vn, f
     v = __fmul_rn(vn, inv_det);
     t = __fmul_rn(tn, inv_det);
     return !(u < 0.0f || u > 1.0f || v < 0.0f || __fadd_rn(u, v) > 1.0f) && tmin < t && t < tcur;
-}
-
-// Signs first: with det > 0 and un < -1e-37 det the quotient u rounds to a negative number, with
-// un > 1.00001 det it rounds above 1, and so for v and u + v; in between the division decides.
-__device__ __forceinline__ bool may_hit(float det, float un, float vn) {
-    const float tiny = __fmul_rn(det, -1e-37f), most = __fmul_rn(det, 1.00001f);
-    return det > 0.00001f && un >= tiny && vn >= tiny && __fadd_rn(un, vn) <= most;
 }
 
 // What a lane is about to do, besides visiting an inner node (reference < kWideMark) or a leaf
@@ -368,45 +362,54 @@ __device__ __forceinline__ void wide_node(WideState &s, Stack &stack, const BvhV
 template <bool kClosest>
 __device__ __forceinline__ void wide_leaf(WideState &s, const BvhView &bvh, float4 r0, float4 r1) {
     const f32x2 dx2 = pack2(r0.w, r0.w), dy2 = pack2(r1.x, r1.x), dz2 = pack2(r1.y, r1.y);
+    const f32x2 ndx2 = pack2(-r0.w, -r0.w), ndy2 = pack2(-r1.x, -r1.x), ndz2 = pack2(-r1.y, -r1.y);
     const f32x2 ox2 = pack2(r0.x, r0.x), oy2 = pack2(r0.y, r0.y), oz2 = pack2(r0.z, r0.z);
     const char *rec = bvh.wide_pairs + (uint64_t)(s.ref & kWideIndex) * kWidePairBytes;
     s.ref = kWidePop;
     for (;; rec += kWidePairBytes) {
         const Sector w0 = ldg_sector(rec), w1 = ldg_sector(rec + 32), w2 = ldg_sector(rec + 64);
         const f32x2 e1x = w0.d, e1y = w1.a, e1z = w1.b, e2x = w1.c, e2y = w1.d, e2z = w2.a;
-        const f32x2 tvx = add2(ox2, neg2(w0.a)), tvy = add2(oy2, neg2(w0.b)), tvz = add2(oz2, neg2(w0.c));
-        const f32x2 px = cross2(dy2, e2z, dz2, e2y);
-        const f32x2 py = cross2(dz2, e2x, dx2, e2z);
-        const f32x2 pz = cross2(dx2, e2y, dy2, e2x);
-        const f32x2 qx = cross2(tvy, e1z, tvz, e1y);
-        const f32x2 qy = cross2(tvz, e1x, tvx, e1z);
-        const f32x2 qz = cross2(tvx, e1y, tvy, e1x);
-        float det0, det1, un0, un1, vn0, vn1, tn0, tn1;
-        unpack2(dot2(e1x, e1y, e1z, px, py, pz), det0, det1);
-        unpack2(dot2(tvx, tvy, tvz, px, py, pz), un0, un1);
-        unpack2(dot2(dx2, dy2, dz2, qx, qy, qz), vn0, vn1);
-        unpack2(dot2(e2x, e2y, e2z, qx, qy, qz), tn0, tn1);
+        const f32x2 tvx = add2(ox2, w0.a), tvy = add2(oy2, w0.b), tvz = add2(oz2, w0.c);
+        const f32x2 px = cross2(dy2, e2z, ndz2, e2y);
+        const f32x2 py = cross2(dz2, e2x, ndx2, e2z);
+        const f32x2 pz = cross2(dx2, e2y, ndy2, e2x);
+        const f32x2 qx = cross2(tvy, e1z, neg2(tvz), e1y);
+        const f32x2 qy = cross2(tvz, e1x, neg2(tvx), e1z);
+        const f32x2 qz = cross2(tvx, e1y, neg2(tvy), e1x);
+        const f32x2 det = dot2(e1x, e1y, e1z, px, py, pz), un = dot2(tvx, tvy, tvz, px, py, pz);
+        const f32x2 vn = dot2(dx2, dy2, dz2, qx, qy, qz), tn = dot2(e2x, e2y, e2z, qx, qy, qz);
         const int slot = (int)(uint32_t)w2.b;
         const uint32_t flags = (uint32_t)(w2.b >> 32);
-        const bool m0 = may_hit(det0, un0, vn0), m1 = may_hit(det1, un1, vn1);
-        if (m0 || m1) {
-            float u, v, t;
-            if (m0 && accept_triangle(det0, un0, vn0, tn0, s.tmin, s.t, u, v, t)) {
+        // Signs first: with det > 0 and un < -1e-37 det the quotient u rounds to a negative number,
+        // and so for v, and with un + vn > 1.00001 det u or u + v rounds above 1; in between the
+        // division decides. (Most triangles end here; so does the padding of an odd leaf, det = 0.)
+        float det0, det1, un0, un1, vn0, vn1, lo0, lo1, hi0, hi1, sum0, sum1;
+        unpack2(det, det0, det1);
+        unpack2(un, un0, un1);
+        unpack2(vn, vn0, vn1);
+        unpack2(mul2(det, pack2(-1e-37f, -1e-37f)), lo0, lo1);
+        unpack2(mul2(det, pack2(1.00001f, 1.00001f)), hi0, hi1);
+        unpack2(add2(un, vn), sum0, sum1);
+        const bool m0 = det0 > 0.00001f && fminf(un0, vn0) >= lo0 && sum0 <= hi0;
+        const bool m1 = det1 > 0.00001f && fminf(un1, vn1) >= lo1 && sum1 <= hi1;
+        bool more = m0 || m1, first = m0;
+        while (more) {  // one pass unless both are left
+            float tn0, tn1, u, v, t;
+            unpack2(tn, tn0, tn1);
+            const bool hit = accept_triangle(first ? det0 : det1, first ? un0 : un1, first ? vn0 : vn1,
+                                             first ? tn0 : tn1, s.tmin, s.t, u, v, t);
+            if (hit) {
                 s.t = t;
                 s.u = u;
                 s.v = v;
-                s.addr = slot;
-                if (!kClosest) s.ref = kWideDone;
+                s.addr = slot + (first ? 0 : 3);
+                if (!kClosest) {
+                    s.ref = kWideDone;
+                    return;
+                }
             }
-            if (m1 && (kClosest || s.ref != kWideDone) &&
-                accept_triangle(det1, un1, vn1, tn1, s.tmin, s.t, u, v, t)) {
-                s.t = t;
-                s.u = u;
-                s.v = v;
-                s.addr = slot + 3;
-                if (!kClosest) s.ref = kWideDone;
-            }
-            if (!kClosest && s.ref == kWideDone) return;
+            more = first && m1;
+            first = false;
         }
         if (flags & kPairLast) return;
     }
@@ -463,6 +466,8 @@ __device__ __forceinline__ void trace_queue(Stack &stack, const BvhView &bvh, un
     s.ref = kWideIdle;
     unsigned slot = 0;
     bool more = true;  // the queue may have rays left
+    unsigned base = 0;
+    const unsigned warps = gridDim.x * blockDim.x / 32, few = min(n / warps, 3u);
     for (;;) {
         const unsigned inner = __ballot_sync(0xffffffffu, s.ref < kWideMark);
         if (__popc(inner) < kInner) {
@@ -482,12 +487,14 @@ __device__ __forceinline__ void trace_queue(Stack &stack, const BvhView &bvh, un
             }
             __syncwarp();
             if (more) {
+                // no more than the warp's share of what is left, but a few
                 const unsigned want = ~inner;
-                const unsigned base = claim(__popc(want));
-                more = base < n && n - base > (unsigned)__popc(want);
+                const unsigned count = min((unsigned)__popc(want), max((n - base) / warps, few) + 1u);
+                base = claim((int)count);
+                more = base < n && n - base > count;
                 if (s.ref == kWideIdle) {
                     const unsigned off = __popc(want & ((1u << (threadIdx.x & 31)) - 1u));
-                    if (base < n && off < n - base) {
+                    if (off < count && base < n && off < n - base) {
                         slot = base + off;
                         float4 r0, r1;
                         fetch(slot, r0, r1);
@@ -523,9 +530,9 @@ __device__ __forceinline__ void wide_fill_pairs(const float4 *verts, uint32_t sl
         for (int k = 0; k < 2; k++) {
             if (__float_as_int(head.x) == (int)0x80000000) break;  // terminator: an empty leaf or second
             const float4 v1 = verts[slot + 3 * k + 1], v2 = verts[slot + 3 * k + 2];
-            f[k] = head.x;
-            f[2 + k] = head.y;
-            f[4 + k] = head.z;
+            f[k] = -head.x;
+            f[2 + k] = -head.y;
+            f[4 + k] = -head.z;
             f[6 + k] = __fsub_rn(v1.x, head.x);
             f[8 + k] = __fsub_rn(v1.y, head.y);
             f[10 + k] = __fsub_rn(v1.z, head.z);

@@ -17,8 +17,8 @@
 // An empty slot has lo = +inf, hi = -inf (no ray passes it) and the reference kWideEmpty.
 //
 // Triangle pair: 96 bytes, two triangles of a leaf side by side for the packed two-lane float
-// instructions; v0 and the edges e1 = v1 - v0, e2 = v2 - v0 as the leaf test forms them:
-//   float v0x[2], v0y[2], v0z[2], e1x[2], e1y[2], e1z[2], e2x[2], e2y[2], e2z[2]
+// instructions; -v0 and the edges e1 = v1 - v0, e2 = v2 - v0 as the leaf test forms them:
+//   float nv0x[2], nv0y[2], nv0z[2], e1x[2], e1y[2], e1z[2], e2x[2], e2y[2], e2z[2]
 //   int32_t slot      float4 slot of the first triangle in the compact vertex array (second: + 3)
 //   uint32_t flags    kPairLast: the leaf ends here
 //   uint32_t spare[4]
