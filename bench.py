@@ -178,11 +178,11 @@ class Clocks:
 
 
 def trace_call_launches(dbvh) -> int:
-    """Kernels one DeviceBVH.intersect call launches: with the ray-ordered variants the ordering
-    probe, keys, scan and scatter, the trace and the hit gather (the ordering kernels return at
-    once when the probe finds the rays coherent, but they are still launched); otherwise the
+    """Kernels one DeviceBVH.intersect call of this workload's size launches: with the ray-ordered
+    variants the ordering probe, keys, scan and scatter and the trace (the ordering kernels return
+    at once when the probe finds the rays coherent, but they are still launched); otherwise the
     trace alone."""
-    return 6 if dbvh.variant in (dbvh.VARIANT_SORTED, dbvh.VARIANT_SORTED_OCC) else 1
+    return 5 if dbvh.variant in (dbvh.VARIANT_SORTED, dbvh.VARIANT_SORTED_OCC) else 1
 
 
 def bytes_per_ray(counters: np.ndarray) -> float:

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from tests.test_wide_bvh import SCENES, rays_for, soup
-from trenchanttracer_gb300 import BVHCompact, DeviceBVH, Scene
+from trenchanttracer_gb300 import BVHCompact, DeviceBVH, Renderer, Scene, make_camera_meta, render_params, scenes
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -40,3 +40,35 @@ def test_four_wide_equals_two_wide_on_the_gpu(name):
                 ref = hits(dbvh, r, DeviceBVH.VARIANT_DYNAMIC, closest, ext)
                 for variant in DeviceBVH.DETERMINISTIC_VARIANTS if n in (33, 40000) else (DeviceBVH.VARIANT_SORTED,):
                     assert np.array_equal(hits(dbvh, r, variant, closest, ext), ref), (n, closest, ext, variant)
+
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20, (1 << 20) + 37])
+def test_ordered_ray_sets_around_the_threshold(n):
+    """From 2^20 rays on the default variant traces them in sorted order; every hit is its own ray's."""
+    sc, alpha, leaf, extent = SCENES["spheres"]()
+    dbvh = DeviceBVH(BVHCompact.build(sc, alpha, 1, leaf))
+    rays = torch.from_numpy(rays_for(extent, 5, n)).cuda()
+    for closest, ext in ((True, False), (False, True)):
+        ref = hits(dbvh, rays, DeviceBVH.VARIANT_DYNAMIC, closest, ext)
+        for variant in (DeviceBVH.VARIANT_SORTED, DeviceBVH.VARIANT_SORTED_OCC):
+            assert np.array_equal(hits(dbvh, rays, variant, closest, ext), ref), (closest, ext, variant)
+
+
+@pytest.mark.parametrize("streamed", [0, 1])
+def test_ordered_queues_give_the_unordered_image(streamed):
+    """Queues of 2^22 rays and more are ordered: waves whose queues cross that length, and a streamed pool of
+    more slots than that."""
+    sc = Scene.from_mesh(scenes.multi_material(12, 3))
+    sc.set_env(scenes.sky_env(64, 32, sun_radiance=5e2, sun_diameter_deg=10.0))
+    r = Renderer(DeviceBVH(BVHCompact.build(sc, 1e-5, 1, 8)), sc)
+    w, h = 2311, 1999
+    cam = make_camera_meta(w, h, [0.0, 14.0, 34.0], [0.0, -12.0, -34.0], fov=(60.0, 53.0))
+    params = render_params(spp=3 if streamed else 1, max_depth=5, rr_depth=3, seed=3)
+    images = []
+    for ordered in (0, 1):
+        r.set_launch(128, 8, 6000000, ordered, streamed)
+        acc = torch.zeros(3 * w * h, device="cuda")
+        r.render_native(cam, params, acc)
+        r.check()
+        images.append(acc.cpu().numpy().view(np.uint32))
+    assert np.array_equal(*images)

@@ -98,25 +98,22 @@ struct CacheView {
     int *block_counts;        // filled slots per 1024-slot block
 };
 
-// Ordering of an extension queue (tt_reorder.cu): when order_built(state), k_extend reads the
-// ordered copy of the queue's first *n_sorted rays and writes their hits by ordered slot, and
-// k_order_gather_hits moves each of those hits back to its queue slot (pos: the ordered slot of
-// each queue slot). The rest of the queue (a streamed render's new camera rays, coherent as they
-// are) is traced in place.
+// Ordering of an extension queue (tt_reorder.cu): when order_built(state), k_extend takes the
+// queue's first *n_sorted slots in the order of src and writes their hits by place, and
+// k_order_gather_hits moves each of those hits back to its queue slot (pos: the place of each queue
+// slot). The rest of the queue (a streamed render's new camera rays, coherent as they are) is
+// traced in place.
 struct OrderView {
-    const float4 *sorted;  // nullptr: ordering off
-    float *hit_t, *hit_u, *hit_v;
-    int *hit_prim;
+    const int *src;  // nullptr: ordering off
+    float4 *hits;    // t, u, v, primitive by place
     const int *pos;
     const unsigned long long *state;
     const int *n_sorted;
 };
 
-// Ordering of the shadow queue: when order_built(state), k_shadow traces the queue in the order of
-// `sorted` and takes each ray's path and value from its original slot src[p].
+// Ordering of the shadow queue: when order_built(state), k_shadow takes its slots in the order of src.
 struct ShadowOrderView {
-    const float4 *sorted;  // nullptr: ordering off
-    const int *src;
+    const int *src;  // nullptr: ordering off
     const unsigned long long *state;
 };
 

@@ -29,8 +29,8 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
     WideStackOf<kSh, kBlock, true> stack;
     stack.sh = sh_stack + threadIdx.x;
     uint32_t err = 0;
-    // an ordered queue prefix: rays and hits by ordered slot, moved back by k_order_gather_hits
-    const bool ordered = a.order.sorted && order_built(a.order.state);
+    // an ordered queue prefix: hits by place, moved back by k_order_gather_hits
+    const bool ordered = a.order.src && order_built(a.order.state);
     const int n_sorted = ordered ? (kPrefix ? *a.order.n_sorted : n) : 0;
     trace_queue<true, kWideInner>(
         stack, a.bvh, (unsigned)n, err,
@@ -39,24 +39,31 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
             if (lane == 0) base = atomicAdd(a.ps.counts + 3, count);
             return (unsigned)__shfl_sync(0xffffffffu, base, 0);
         },
+        [&](unsigned place) {
+            const bool srt = kPrefix ? (int)place < n_sorted : ordered;
+            if (!srt) return place;
+            const unsigned q = (unsigned)a.order.src[place];
+            return q < (unsigned)n ? q : place;  // (always, with a consistent ordering)
+        },
         [&](unsigned q, float4 &r0, float4 &r1) {
-            const float4 *rays = (kPrefix ? (int)q < n_sorted : ordered) ? a.order.sorted : a.ps.ray[cur];
-            r0 = rays[2 * (size_t)q];
-            r1 = rays[2 * (size_t)q + 1];
+            r0 = a.ps.ray[cur][2 * (size_t)q];
+            r1 = a.ps.ray[cur][2 * (size_t)q + 1];
         },
         [&](unsigned lanes, unsigned q, const TraceResult &tr) {
-            const bool srt = kPrefix ? (int)q < n_sorted : ordered;
             float t = tr.t, hu = tr.u, hv = tr.v;
             int prim = tr.addr;
             if (a.num_geoms) {
-                const float4 *rays = srt ? a.order.sorted : a.ps.ray[cur];
-                const float4 r0 = rays[2 * (size_t)q], r1 = rays[2 * (size_t)q + 1];
+                const float4 r0 = a.ps.ray[cur][2 * (size_t)q], r1 = a.ps.ray[cur][2 * (size_t)q + 1];
                 analytic_hit(a, lanes, true, V3(r0.x, r0.y, r0.z), V3(r0.w, r1.x, r1.y), r1.z, t, prim, hu, hv, false);
             }
-            (srt ? a.order.hit_t : a.ps.hit_t)[q] = t;
-            (srt ? a.order.hit_prim : a.ps.hit_prim)[q] = prim;
-            (srt ? a.order.hit_u : a.ps.hit_u)[q] = hu;
-            (srt ? a.order.hit_v : a.ps.hit_v)[q] = hv;
+            if (kPrefix ? (int)q < n_sorted : ordered) {
+                a.order.hits[a.order.pos[q]] = make_float4(t, hu, hv, __int_as_float(prim));
+            } else {
+                a.ps.hit_t[q] = t;
+                a.ps.hit_prim[q] = prim;
+                a.ps.hit_u[q] = hu;
+                a.ps.hit_v[q] = hv;
+            }
         });
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.stats + 0, (unsigned long long)n);
     if (err) atomicOr(a.err, err);
@@ -71,9 +78,7 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
     WideStackOf<kSh, kBlock, false> stack;
     stack.sh = sh_stack + threadIdx.x;
     uint32_t err = 0;
-    // an ordered queue: rays in sorted order, each ray's path and value at its original slot
-    const bool ordered = a.shadow_order.sorted && order_built(a.shadow_order.state);
-    const float4 *rays = ordered ? a.shadow_order.sorted : a.ps.shadow_ray;
+    const bool ordered = a.shadow_order.src && order_built(a.shadow_order.state);
     trace_queue<false, kWideInner>(
         stack, a.bvh, (unsigned)n, err,
         [&](int count) {
@@ -81,29 +86,31 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
             if (lane == 0) base = atomicAdd(a.ps.counts + 4, count);
             return (unsigned)__shfl_sync(0xffffffffu, base, 0);
         },
+        [&](unsigned place) {
+            if (!ordered) return place;
+            const unsigned j = (unsigned)a.shadow_order.src[place];
+            return j < (unsigned)n ? j : place;  // (always, with a consistent ordering)
+        },
         [&](unsigned j, float4 &r0, float4 &r1) {
-            r0 = rays[2 * (size_t)j];
-            r1 = rays[2 * (size_t)j + 1];
+            r0 = a.ps.shadow_ray[2 * (size_t)j];
+            r1 = a.ps.shadow_ray[2 * (size_t)j + 1];
         },
         [&](unsigned lanes, unsigned j, const TraceResult &tr) {
             bool blocked = tr.addr >= 0;
             if (a.num_geoms) {
-                const float4 r0 = rays[2 * (size_t)j], r1 = rays[2 * (size_t)j + 1];
+                const float4 r0 = a.ps.shadow_ray[2 * (size_t)j], r1 = a.ps.shadow_ray[2 * (size_t)j + 1];
                 float t = r1.w, hu, hv;
                 int prim = -1;
                 analytic_hit(a, lanes, !blocked, V3(r0.x, r0.y, r0.z), V3(r0.w, r1.x, r1.y), r1.z, t, prim, hu, hv,
                              true);
                 blocked = blocked || prim != -1;
             }
-            const int src = ordered ? a.shadow_order.src[j] : (int)j;
-            if ((unsigned)src >= (unsigned)n) {  // not reachable with a consistent ordering
-                err |= kErrOrder;
-            } else if (!blocked) {
+            if (!blocked) {
                 // a path's radiance: L[3 * t] for t >= 0, else (an ended path of a streamed
                 // render) ring entry -1 - t
-                const int t = a.ps.shadow_path[src];
+                const int t = a.ps.shadow_path[j];
                 float *L = t >= 0 ? a.ps.L + 3ll * t : a.stream.ring + 3ll * (-1ll - t);
-                const float *c = a.ps.shadow_val + 3ll * src;
+                const float *c = a.ps.shadow_val + 3ll * j;
                 L[0] = PT_ADD(L[0], c[0]);
                 L[1] = PT_ADD(L[1], c[1]);
                 L[2] = PT_ADD(L[2], c[2]);
@@ -114,16 +121,17 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_order_gather_hits(NativeArgs a, int cur) {
-    if (!a.order.sorted || !order_built(a.order.state)) return;
+    if (!a.order.src || !order_built(a.order.state)) return;
     const int n = *a.order.n_sorted;
     unsigned bad = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int p = __ldcs(a.order.pos + i);
         if ((unsigned)p < (unsigned)n) {
-            a.ps.hit_t[i] = a.order.hit_t[p];
-            a.ps.hit_u[i] = a.order.hit_u[p];
-            a.ps.hit_v[i] = a.order.hit_v[p];
-            a.ps.hit_prim[i] = a.order.hit_prim[p];
+            const float4 h = a.order.hits[p];
+            a.ps.hit_t[i] = h.x;
+            a.ps.hit_u[i] = h.y;
+            a.ps.hit_v[i] = h.z;
+            a.ps.hit_prim[i] = __float_as_int(h.w);
         } else {  // not reachable with a consistent ordering: report, and let the path miss
             a.ps.hit_prim[i] = -1;
             bad = 1;

@@ -1315,9 +1315,8 @@ static bool has_shadows(const NativeArgs &a) { return a.env.w > 0 && !(a.p.flags
 static tt_status order_shadows(NativeArgs &a, long long cap, const OrderPlan &plan, cudaStream_t s) {
     OrderOut so;
     const tt_status st = reorder_rays(a.ps.shadow_ray, cap, a.ps.counts + 2, plan.lo, plan.hi, plan.scratch,
-                                      plan.state_at, a.err, s, &so, true);
+                                      plan.state_at, kOrderMinQueue, a.err, s, &so);
     if (st != TT_OK) return st;
-    a.shadow_order.sorted = so.sorted;
     a.shadow_order.src = so.src;
     a.shadow_order.state = so.state;
     return TT_OK;
@@ -1350,17 +1349,10 @@ static tt_status issue_waves(NativeArgs a, long long total, const Launch &L, con
             if (L.order) {  // order the queue; the probe leaves coherent queues (camera rays) alone
                 OrderOut oo;
                 const tt_status st = reorder_rays(a.ps.ray[b & 1], qcap, a.ps.counts + (b & 1), plan.lo, plan.hi,
-                                                  plan.scratch, plan.state_at, a.err, s, &oo);
+                                                  plan.scratch, plan.state_at,
+                              kOrderMinQueue, a.err, s, &oo, true);
                 if (st != TT_OK) return st;
-                float *h = static_cast<float *>(oo.sorted_hits);
-                a.order.n_sorted = a.ps.counts + (b & 1);
-                a.order.sorted = oo.sorted;
-                a.order.pos = oo.pos;
-                a.order.state = oo.state;
-                a.order.hit_t = h;
-                a.order.hit_u = h + qcap;
-                a.order.hit_v = h + 2 * qcap;
-                a.order.hit_prim = reinterpret_cast<int *>(h + 3 * qcap);
+                a.order = OrderView{oo.src, static_cast<float4 *>(oo.hits), oo.pos, oo.state, a.ps.counts + (b & 1)};
             }
             L.tk.extend<<<L.grid_trace, L.block, 0, s>>>(a, b & 1);
             if (L.order) k_order_gather_hits<<<L.grid_gather, 256, 0, s>>>(a, b & 1);
@@ -1484,17 +1476,10 @@ static tt_status issue_stream(NativeArgs a, long long total, const Launch &L, co
             // them are coherent already
             OrderOut oo;
             const int *n_sorted = &sv.plan->new_at;
-            st = reorder_rays(a.ps.ray[c], pool, n_sorted, plan.lo, plan.hi, plan.scratch, plan.state_at, a.err, s, &oo);
+            st = reorder_rays(a.ps.ray[c], pool, n_sorted, plan.lo, plan.hi, plan.scratch, plan.state_at,
+                              kOrderMinQueue, a.err, s, &oo, true);
             if (st != TT_OK) return st;
-            float *h = static_cast<float *>(oo.sorted_hits);
-            a.order.n_sorted = n_sorted;
-            a.order.sorted = oo.sorted;
-            a.order.pos = oo.pos;
-            a.order.state = oo.state;
-            a.order.hit_t = h;
-            a.order.hit_u = h + pool;
-            a.order.hit_v = h + 2 * pool;
-            a.order.hit_prim = reinterpret_cast<int *>(h + 3 * pool);
+            a.order = OrderView{oo.src, static_cast<float4 *>(oo.hits), oo.pos, oo.state, n_sorted};
         }
         (L.order ? L.tk.extend_prefix : L.tk.extend)<<<L.grid_trace, L.block, 0, s>>>(a, c);
         if (L.order) k_order_gather_hits<<<L.grid_gather, 256, 0, s>>>(a, c);

@@ -15,13 +15,10 @@
 // in their own order. (2) Keys, and for each ray its rank among the rays of its key, from one
 // atomic per group of equal keys in a warp (__match_any_sync). (3) Exclusive scan of the counts in
 // 2048-entry chunks, chunk totals aside. (4) Every block scans the 1024 chunk totals in shared
-// memory; each ray goes to slot chunk offset + count offset + rank, where the kernel writes the
-// ray itself (the trace kernel then reads rays and writes hits contiguously, in sorted order); the
-// slot is kept per ray, and after the trace a gather pass moves every hit to its own ray's place,
-// reading the sorted hits (32 MB for 4M rays: L2-resident) at random and writing the output in
-// order. Slots are bounds-checked. The order inside a key is whatever the atomics give; only the
-// grouping matters. Plain launches on the caller's stream, so copies on other streams keep
-// overlapping them.
+// memory; each ray's slot is chunk offset + count offset + rank, where the kernel writes the ray's
+// index; the trace kernel reads each ray, one 32-byte sector, through that index. Slots are
+// bounds-checked. The order inside a key is whatever the atomics give; only the grouping matters.
+// Plain launches on the caller's stream, so copies on other streams keep overlapping them.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -50,12 +47,12 @@ struct OrderArgs {
     const int *n_dev;  // rays = min(*n_dev, n) when set
     OrderGrid g;
     uint2 *kr;         // per ray: key, rank within the key
-    int *pos;          // per ray: its sorted slot
-    int *src;          // per sorted slot: its ray (nullptr: not wanted)
-    float4 *sorted;    // per sorted slot: the ray
+    int *pos;          // per ray: its sorted slot (nullptr: not wanted)
+    int *src;          // per sorted slot: its ray
     unsigned *counts;  // 2^key_bits
     unsigned *sums;    // chunk totals
     int key_bits;
+    int64_t min_rays;
     unsigned long long *state;
     unsigned *err;
 };
@@ -128,8 +125,8 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
         __threadfence();
         if (atomicAdd(a.state + 2, 1ull) == (unsigned long long)gridDim.x - 1) {  // every block's counts are in
             const unsigned long long u = atomicAdd(a.state + 0, 0ull), f = atomicAdd(a.state + 1, 0ull);
-            // ordered unless mostly uniform; fewer than kOrderMinRays stay in their own order
-            a.state[3] = (f > 0 && 2 * u <= f && n >= kOrderMinRays) ? 1ull : 0ull;
+            // ordered unless mostly uniform; fewer than min_rays stay in their own order
+            a.state[3] = (f > 0 && 2 * u <= f && n >= a.min_rays) ? 1ull : 0ull;
             a.state[0] = 0ull;
             a.state[1] = 0ull;
             a.state[2] = 0ull;
@@ -182,7 +179,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_scan(OrderArgs a) {
     if (threadIdx.x == 0) a.sums[blockIdx.x] = total;
 }
 
-// (4) chunk offsets (every block), then each ray and its slot
+// (4) chunk offsets (every block), then each ray's slot
 __global__ void __launch_bounds__(kOrderBlock) k_order_scatter(OrderArgs a) {
     if (!order_built(a.state)) return;
     __shared__ unsigned s_warp[kOrderBlock / 32];
@@ -206,19 +203,13 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_scatter(OrderArgs a) {
     const int64_t n = order_rays(a);
     for (int64_t i = (int64_t)blockIdx.x * kOrderBlock + threadIdx.x; i < n; i += (int64_t)gridDim.x * kOrderBlock) {
         const uint2 kr = a.kr[i];
-        if (kr.x >= (1u << a.key_bits)) {
-            a.pos[i] = -1;
-            bad = 1;
-            continue;
-        }
-        const uint64_t pos = (uint64_t)s_prefix[kr.x / kScanChunk] + a.counts[kr.x] + kr.y;
+        uint64_t pos = ~0ull;
+        if (kr.x < (1u << a.key_bits)) pos = (uint64_t)s_prefix[kr.x / kScanChunk] + a.counts[kr.x] + kr.y;
         if (pos < (uint64_t)n) {
-            a.sorted[2 * pos] = __ldg(a.rays + 2 * i);
-            a.sorted[2 * pos + 1] = __ldg(a.rays + 2 * i + 1);
-            a.pos[i] = (int)pos;
-            if (a.src) a.src[pos] = (int)i;
+            a.src[pos] = (int)i;
+            if (a.pos) a.pos[i] = (int)pos;
         } else {
-            a.pos[i] = -1;
+            if (a.pos) a.pos[i] = -1;
             bad = 1;
         }
     }
@@ -292,7 +283,7 @@ bool host_rays_coherent(const float *rays, int64_t n, const float lo[3], const f
 static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 size_t reorder_state_offset(int64_t n) {
-    return al256(8ull * n) + al256(4ull * n) + al256(32ull * n) + al256(24ull * n) + al256(4ull << kOrderBits) +
+    return al256(8ull * n) + al256(4ull * n) + al256(4ull * n) + al256(16ull * n) + al256(4ull << kOrderBits) +
            al256(4ull * kNumChunks);
 }
 
@@ -301,7 +292,8 @@ size_t reorder_scratch_bytes(int64_t n) { return reorder_state_offset(n) + 256; 
 static std::atomic<int> g_order_sms[64];  // SMs per device (0 = not yet known)
 
 tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const float lo[3], const float hi[3],
-                       void *scratch, size_t state_at, unsigned *err, cudaStream_t s, OrderOut *out, bool with_src) {
+                       void *scratch, size_t state_at, int64_t min_rays, unsigned *err, cudaStream_t s, OrderOut *out,
+                       bool with_pos) {
     if (n <= 0 || n >= ((int64_t)1 << 31)) return fail(TT_ERR_INVALID, "ray ordering: n must be in 1..2^31-1");
     if (state_at < reorder_state_offset(n) || (state_at & 255))
         return fail(TT_ERR_INVALID, "ray ordering: scratch too small for this many rays");
@@ -320,18 +312,18 @@ tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const fl
     a.rays = rays;
     a.n = n;
     a.n_dev = n_dev;
+    a.min_rays = min_rays;
     const int ob = order_origin_bits(n);
     a.g = order_grid(lo, hi, ob);
     a.key_bits = kOrderDirBits + ob;
     a.kr = reinterpret_cast<uint2 *>(p);
     p += al256(8ull * n);
-    a.pos = reinterpret_cast<int *>(p);
+    a.src = reinterpret_cast<int *>(p);
     p += al256(4ull * n);
-    a.sorted = reinterpret_cast<float4 *>(p);
-    p += al256(32ull * n);
-    void *sorted_hits = p;
-    a.src = with_src ? static_cast<int *>(sorted_hits) : nullptr;
-    p += al256(24ull * n);
+    a.pos = with_pos ? reinterpret_cast<int *>(p) : nullptr;
+    p += al256(4ull * n);
+    void *hits = p;
+    p += al256(16ull * n);
     a.counts = reinterpret_cast<unsigned *>(p);
     p += al256(4ull << kOrderBits);
     a.sums = reinterpret_cast<unsigned *>(p);
@@ -346,52 +338,9 @@ tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const fl
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("ray ordering: ") + cudaGetErrorString(e));
     out->pos = a.pos;
-    out->sorted = a.sorted;
-    out->sorted_hits = sorted_hits;
-    out->state = a.state;
     out->src = a.src;
-    return TT_OK;
-}
-
-// hits[i] = sorted_hits[pos[i]], one record of Rec per ray
-template <typename Rec>
-__global__ void __launch_bounds__(256) k_order_unpermute(Rec *hits, const Rec *sorted_hits, const int *pos, int64_t n,
-                                                         const unsigned long long *state, unsigned *err) {
-    if (!order_built(state)) return;
-    unsigned bad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int p = __ldcs(pos + i);
-        if ((uint64_t)(int64_t)p < (uint64_t)n) hits[i] = sorted_hits[p];
-        else bad = 1;
-    }
-    if (bad) atomicOr(err, kErrOrder);
-}
-
-struct HitExtRec {  // tt_hit_ext as three 8-byte words
-    uint2 w[3];
-};
-
-tt_status reorder_unpermute(const OrderOut &out, int64_t n, void *hits, size_t hit_bytes, unsigned *err,
-                            cudaStream_t s) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("ray ordering: ") + cudaGetErrorString(e));
-    const int sms = (dev >= 0 && dev < 64) ? g_order_sms[dev].load() : 0;
-    const int64_t want = (n + 255) / 256;
-    const int64_t cap = (int64_t)(sms > 0 ? sms : 132) * 8;
-    const unsigned grid = (unsigned)(want < cap ? want : cap);
-    if (hit_bytes == 8)
-        k_order_unpermute<uint2><<<grid, 256, 0, s>>>(static_cast<uint2 *>(hits),
-                                                       static_cast<const uint2 *>(out.sorted_hits), out.pos, n,
-                                                       out.state, err);
-    else if (hit_bytes == 24)
-        k_order_unpermute<HitExtRec><<<grid, 256, 0, s>>>(static_cast<HitExtRec *>(hits),
-                                                           static_cast<const HitExtRec *>(out.sorted_hits), out.pos,
-                                                           n, out.state, err);
-    else
-        return fail(TT_ERR_INVALID, "ray ordering: hit records are 8 or 24 bytes");
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("ray ordering: ") + cudaGetErrorString(e));
+    out->hits = hits;
+    out->state = a.state;
     return TT_OK;
 }
 

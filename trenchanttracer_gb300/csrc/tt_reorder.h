@@ -19,9 +19,17 @@ constexpr int kOrderOriginBits = 13;
 constexpr int kOrderMinOriginBits = 6;
 constexpr int kOrderBits = kOrderDirBits + kOrderOriginBits;  // the largest key
 static_assert(kOrderDirBits % 2 == 0 && kOrderBits <= 21, "direction cells square; counts for 2^21 keys at most");
-// Fewer rays than this are traced in their own order: ordering them cannot pay for the scan of
-// the 2^21 key counts.
-constexpr int64_t kOrderMinRays = 1 << 15;
+// Fewer rays than this are traced in their own order: ordering them does not pay for its passes.
+// Measured on hashed cosine bounces and shadow rays, ordered against not, in us: on a
+// 2,097,152-triangle terrain 287 / 269 at 1M, 451 / 457 at 2M, 790 / 835 at 4M (shadow rays 371 / 382
+// and 1,166 / 1,310 at 1M and 4M); on 400 spheres of 5,120 triangles 201 / 179 at 300K, 395 / 407 at 1M,
+// 1,215 / 1,398 at 4M (shadow rays 342 / 370 and 1,092 / 1,284).
+constexpr int64_t kOrderMinRays = 1 << 20;
+// The same for the queues of a render. They follow the image, so neighbours start close together
+// and go less far astray: with queues from 1M rays on ordered, 12 uneven views of a terrain (4M-slot
+// pool) take 3.35 ms, from 2M on 2.88, from 4M on 2.65; 960 x 540 x 16 samples of 400 spheres 15.5, 15.2
+// and 15.2 ms.
+constexpr int64_t kOrderMinQueue = 1 << 22;
 // Error-word bit: a sorted slot came out of range (the ray's hit is then left unwritten).
 constexpr uint32_t kErrOrder = 4u;
 
@@ -78,19 +86,18 @@ OrderGrid order_grid(const float lo[3], const float hi[3], int origin_bits);
 // the device probe, for callers that still hold the rays on the host.
 bool host_rays_coherent(const float *rays, int64_t n, const float lo[3], const float hi[3]);
 
-// Device scratch for ordering n rays: key + rank, sorted slot of each ray, sorted ray copy, sorted
-// hit records (up to 24 B), 2^21 counts, the scan's chunk totals and the 256-byte state block
-// (which must be zero when the scratch is new).
+// Device scratch for ordering n rays: key + rank, the ray of each sorted slot, the sorted slot of
+// each ray, 16 B per ray for a caller's hits in sorted order, 2^21 counts, the scan's chunk totals and
+// the 256-byte state block (which must be zero when the scratch is new).
 size_t reorder_scratch_bytes(int64_t n);
 // Byte offset of the state block inside the scratch (to clear it on allocation).
 size_t reorder_state_offset(int64_t n);
 
 struct OrderOut {
-    const int *pos;                   // sorted slot of each ray
-    const float4 *sorted;             // 2 float4 per sorted slot
-    void *sorted_hits;                // hit record per sorted slot, written by the trace kernel
-    const unsigned long long *state;  // order_built(state): whether pos / sorted were built
-    const int *src;                   // with_src: the ray slot of each sorted slot (in sorted_hits)
+    const int *src;                   // ray of each sorted slot
+    const int *pos;                   // sorted slot of each ray (with_pos)
+    void *hits;                       // 16 B per ray
+    const unsigned long long *state;  // order_built(state): whether src / pos were built
 };
 
 // Launches (on stream s) the ordering of n rays (or of min(*n_dev, n) when n_dev is set: a count
@@ -98,21 +105,20 @@ struct OrderOut {
 // reorder_scratch_bytes(n); its 256-byte state block sits at byte state_at, zeroed when the
 // scratch was made and fixed for its life (reorder_state_offset of the size it was made for).
 // Calls on one scratch must be ordered (one stream). Launches only, no allocation, so a call can
-// be captured in a CUDA graph. Device-side errors go to *err as kErrOrder. with_src: the scatter
-// also writes the inverse permutation (out->src, over the sorted_hits region), for a pass that
-// reads the rays in sorted order and their other records by original slot.
+// be captured in a CUDA graph. Fewer than min_rays rays keep their own order. Device-side errors go
+// to *err as kErrOrder. with_pos: also the
+// inverse permutation.
+//
+// The rays themselves stay where they are and a trace kernel reads them through src. A copy in
+// sorted order, undone for the hits by a last pass, cost more than the scattered sectors do in a trace
+// that takes 3 % of the memory bandwidth: 4M terrain bounces 840 us with the copy, 790 without.
 tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const float lo[3], const float hi[3],
-                       void *scratch, size_t state_at, unsigned *err, cudaStream_t s, OrderOut *out, bool with_src = false);
-
-// After the trace kernel wrote hits of hit_bytes (8 or 24) per sorted slot into out.sorted_hits:
-// moves each ray's hit to hits[ray] (launch only; nothing to do when the order was not built).
-tt_status reorder_unpermute(const OrderOut &out, int64_t n, void *hits, size_t hit_bytes, unsigned *err,
-                            cudaStream_t s);
+                       void *scratch, size_t state_at, int64_t min_rays, unsigned *err, cudaStream_t s, OrderOut *out,
+                       bool with_pos = false);
 
 // Whether this call's rays were ordered: false when more than half of the sampled warps held 32
 // equal keys (the rays are coherent already: camera rays share one origin cell and neighbouring
-// pixels one direction cell) or fewer than kOrderMinRays rays came; they are then traced in their
-// own order.
+// pixels one direction cell) or too few rays came; they are then traced in their own order.
 __device__ __forceinline__ bool order_built(const unsigned long long *state) { return state[3] == 1ull; }
 
 }  // namespace tt

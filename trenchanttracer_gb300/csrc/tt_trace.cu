@@ -16,10 +16,9 @@
 //                         active at the vote depends on how the warp re-converges, so in float
 //                         corner cases (a leaf box whose entry rounds above a nearly equal hit
 //                         distance) the result can depend on the other rays of the warp.
-//   TT_VARIANT_SORTED     with 8 shared stack entries, over the rays in the order of a counting sort
-//                         by origin cell and direction cell (tt_reorder.cu), or in their own order
-//                         when a sample finds them coherent; each hit still goes to its own ray's
-//                         slot.
+//   TT_VARIANT_SORTED     with 8 shared stack entries, 1M rays and more in the order of a counting
+//                         sort by origin cell and direction cell (tt_reorder.cu) unless a sample
+//                         finds them coherent; each hit still goes to its own ray's slot.
 //   TT_VARIANT_SH16_OCC,  WARP_SH16 and SORTED (16 entries) compiled for 12 resident blocks per SM (40
 //   TT_VARIANT_SORTED_OCC registers and spilled values), trading spills for more warps.
 // All but WARP_VOTE return the per-ray result of the reference's algorithm, bit for bit.
@@ -110,10 +109,8 @@ struct TraceArgs {
     void *hits;
     unsigned long long *counter;
     unsigned int *err;
-    // TT_VARIANT_SORTED, when order_built(order_state): rays and hits by sorted slot (the hits
-    // are moved to their rays' places afterwards)
-    const float4 *sorted;
-    void *sorted_hits;
+    // TT_VARIANT_SORTED, when order_built(order_state): the ray in each place of the order
+    const int *order_src;
     const unsigned long long *order_state;
 };
 
@@ -140,7 +137,7 @@ __device__ __forceinline__ void store_hit(const TraceArgs &a, void *hits, int64_
     }
 }
 
-// The four-wide tree (kPerm: over the slots of the sorted ray copy, when the ordering built one). kSh
+// The four-wide tree (kPerm: in the rays' order, when the ordering built one). kSh
 // stack entries live in shared memory.
 template <bool kClosest, bool kExt, int kSh, bool kPerm, int kMinBlocks>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(TraceArgs a) {
@@ -149,10 +146,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
     uint32_t err = 0;
     WideStackOf<kSh, kTraceBlock, kClosest> stack;
     stack.sh = sh_stack + threadIdx.x;
-    const bool use_perm = kPerm && order_built(a.order_state);
-    // sorted: rays and hits by sorted slot (contiguous); else by ray
-    const float4 *rays = use_perm ? a.sorted : a.rays;
-    void *hits = use_perm ? a.sorted_hits : a.hits;
+    const bool use_perm = kPerm && a.order_state && order_built(a.order_state);
     trace_queue<kClosest, kWideInner>(
         stack, a.bvh, (unsigned)a.n, err,
         [&](int count) {
@@ -160,11 +154,12 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
             if (lane == 0) b = (unsigned)atomicAdd(a.counter, (unsigned long long)count);
             return __shfl_sync(0xffffffffu, b, 0);
         },
+        [&](unsigned place) { return use_perm ? (unsigned)__ldg(a.order_src + place) : place; },
         [&](unsigned i, float4 &r0, float4 &r1) {
-            r0 = __ldg(rays + 2 * (size_t)i);
-            r1 = __ldg(rays + 2 * (size_t)i + 1);
+            r0 = __ldg(a.rays + 2 * (size_t)i);
+            r1 = __ldg(a.rays + 2 * (size_t)i + 1);
         },
-        [&](unsigned, unsigned i, const TraceResult &tr) { store_hit<kExt>(a, hits, i, tr); });
+        [&](unsigned, unsigned i, const TraceResult &tr) { store_hit<kExt>(a, a.hits, i, tr); });
     if (err) atomicOr(a.err, err);
 }
 
@@ -184,14 +179,13 @@ __global__ void __launch_bounds__(kTraceBlock) trace_warp_kernel(TraceArgs a) {
         if ((int64_t)base >= a.n) break;
         const int64_t slot = (int64_t)base + lane;
         if (slot < a.n) {
-            // sorted: rays and hits by sorted slot (contiguous); else by ray
-            const float4 *rays = use_perm ? a.sorted : a.rays;
-            const float4 r0 = __ldg(rays + 2 * slot), r1 = __ldg(rays + 2 * slot + 1);
+            const int64_t i = use_perm ? (int64_t)__ldg(a.order_src + slot) : slot;
+            const float4 r0 = __ldg(a.rays + 2 * i), r1 = __ldg(a.rays + 2 * i + 1);
             TravState s;
             trav_init(s, stack, r0, r1);
             while (!trav_iterate<kClosest, kSpec>(s, stack, a.bvh, err, r1.w)) {
             }
-            store_hit<kExt>(a, use_perm ? a.sorted_hits : a.hits, slot, s);
+            store_hit<kExt>(a, a.hits, i, s);
         }
         __syncwarp();
     }
@@ -390,7 +384,7 @@ static void setup_l2_window(DeviceBVH &d) {
     cudaGetLastError();
 }
 
-// unordered = true traces a SORTED / SORTED_OCC variant's rays in their own order (its unsorted twin).
+// unordered = true traces a SORTED / SORTED_OCC variant's rays in their own order.
 static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n, void *d_hits, bool closest,
                               bool ext, cudaStream_t stream, int counter_slot = 0, bool unordered = false) {
     if (n < 0 || n > ((int64_t)1 << 40)) return fail(TT_ERR_INVALID, "ray count out of range");
@@ -415,16 +409,13 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     a.hits = d_hits;
     a.counter = d.scratch + counter_slot;
     a.err = reinterpret_cast<unsigned int *>(d.scratch + kScratchErr);
-    a.sorted = nullptr;
-    a.sorted_hits = nullptr;
+    a.order_src = nullptr;
     a.order_state = nullptr;
     OrderOut order{};
     int variant = d.variant;
-    const bool sorted = variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC;
     // too few rays cannot pay for the ordering
-    if (sorted && (unordered || n < kOrderMinRays))
-        variant = variant == VARIANT_SORTED_OCC ? VARIANT_SH16_OCC : VARIANT_WARP_SH16;
-    const bool order_rays = variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC;
+    const bool order_rays =
+        (variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC) && !unordered && n >= kOrderMinRays;
     if (!d.view.wide_nodes && variant != VARIANT_DYNAMIC && variant != VARIANT_WARP_VOTE) variant = VARIANT_TWO_WIDE;
     if (order_rays) {
         // one scratch per work-counter slot, so the pipeline streams never share one
@@ -443,10 +434,10 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
             if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("ray ordering scratch: ") + cudaGetErrorString(e));
         }
         const tt_status st =
-            reorder_rays(a.rays, n, nullptr, d.lo, d.hi, dm.order[k], dm.order_state_at[k], a.err, stream, &order);
+            reorder_rays(a.rays, n, nullptr, d.lo, d.hi, dm.order[k], dm.order_state_at[k], kOrderMinRays, a.err, stream,
+                         &order);
         if (st != TT_OK) return st;
-        a.sorted = order.sorted;
-        a.sorted_hits = order.sorted_hits;
+        a.order_src = order.src;
         a.order_state = order.state;
     }
     // Four rays a warp before a second warp is left out: a small set is bound by its longest chain of
@@ -463,7 +454,6 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     else le = ext ? launch_variant<false, true>(d, variant, (unsigned)blocks, stream, a)
                   : launch_variant<false, false>(d, variant, (unsigned)blocks, stream, a);
     TT_CUDA(le);
-    if (a.order_state) return reorder_unpermute(order, n, d_hits, ext ? sizeof(tt_hit_ext) : sizeof(tt_hit), a.err, stream);
     return TT_OK;
 }
 

@@ -221,16 +221,6 @@ __device__ __noinline__ TraceResult traverse_two_wide(const BvhView &bvh, float4
     return traverse<kClosest>(bvh, r0, r1, err);
 }
 
-// The rest of trav_leaf_phase's test, for a triangle whose cheap tests did not refuse it.
-__device__ __forceinline__ bool accept_triangle(float det, float un, float vn, float tn, float tmin, float tcur,
-                                                float &u, float &v, float &t) {
-    const float inv_det = __frcp_rn(det);
-    u = __fmul_rn(un, inv_det);
-    v = __fmul_rn(vn, inv_det);
-    t = __fmul_rn(tn, inv_det);
-    return !(u < 0.0f || u > 1.0f || v < 0.0f || __fadd_rn(u, v) > 1.0f) && tmin < t && t < tcur;
-}
-
 // What a lane is about to do, besides visiting an inner node (reference < kWideMark) or a leaf
 // (bit 31 set).
 constexpr uint32_t kWidePop = 0x7ffffffeu;   // take the next stack entry
@@ -358,6 +348,16 @@ __device__ __forceinline__ void wide_node(WideState &s, Stack &stack, const BvhV
     s.ref = n0 < kNone ? qn0 : kWidePop;
 }
 
+// The rest of trav_leaf_phase's test, for a triangle whose cheap tests did not refuse it.
+__device__ __forceinline__ bool accept_triangle(float det, float un, float vn, float tn, float tmin, float tcur,
+                                                float &u, float &v, float &t) {
+    const float inv_det = __frcp_rn(det);
+    u = __fmul_rn(un, inv_det);
+    v = __fmul_rn(vn, inv_det);
+    t = __fmul_rn(tn, inv_det);
+    return !(u < 0.0f || u > 1.0f || v < 0.0f || __fadd_rn(u, v) > 1.0f) && tmin < t && t < tcur;
+}
+
 // Tests the triangles of leaf s.ref.
 template <bool kClosest>
 __device__ __forceinline__ void wide_leaf(WideState &s, const BvhView &bvh, float4 r0, float4 r1) {
@@ -453,15 +453,16 @@ constexpr int kWideInner = 8;
 // stand at inner nodes they step on; then the lanes that wait at leaves test their triangles
 // together, and where none does, the lanes whose rays are finished store them and take the queue's
 // next ones (one claim; consecutive slots, so an ordered queue's neighbours start together).
-// claim(count): the first of `count` slots, all lanes taking part (slots from n on do not exist);
-// fetch(slot, r0, r1): a slot's ray; store(lanes, slot, result): the lanes of `lanes` store together.
+// claim(count): the first of `count` queue places, all lanes taking part (places from n on do not
+// exist); at(place): the slot in that place; fetch(slot, r0, r1): a slot's ray; store(lanes, slot,
+// result): the lanes of `lanes` store together.
 //
 // Measured on 4M rays over a 2,097,152-triangle terrain against one warp-wide loop per 32 rays (each
 // lane runs its own ray to its end): cosine bounces 0.86 against 1.05 ms, camera rays 0.49 against
 // 0.54 ms; 18 of 32 lanes busy instead of 10.
-template <bool kClosest, int kInner, class Stack, class Claim, class Fetch, class Store>
+template <bool kClosest, int kInner, class Stack, class Claim, class At, class Fetch, class Store>
 __device__ __forceinline__ void trace_queue(Stack &stack, const BvhView &bvh, unsigned n, uint32_t &err, Claim claim,
-                                            Fetch fetch, Store store) {
+                                            At at, Fetch fetch, Store store) {
     WideState s;
     s.ref = kWideIdle;
     unsigned slot = 0;
@@ -495,7 +496,7 @@ __device__ __forceinline__ void trace_queue(Stack &stack, const BvhView &bvh, un
                 if (s.ref == kWideIdle) {
                     const unsigned off = __popc(want & ((1u << (threadIdx.x & 31)) - 1u));
                     if (off < count && base < n && off < n - base) {
-                        slot = base + off;
+                        slot = at(base + off);
                         float4 r0, r1;
                         fetch(slot, r0, r1);
                         if (!wide_start(s, bvh, r0, r1)) {
