@@ -7,6 +7,7 @@
 // stack depth in kBlockShapes x kStackShapes; the renderer's autotuner picks one.
 #include <cuda_runtime.h>
 
+#include "tt_launch.cuh"
 #include "tt_native.cuh"
 #include "tt_wide.cuh"
 
@@ -18,6 +19,7 @@ using namespace pt;
 // survivors); the rest is traced in place. Without it an ordered queue is ordered whole.
 template <int kBlock, int kSh, bool kPrefix>
 __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
+    chain_begin();
     __shared__ uint2 sh_stack[(kSh > 0 ? kSh : 1) * kBlock];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.ps.counts[cur ^ 1] = 0;
@@ -71,6 +73,7 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
 
 template <int kBlock, int kSh>
 __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
+    chain_begin();
     __shared__ uint32_t sh_stack[(kSh > 0 ? kSh : 1) * kBlock];
     if (blockIdx.x == 0 && threadIdx.x == 0) a.ps.counts[3] = 0;  // the next extend's work counter
     const int n = a.ps.counts[2];
@@ -121,6 +124,7 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_order_gather_hits(NativeArgs a, int cur) {
+    chain_begin();
     if (!a.order.src || !order_built(a.order.state)) return;
     const int n = *a.order.n_sorted;
     unsigned bad = 0;

@@ -43,6 +43,7 @@
 #include <string>
 #include <vector>
 
+#include "tt_launch.cuh"
 #include "tt_native.cuh"
 #include "tt_nrc_host.h"
 
@@ -394,6 +395,7 @@ __device__ __forceinline__ bool cache_vertex(const NativeArgs &a, int i, int dep
 
 // Filled training slots per 1024-slot block.
 __global__ void __launch_bounds__(1024) k_cache_count(NativeArgs a) {
+    chain_begin();
     const int s = blockIdx.x * 1024 + threadIdx.x;
     const int filled = __syncthreads_count(s < a.cache.train_slots && a.cache.s_path[s] >= 0);
     if (threadIdx.x == 0) a.cache.block_counts[blockIdx.x] = filled;
@@ -402,6 +404,7 @@ __global__ void __launch_bounds__(1024) k_cache_count(NativeArgs a) {
 // The filled training slots, in slot order, into the record arrays the targets and the training
 // read; counts[1] = their number.
 __global__ void __launch_bounds__(1024) k_cache_compact(NativeArgs a) {
+    chain_begin();
     __shared__ int s_base, s_warp[32];
     const int s = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
@@ -440,6 +443,7 @@ __global__ void __launch_bounds__(1024) k_cache_compact(NativeArgs a) {
 
 // Adds throughput x cache radiance of every query to its path.
 __global__ void __launch_bounds__(kShadeBlockMax) k_cache_resolve(NativeArgs a) {
+    chain_begin();
     const int n = a.cache.counts[0];
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         float *L = a.ps.L + 3ll * a.cache.q_path[q];
@@ -452,6 +456,7 @@ __global__ void __launch_bounds__(kShadeBlockMax) k_cache_resolve(NativeArgs a) 
 
 // Training targets: the radiance each training path measured from its record vertex on.
 __global__ void __launch_bounds__(kShadeBlockMax) k_cache_targets(NativeArgs a) {
+    chain_begin();
     const int n = min(a.cache.counts[1], a.cache.train_cap);
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const float *L = a.ps.L + 3ll * a.cache.t_path[s];
@@ -530,6 +535,7 @@ __device__ __forceinline__ void start_path(const PathState &S, int i, float4 *ra
 
 // Camera rays of the wave's paths into queue 0.
 __global__ void __launch_bounds__(kShadeBlockMax) k_raygen(NativeArgs a) {
+    chain_begin();
     const int stride = gridDim.x * blockDim.x;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.ps.counts[0] = a.wave_paths;
@@ -563,6 +569,7 @@ __global__ void __launch_bounds__(kShadeBlockMax) k_raygen(NativeArgs a) {
 // into the frontier (all paths below it have ended), the range to accumulate and the refill.
 
 __global__ void k_stream_init(NativeArgs a) {
+    chain_begin();
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     StreamPlan *pl = a.stream.plan;
     pl->next = 0;
@@ -576,6 +583,7 @@ __global__ void k_stream_init(NativeArgs a) {
 
 // final = 1: no refill, and the frontier must have reached the end of the index space.
 __global__ void k_stream_plan(NativeArgs a, int c, int pool, int final) {
+    chain_begin();
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     StreamPlan *pl = a.stream.plan;
     const int alive = a.ps.counts[c];
@@ -602,6 +610,7 @@ __global__ void k_stream_plan(NativeArgs a, int c, int pool, int final) {
 
 // The refill: new paths behind the survivors in queue c.
 __global__ void __launch_bounds__(kShadeBlockMax) k_regen(NativeArgs a, int c) {
+    chain_begin();
     const StreamPlan *pl = a.stream.plan;
     const int n = pl->new_n, at = pl->new_at;
     const long long first = pl->new_first;
@@ -808,9 +817,15 @@ __device__ __forceinline__ void shade_queue(const NativeArgs &a, int cur) {
 #undef TT_ST
 }
 
-__global__ void __launch_bounds__(kShadeBlockMax) k_shade(NativeArgs a, int cur) { shade_queue<false>(a, cur); }
+__global__ void __launch_bounds__(kShadeBlockMax) k_shade(NativeArgs a, int cur) {
+    chain_begin();
+    shade_queue<false>(a, cur);
+}
 
-__global__ void __launch_bounds__(kShadeBlockMax) k_shade_stream(NativeArgs a, int cur) { shade_queue<true>(a, cur); }
+__global__ void __launch_bounds__(kShadeBlockMax) k_shade_stream(NativeArgs a, int cur) {
+    chain_begin();
+    shade_queue<true>(a, cur);
+}
 
 // Adds the radiance of paths [first, first + n) to the views' accumulation blocks. The thread of
 // a pixel's first path in the range adds all of that pixel's paths in the range, in sample order,
@@ -842,11 +857,13 @@ __device__ __forceinline__ void accumulate_range(const NativeArgs &a, T *accum, 
 
 template <typename T>
 __global__ void __launch_bounds__(kShadeBlockMax) k_accumulate(NativeArgs a, T *accum) {
+    chain_begin();
     accumulate_range<T, false>(a, accum, a.wave_first, a.wave_paths, a.ps.L);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kShadeBlockMax) k_accumulate_stream(NativeArgs a, T *accum) {
+    chain_begin();
     const long long lo = a.stream.plan->acc_lo, hi = a.stream.plan->acc_hi;
     accumulate_range<T, true>(a, accum, lo, hi - lo, a.stream.ring);
 }
@@ -1343,7 +1360,7 @@ static tt_status issue_waves(NativeArgs a, long long total, const Launch &L, con
             if (a.cache.train_slots > a.cache.train_cap)
                 return fail(TT_ERR_INVALID, "cache: more training paths in a wave than training slots");
         }
-        k_raygen<<<L.grid_shade, L.block, 0, s>>>(a);
+        launch_chained(k_raygen, L.grid_shade, L.block, 0, s, a);
         r->launches += 1 + (accum ? 1 : 0) + (unsigned long long)a.p.max_depth * (L.order ? (has_shadows(a) ? 12 : 8) : 3);
         for (int b = 0; b < a.p.max_depth; b++) {
             if (L.order) {  // order the queue; the probe leaves coherent queues (camera rays) alone
@@ -1354,35 +1371,35 @@ static tt_status issue_waves(NativeArgs a, long long total, const Launch &L, con
                 if (st != TT_OK) return st;
                 a.order = OrderView{oo.src, static_cast<float4 *>(oo.hits), oo.pos, oo.state, a.ps.counts + (b & 1)};
             }
-            L.tk.extend<<<L.grid_trace, L.block, 0, s>>>(a, b & 1);
-            if (L.order) k_order_gather_hits<<<L.grid_gather, 256, 0, s>>>(a, b & 1);
-            k_shade<<<L.grid_shade, L.block, 0, s>>>(a, b & 1);
+            launch_chained(L.tk.extend, L.grid_trace, L.block, 0, s, a, b & 1);
+            if (L.order) launch_chained(k_order_gather_hits, L.grid_gather, 256, 0, s, a, b & 1);
+            launch_chained(k_shade, L.grid_shade, L.block, 0, s, a, b & 1);
             if (L.order && has_shadows(a)) {  // the shadow queue too (scratch shared with the extension queue's)
                 const tt_status st = order_shadows(a, qcap, plan, s);
                 if (st != TT_OK) return st;
             }
-            L.tk.shadow<<<L.grid_trace, L.block, 0, s>>>(a);
+            launch_chained(L.tk.shadow, L.grid_trace, L.block, 0, s, a);
         }
         if (cache) {  // every path queries at most once, so all queries of the wave fit
             const tt_status st = nrc::cache_infer_device(cache, a.cache.q_rec, a.cache.counts, a.wave_paths,
                                                          a.cache.q_rgb, nrc::cache_params(cache).use_ema, a.err, s);
             if (st != TT_OK) return st;
-            k_cache_resolve<<<L.grid_shade, L.block, 0, s>>>(a);
+            launch_chained(k_cache_resolve, L.grid_shade, L.block, 0, s, a);
             r->launches += 1;
         }
         if (cache && train) {
             if (a.cache.train_slots > 0) {  // the records in slot order
                 const unsigned nb = (unsigned)((a.cache.train_slots + 1023) / 1024);
-                k_cache_count<<<nb, 1024, 0, s>>>(a);
-                k_cache_compact<<<nb, 1024, 0, s>>>(a);
+                launch_chained(k_cache_count, nb, 1024, 0, s, a);
+                launch_chained(k_cache_compact, nb, 1024, 0, s, a);
                 r->launches += 2;
             }
-            k_cache_targets<<<L.grid_shade, L.block, 0, s>>>(a);
+            launch_chained(k_cache_targets, L.grid_shade, L.block, 0, s, a);
             r->launches += 1;
         }
         if (accum) {
-            if (f64) k_accumulate<double><<<L.grid_shade, L.block, 0, s>>>(a, (double *)accum);
-            else k_accumulate<float><<<L.grid_shade, L.block, 0, s>>>(a, (float *)accum);
+            if (f64) launch_chained(k_accumulate<double>, L.grid_shade, L.block, 0, s, a, (double *)accum);
+            else launch_chained(k_accumulate<float>, L.grid_shade, L.block, 0, s, a, (float *)accum);
         }
         if (cache && train) {
             const tt_status st = nrc::cache_train_device(cache, a.cache.t_rec, a.cache.t_target, a.cache.counts + 1, s);
@@ -1460,17 +1477,17 @@ static tt_status issue_stream(NativeArgs a, long long total, const Launch &L, co
     // accumulate
     r->launches += 1 + (unsigned long long)iters * ((accum ? 6 : 5) + (L.order ? (has_shadows(a) ? 9 : 5) : 0)) +
                    (accum ? 2 : 1);
-    k_stream_init<<<1, 32, 0, s>>>(a);
+    launch_chained(k_stream_init, 1, 32, 0, s, a);
     for (long long it = 0; it <= iters; it++) {
         const int c = (int)(it & 1);
         const bool last = it == iters;
-        k_stream_plan<<<1, 32, 0, s>>>(a, c, (int)pool, last ? 1 : 0);
+        launch_chained(k_stream_plan, 1, 32, 0, s, a, c, (int)pool, last ? 1 : 0);
         if (accum) {
-            if (f64) k_accumulate_stream<double><<<L.grid_shade, L.block, 0, s>>>(a, (double *)accum);
-            else k_accumulate_stream<float><<<L.grid_shade, L.block, 0, s>>>(a, (float *)accum);
+            if (f64) launch_chained(k_accumulate_stream<double>, L.grid_shade, L.block, 0, s, a, (double *)accum);
+            else launch_chained(k_accumulate_stream<float>, L.grid_shade, L.block, 0, s, a, (float *)accum);
         }
         if (last) break;
-        k_regen<<<L.grid_shade, L.block, 0, s>>>(a, c);
+        launch_chained(k_regen, L.grid_shade, L.block, 0, s, a, c);
         if (L.order) {
             // the survivors (queue slots below new_at) are ordered; the new camera rays behind
             // them are coherent already
@@ -1481,16 +1498,16 @@ static tt_status issue_stream(NativeArgs a, long long total, const Launch &L, co
             if (st != TT_OK) return st;
             a.order = OrderView{oo.src, static_cast<float4 *>(oo.hits), oo.pos, oo.state, n_sorted};
         }
-        (L.order ? L.tk.extend_prefix : L.tk.extend)<<<L.grid_trace, L.block, 0, s>>>(a, c);
-        if (L.order) k_order_gather_hits<<<L.grid_gather, 256, 0, s>>>(a, c);
-        k_shade_stream<<<L.grid_shade, L.block, 0, s>>>(a, c);
+        launch_chained((L.order ? L.tk.extend_prefix : L.tk.extend), L.grid_trace, L.block, 0, s, a, c);
+        if (L.order) launch_chained(k_order_gather_hits, L.grid_gather, 256, 0, s, a, c);
+        launch_chained(k_shade_stream, L.grid_shade, L.block, 0, s, a, c);
         if (L.order && has_shadows(a)) {
             st = order_shadows(a, pool, plan, s);
             if (st != TT_OK) return st;
         }
         NativeArgs as = a;  // shadow rays of survivors add to their state in the next queue
         as.ps.L = sv.st[c ^ 1].L;
-        L.tk.shadow<<<L.grid_trace, L.block, 0, s>>>(as);
+        launch_chained(L.tk.shadow, L.grid_trace, L.block, 0, s, as);
     }
     TT_CUDA_N(cudaGetLastError());
     return TT_OK;

@@ -27,6 +27,7 @@
 #include <string>
 
 #include "tt_internal.h"
+#include "tt_launch.cuh"
 #include "tt_reorder.h"
 
 namespace tt {
@@ -94,11 +95,16 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned x, unsigned *s
 
 // (1) clear the counts; probe; the last block decides
 __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
+    chain_begin();
     __shared__ unsigned s_probe[2];
     const int lane = threadIdx.x & 31;
     const int64_t tid = (int64_t)blockIdx.x * kOrderBlock + threadIdx.x;
     const int64_t nthreads = (int64_t)gridDim.x * kOrderBlock;
     const int64_t n = order_rays(a);
+    if (n < a.min_rays) {  // nothing to look at
+        if (tid == 0) a.state[3] = 0ull;
+        return;
+    }
     for (int64_t j = tid; j < (1 << a.key_bits) / 4; j += nthreads)
         reinterpret_cast<uint4 *>(a.counts)[j] = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < 2) s_probe[threadIdx.x] = 0u;
@@ -108,7 +114,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
     for (int64_t w = (tid >> 5) * kProbeStride; w < warps; w += (nthreads >> 5) * kProbeStride) {
         if (w * 32 + 32 > n) continue;  // only full warps count; w is the same in every lane
         const int64_t i = w * 32 + lane;
-        const unsigned key = order_key(__ldg(a.rays + 2 * i), __ldg(a.rays + 2 * i + 1), a.g);
+        const unsigned key = order_key(a.rays[2 * i], a.rays[2 * i + 1], a.g);
         full++;
         if (__match_any_sync(0xffffffffu, key) == 0xffffffffu) uniform++;
     }
@@ -125,8 +131,8 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
         __threadfence();
         if (atomicAdd(a.state + 2, 1ull) == (unsigned long long)gridDim.x - 1) {  // every block's counts are in
             const unsigned long long u = atomicAdd(a.state + 0, 0ull), f = atomicAdd(a.state + 1, 0ull);
-            // ordered unless mostly uniform; fewer than min_rays stay in their own order
-            a.state[3] = (f > 0 && 2 * u <= f && n >= a.min_rays) ? 1ull : 0ull;
+            // ordered unless mostly uniform
+            a.state[3] = (f > 0 && 2 * u <= f) ? 1ull : 0ull;
             a.state[0] = 0ull;
             a.state[1] = 0ull;
             a.state[2] = 0ull;
@@ -137,6 +143,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
 
 // (2) keys and ranks
 __global__ void __launch_bounds__(kOrderBlock) k_order_keys(OrderArgs a) {
+    chain_begin();
     if (!order_built(a.state)) return;
     const int lane = threadIdx.x & 31;
     const int64_t nthreads = (int64_t)gridDim.x * kOrderBlock;
@@ -146,7 +153,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_keys(OrderArgs a) {
         const int64_t i = base + lane;
         const bool valid = i < n;
         unsigned key = 0xffffffffu;  // no real key has bit 31 set
-        if (valid) key = order_key(__ldg(a.rays + 2 * i), __ldg(a.rays + 2 * i + 1), a.g);
+        if (valid) key = order_key(a.rays[2 * i], a.rays[2 * i + 1], a.g);
         const unsigned peers = __match_any_sync(0xffffffffu, key);
         const int leader = __ffs(peers) - 1;
         unsigned first = 0;
@@ -158,6 +165,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_keys(OrderArgs a) {
 
 // (3) exclusive scan of each chunk of counts (one chunk per block); chunk totals to sums
 __global__ void __launch_bounds__(kOrderBlock) k_order_scan(OrderArgs a) {
+    chain_begin();
     if (!order_built(a.state)) return;
     __shared__ unsigned s_warp[kOrderBlock / 32];
     uint4 *blk = reinterpret_cast<uint4 *>(a.counts + (size_t)blockIdx.x * kScanChunk);
@@ -181,6 +189,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_scan(OrderArgs a) {
 
 // (4) chunk offsets (every block), then each ray's slot
 __global__ void __launch_bounds__(kOrderBlock) k_order_scatter(OrderArgs a) {
+    chain_begin();
     if (!order_built(a.state)) return;
     __shared__ unsigned s_warp[kOrderBlock / 32];
     __shared__ unsigned s_prefix[kNumChunks];
@@ -331,11 +340,10 @@ tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const fl
     a.err = err;
     const int64_t want = (n + kOrderBlock - 1) / kOrderBlock;
     const unsigned grid = (unsigned)(want < (int64_t)sms * 8 ? want : (int64_t)sms * 8);
-    k_order_probe<<<(unsigned)sms * 4, kOrderBlock, 0, s>>>(a);
-    k_order_keys<<<grid, kOrderBlock, 0, s>>>(a);
-    k_order_scan<<<(1u << a.key_bits) / kScanChunk, kOrderBlock, 0, s>>>(a);
-    k_order_scatter<<<grid, kOrderBlock, 0, s>>>(a);
-    e = cudaGetLastError();
+    e = launch_chained(k_order_probe, (unsigned)sms * 4, kOrderBlock, 0, s, a);
+    if (e == cudaSuccess) e = launch_chained(k_order_keys, grid, kOrderBlock, 0, s, a);
+    if (e == cudaSuccess) e = launch_chained(k_order_scan, (1u << a.key_bits) / kScanChunk, kOrderBlock, 0, s, a);
+    if (e == cudaSuccess) e = launch_chained(k_order_scatter, grid, kOrderBlock, 0, s, a);
     if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("ray ordering: ") + cudaGetErrorString(e));
     out->pos = a.pos;
     out->src = a.src;

@@ -32,6 +32,7 @@
 #include <string>
 
 #include "tt_internal.h"
+#include "tt_launch.cuh"
 #include "tt_reorder.h"
 #include "tt_wide.cuh"
 #include "tt_wide_build.h"
@@ -141,26 +142,37 @@ __device__ __forceinline__ void store_hit(const TraceArgs &a, void *hits, int64_
 // stack entries live in shared memory.
 template <bool kClosest, bool kExt, int kSh, bool kPerm, int kMinBlocks>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(TraceArgs a) {
+    chain_begin();
     __shared__ typename WideEntry<kClosest>::type sh_stack[(kSh > 0 ? kSh : 1) * kTraceBlock];
     const int lane = threadIdx.x & 31;
     uint32_t err = 0;
     WideStackOf<kSh, kTraceBlock, kClosest> stack;
     stack.sh = sh_stack + threadIdx.x;
     const bool use_perm = kPerm && a.order_state && order_built(a.order_state);
+    unsigned *queue = reinterpret_cast<unsigned *>(a.counter);  // the next ray; blocks done
     trace_queue<kClosest, kWideInner>(
         stack, a.bvh, (unsigned)a.n, err,
         [&](int count) {
             unsigned b = 0;
-            if (lane == 0) b = (unsigned)atomicAdd(a.counter, (unsigned long long)count);
+            if (lane == 0) b = atomicAdd(queue, (unsigned)count);
             return __shfl_sync(0xffffffffu, b, 0);
         },
-        [&](unsigned place) { return use_perm ? (unsigned)__ldg(a.order_src + place) : place; },
+        [&](unsigned place) { return use_perm ? (unsigned)a.order_src[place] : place; },
         [&](unsigned i, float4 &r0, float4 &r1) {
             r0 = __ldg(a.rays + 2 * (size_t)i);
             r1 = __ldg(a.rays + 2 * (size_t)i + 1);
         },
         [&](unsigned, unsigned i, const TraceResult &tr) { store_hit<kExt>(a, a.hits, i, tr); });
     if (err) atomicOr(a.err, err);
+    // the last block to finish leaves the counter at 0 for the next launch (every claim is made by then)
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(queue + 1, 1u) == gridDim.x - 1) {
+            queue[0] = 0u;
+            queue[1] = 0u;
+        }
+    }
 }
 
 // The two-wide tree: each warp claims 32 consecutive rays. kSpec: with the reference's warp vote.
@@ -342,14 +354,15 @@ static void release(DeviceBVH &d) {
 // (rays, triangles, hits lie outside it) keeps the normal policy, so streaming triangles cannot
 // push the nodes out.
 template <bool kClosest, bool kExt>
-static cudaError_t launch_variant(const DeviceBVH &d, int variant, unsigned blocks, cudaStream_t stream,
+static cudaError_t launch_variant(const DeviceBVH &d, int variant, unsigned blocks, bool chained, cudaStream_t stream,
                                   TraceArgs a) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kTraceBlock);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
     if (d.l2_window_bytes && variant != VARIANT_TWO_WIDE && variant != VARIANT_WARP_VOTE && variant != VARIANT_DYNAMIC) {
         attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
         attr[0].val.accessPolicyWindow.base_ptr = const_cast<char *>(d.view.wide_nodes);
@@ -357,8 +370,11 @@ static cudaError_t launch_variant(const DeviceBVH &d, int variant, unsigned bloc
         attr[0].val.accessPolicyWindow.hitRatio = d.l2_hit_ratio;
         attr[0].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
         attr[0].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
-        cfg.attrs = attr;
         cfg.numAttrs = 1;
+    }
+    if (chained) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
     void *args[] = {&a};
     return cudaLaunchKernelExC(&cfg, kernel_for<kClosest, kExt>(variant), args);
@@ -401,7 +417,6 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
         d_hits = static_cast<char *>(d_hits) + (ext ? sizeof(tt_hit_ext) : sizeof(tt_hit)) * kMaxLaunchRays;
     }
     if (!d.l2_setup) setup_l2_window(const_cast<DeviceBVH &>(d));
-    TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
     TraceArgs a;
     a.bvh = d.view;
     a.rays = reinterpret_cast<const float4 *>(d_rays);
@@ -448,12 +463,17 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     int64_t blocks = (int64_t)d.num_sms * d.blocks_per_sm[variant];
     if (blocks > max_useful) blocks = max_useful;
     if (blocks < 1) blocks = 1;
+    // the four-wide kernels find their counter at 0 and leave it so
+    const bool counts_up = variant == VARIANT_TWO_WIDE || variant == VARIANT_DYNAMIC || variant == VARIANT_WARP_VOTE;
+    if (counts_up) TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
     cudaError_t le;
-    if (closest) le = ext ? launch_variant<true, true>(d, variant, (unsigned)blocks, stream, a)
-                          : launch_variant<true, false>(d, variant, (unsigned)blocks, stream, a);
-    else le = ext ? launch_variant<false, true>(d, variant, (unsigned)blocks, stream, a)
-                  : launch_variant<false, false>(d, variant, (unsigned)blocks, stream, a);
+    const bool chained = order_rays && !counts_up;
+    if (closest) le = ext ? launch_variant<true, true>(d, variant, (unsigned)blocks, chained, stream, a)
+                          : launch_variant<true, false>(d, variant, (unsigned)blocks, chained, stream, a);
+    else le = ext ? launch_variant<false, true>(d, variant, (unsigned)blocks, chained, stream, a)
+                  : launch_variant<false, false>(d, variant, (unsigned)blocks, chained, stream, a);
     TT_CUDA(le);
+    if (counts_up) TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
     return TT_OK;
 }
 
