@@ -608,6 +608,30 @@ __global__ void k_stream_plan(NativeArgs a, int c, int pool, int final) {
     a.ps.counts[c] = alive + (int)n_new;
 }
 
+// Which path takes the place of path g in the refill of the paths [lo, hi): in every whole band of
+// four image rows that lies in the range, 8 x 4 pixel tiles follow one another (a bijection of the
+// range). A warp's rays, and with them its hits and next bounces, then lie closer together than
+// 32 pixels of one row do: 960 x 540 x 16 samples of 400 spheres take 12.7 ms, in row order 13.0. (In
+// waves the state stays in path order, and reading it tile by tile costs more than it gives: the
+// Cornell box at 512 x 512 x 16 3.44 ms against 3.39.)
+__device__ __forceinline__ long long tiled_path(const NativeArgs &a, long long g, long long lo, long long hi) {
+    const ViewRec &vw = a.views ? a.views[find_view(a, g)] : a.view0;
+    const long long l = g - vw.first;
+    const int w = vw.width, p = (int)(l % vw.npix), band = p / (4 * w), r = p - band * 4 * w;
+    const long long b0 = g - r;
+    if ((band + 1) * 4 > vw.height || b0 < lo || b0 + 4ll * w > hi) return g;
+    const int w8 = w & ~7, c = r - 4 * w8;
+    int x, y;
+    if (c < 0) {
+        x = (r >> 5) * 8 + (r & 7);
+        y = (r >> 3) & 3;
+    } else {  // the columns beyond the last whole tile
+        y = c / (w - w8);
+        x = w8 + c - y * (w - w8);
+    }
+    return b0 + (long long)y * w + x;
+}
+
 // The refill: new paths behind the survivors in queue c.
 __global__ void __launch_bounds__(kShadeBlockMax) k_regen(NativeArgs a, int c) {
     chain_begin();
@@ -618,7 +642,7 @@ __global__ void __launch_bounds__(kShadeBlockMax) k_regen(NativeArgs a, int c) {
     const PathState &S = a.stream.st[c];
     CamFrame cc;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const long long g = first + t;
+        const long long g = tiled_path(a, first + t, first, first + n);
         V3 org, dir;
         Rng rg;
         long long gid;
