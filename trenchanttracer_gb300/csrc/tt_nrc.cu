@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "tt_internal.h"
+#include "tt_launch.cuh"
 #include "tt_nrc.cuh"
 #include "tt_nrc_host.h"
 #include "tt_nrc_tc.h"
@@ -440,6 +441,8 @@ __global__ void __launch_bounds__(kThreads) k_mlp_wgrad(WgradArgs a) {
     else wgrad_layer<kHidden, kOutPad>(a, l, n, sm);
 }
 
+constexpr int kAdamBlock = 128;  // 212 blocks: every SM has one
+
 struct AdamArgs {
     const float *partial;
     int chunks;  // partial rows to sum (chunks with no rows hold zeros)
@@ -468,8 +471,17 @@ __device__ __forceinline__ void k_adam_body(const AdamArgs &a) {
     if (i >= kParams) return;
     long long n = a.n_host;
     if (a.n_dev) n = (long long)*a.n_dev - a.off;
+    // in chunk order; the loads of 16 chunks go out together
     float g = 0.0f;
-    for (int c = 0; c < a.chunks; c++) g += a.partial[(size_t)c * kParams + i];
+    int c = 0;
+    for (; c + 16 <= a.chunks; c += 16) {
+        float p[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) p[k] = a.partial[(size_t)(c + k) * kParams + i];
+#pragma unroll
+        for (int k = 0; k < 16; k++) g += p[k];
+    }
+    for (; c < a.chunks; c++) g += a.partial[(size_t)c * kParams + i];
     if (a.grad) a.grad[i] = g;
     if (!a.update || n <= 0) return;
     const int t = a.step[0] + 1;
@@ -496,10 +508,14 @@ __device__ __forceinline__ void k_adam_body(const AdamArgs &a) {
     if (l >= 1) a.w_tcT_train[tcT_index(l, local % layer_in(l), local / layer_in(l))] = *reinterpret_cast<const uint16_t *>(&wb);
 }
 
-__global__ void k_adam(AdamArgs a) { k_adam_body(a); }
+__global__ void k_adam(AdamArgs a) {
+    chain_begin();
+    k_adam_body(a);
+}
 
 // k_adam with the step counter advanced by its last block to finish, once every block has read it
 __global__ void k_adam_update(AdamArgs a) {
+    chain_begin();
     k_adam_body(a);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -660,7 +676,6 @@ tt_status train_pass(tt_cache *c, const float *rec, const float *target, long lo
             t.lo[i] = a.enc.lo[i];
             t.inv_ext[i] = a.enc.inv_ext[i];
         }
-        t.y = c->y;
         for (int l = 0; l < kLayers; l++) {
             t.h[l] = c->h[l];
             t.dz[l] = c->dz[l];
@@ -714,8 +729,8 @@ tt_status train_pass(tt_cache *c, const float *rec, const float *target, long lo
     ad.eps = c->p.eps;
     ad.ema_f = c->p.ema;
     ad.update = update;
-    if (update) k_adam_update<<<(kParams + 255) / 256, 256, 0, s>>>(ad);  // also the tcgen05-layout copies
-    else k_adam<<<(kParams + 255) / 256, 256, 0, s>>>(ad);
+    // k_adam_update also writes the tcgen05-layout copies
+    launch_chained(update ? k_adam_update : k_adam, (kParams + kAdamBlock - 1) / kAdamBlock, kAdamBlock, 0, s, ad);
     TT_CUDA_C(cudaGetLastError());
     return TT_OK;
 }

@@ -1,8 +1,8 @@
 // The radiance cache's network on 5th-generation tensor cores: tcgen05.mma with the FP32
 // accumulator in tensor memory (TMEM), operands in shared memory, weights and feature records
 // brought in by bulk asynchronous copies (cp.async.bulk) that signal an mbarrier. Inference is
-// described here; training (the same forward kernel storing each layer's input, a backward kernel
-// and a weight-gradient kernel) further down.
+// described here; training runs the same kernel with the backward pass behind it, tile by tile, and a
+// weight-gradient kernel (both further down).
 //
 // One CTA per SM, six warpgroups of 128 threads (kTcGroups) sharing one copy of the network's
 // weights (55.3 KB, loaded once per CTA). Each warpgroup owns its own stream of tiles of 128 rows
@@ -40,6 +40,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "tt_launch.cuh"
 #include "tt_nrc.cuh"
 #include "tt_nrc_tc.h"
 
@@ -73,6 +74,12 @@ __host__ __device__ constexpr int tc_tmem_cols(int g) {
     return 64 * g <= 32 ? 32 : (64 * g <= 64 ? 64 : (64 * g <= 128 ? 128 : (64 * g <= 256 ? 256 : 512)));
 }
 constexpr int kTcSmem = tc_smem(kTcGroups);
+// Training: the transposed weights of layers 1..5 as well; five groups per CTA at most.
+constexpr int kTcTWeightBytes = kTcTWeights * 2;  // 34816
+constexpr int kTrainGroups = 1;                   // few tiles: spread over the SMs
+constexpr int kTrainWideGroups = 5;
+__host__ __device__ constexpr int tc_train_smem(int g) { return tc_smem(g) + kTcTWeightBytes; }
+static_assert(tc_train_smem(kTrainWideGroups) <= 232448 && kTcTWeightBytes % 16 == 0, "training shared memory");
 static_assert(kTcSmem <= 232448, "fits the 227 KB a CTA may use");
 static_assert(kTcWeightBytes % 16 == 0 && kABytes % 16 == 0 && kRecBytes % 16 == 0, "bulk copy sizes");
 static_assert(kTmemCols >= 64 * kTcGroups, "64 accumulator columns per group");
@@ -184,9 +191,14 @@ __device__ __forceinline__ void encode_fill(const EncInputs &in, const float *re
     }
 }
 
+__device__ __forceinline__ bool bf16_pos(uint32_t bits16) { return bits16 != 0u && !(bits16 & 0x8000u); }
+
 // ReLU of this thread's 64 accumulator columns, rounded to BF16, into its row of the next A (and,
-// training, into the row of that layer's input H in global memory, gout).
-__device__ __forceinline__ void relu_to_operand(uint32_t lane_addr, __nv_bfloat16 *A, int r, uint4 *gout = nullptr) {
+// training, into the row of that layer's input H in global memory, gout; the result: a bit per
+// column where H > 0).
+template <bool kTrain>
+__device__ __forceinline__ uint64_t relu_to_operand(uint32_t lane_addr, __nv_bfloat16 *A, int r, uint4 *gout) {
+    uint64_t pos = 0;
 #pragma unroll
     for (int c = 0; c < kHidden; c += 16) {
         float v[16];
@@ -197,9 +209,42 @@ __device__ __forceinline__ void relu_to_operand(uint32_t lane_addr, __nv_bfloat1
         for (int j = 0; j < 8; j++) {
             const __nv_bfloat162 b = __floats2bfloat162_rn(fmaxf(v[2 * j], 0.f), fmaxf(v[2 * j + 1], 0.f));
             w[j] = *reinterpret_cast<const uint32_t *>(&b);
+            if (kTrain) {
+                if (bf16_pos(w[j] & 0xffffu)) pos |= 1ull << (c + 2 * j);
+                if (bf16_pos(w[j] >> 16)) pos |= 1ull << (c + 2 * j + 1);
+            }
         }
         *reinterpret_cast<uint4 *>(A + a_offset(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
         *reinterpret_cast<uint4 *>(A + a_offset(r, c + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
+        if (kTrain && gout) {
+            gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
+            gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+    }
+    return pos;
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&b);
+}
+
+// Training: dZ = dH * [H > 0] for this thread's 64 accumulator columns (pos: a bit per column; 0 for
+// a row past the end), into the operand buffer (A != nullptr) and to gout (!= nullptr).
+__device__ __forceinline__ void mask_to_operand(uint32_t lane_addr, uint64_t pos, __nv_bfloat16 *A, int r, uint4 *gout) {
+#pragma unroll
+    for (int c = 0; c < kHidden; c += 16) {
+        float v[16];
+        tmem_ld16(lane_addr + c, v);
+        tmem_wait_ld();
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            w[j] = pack_bf16(pos >> (c + 2 * j) & 1 ? v[2 * j] : 0.0f, pos >> (c + 2 * j + 1) & 1 ? v[2 * j + 1] : 0.0f);
+        if (A) {
+            *reinterpret_cast<uint4 *>(A + a_offset(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4 *>(A + a_offset(r, c + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
+        }
         if (gout) {
             gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
             gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
@@ -215,8 +260,11 @@ struct TcArgs {
     long long off, cap;
     TcEncoding enc;
     float *rgb;         // inference: radiance, 3 per row
-    float *y;           // training: the raw outputs, 3 per row
     uint16_t *h[kLayers];  // training: each layer's input H_l (BF16 rows of 160 or 64)
+    const uint16_t *wT;    // training: transposed operand-layout weights of layers 1..5 (kTcTWeights bf16)
+    const float *target;   // training: 3 per row
+    uint16_t *dz[kLayers]; // training: the loss gradient of each layer's Z_l
+    float *loss;           // training: loss sum over the rows / rows (atomic), or nullptr
     unsigned *err;
     long long wait_cycles;  // budget of the waits in the main path (the drain at exit keeps ~1 s)
 };
@@ -231,24 +279,36 @@ __device__ __forceinline__ void group_sync(int group) {  // the 128 threads of o
     asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
 }
 
-// kTrain: also writes every layer's input H_l and the raw outputs, for the backward pass.
+// kTrain: also writes every layer's input H_l, and goes back through the layers before the next tile.
+// The loss gradient of the row's three outputs (relative L2 loss sum_c (p - t)^2 / (p^2 + 0.01), p =
+// exp(y), the denominator not differentiated, scaled by 1 / rows) is the K = 16 operand dZ_5
+// (columns 3..15 zero). Then for l = 5 .. 1 one product dH_l = dZ_l W_l (M = 128, N = 64, K = 16 or
+// 64, B = the transposed weights, which come in during the forward pass), and the epilogue keeps the
+// columns where H_l > 0, rounds to BF16 and writes dZ_{l-1} to global memory and, but for l = 1, into
+// the operand buffer. Where H_l > 0 stays in registers, 64 bits a layer: a backward kernel of its own
+// loaded its weights, the outputs and every H_l again, one dependent cache access after another
+// (four steps of 16,384 rows, the cache's batch, with the host's copies 257 to 225 us).
 template <bool kTrain, int kG>
 __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
+    chain_begin();
     extern __shared__ __align__(128) uint8_t smem[];
     const int tid = threadIdx.x, group = tid >> 7, gt = tid & 127, warp_in_group = gt >> 5;
     __nv_bfloat16 *A = reinterpret_cast<__nv_bfloat16 *>(smem + group * kABytes);
     uint16_t *W = reinterpret_cast<uint16_t *>(smem + kG * kABytes);
-    float *R = reinterpret_cast<float *>(smem + kG * kABytes + kTcWeightBytes) +
+    constexpr int kWBytes = kTcWeightBytes + (kTrain ? kTcTWeightBytes : 0);
+    uint16_t *WT = W + kTcWeights;  // training
+    float *R = reinterpret_cast<float *>(smem + kG * kABytes + kWBytes) +
                (size_t)group * kRecBufs * kTcRows * kRec;  // this group's record buffers
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kG * (kABytes + kRecBufs * kRecBytes) + kTcWeightBytes);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kG * (kABytes + kRecBufs * kRecBytes) + kWBytes);
     uint64_t *bar_w = bars;                        // weights
     uint64_t *bar_rec = bars + 1 + 5 * group;      // [0] [1]: the group's record buffers
     uint64_t *bar_ring = bar_rec + 2;              // [0] [1]: the products that read each ring slot
     uint64_t *bar_mma = bar_rec + 4;               // the group's hidden and output layers
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 1 + 5 * kG);
+    uint64_t *bar_wT = bars + 1 + 5 * kG;          // training: transposed weights
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 + 5 * kG);
     int *ok_w = reinterpret_cast<int *>(tmem_slot + 1);  // the weights arrived
     int *ok = ok_w + 1 + group;                          // this group's waits all ended
-    static_assert(8 * (1 + 5 * kG) + 4 + 4 * (1 + kG) <= kTcBarBytes, "barrier block");
+    static_assert(8 * (2 + 5 * kG) + 4 + 4 * (1 + kG) <= kTcBarBytes, "barrier block");
 
     const long long n = tc_rows(a.n_host, a.n_dev, a.off, a.cap);
     const long long ntiles = (n + kTcRows - 1) / kTcRows;
@@ -256,6 +316,7 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
 
     if (tid == 0) {
         mbar_init(bar_w, 1);
+        mbar_init(bar_wT, 1);
         for (int g = 0; g < kG; g++) {
             for (int k = 0; k < 5; k++) mbar_init(bars + 1 + 5 * g + k, 1);
             ok_w[1 + g] = 1;
@@ -283,6 +344,10 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
     if (tid == 0) {
         mbar_expect_tx(bar_w, kTcWeightBytes);
         bulk_load(W, a.w, kTcWeightBytes, bar_w);
+        if (kTrain) {  // comes in while the forward pass runs
+            mbar_expect_tx(bar_wT, kTcTWeightBytes);
+            bulk_load(WT, a.wT, kTcTWeightBytes, bar_wT);
+        }
         if (!mbar_wait(bar_w, 0, a.wait_cycles)) {
             *ok_w = 0;
             w_pending = true;
@@ -299,6 +364,8 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
     if (!weights_ok && gt == 0) *ok = 0;
     group_sync(group);
     int buf = 0;
+    const float inv_n = 1.0f / (float)n;
+    float loss = 0.0f;
     for (long long tile = first; weights_ok && tile < ntiles; tile += tstride) {
         const long long r0 = tile * kTcRows;
         const int rows = (int)((n - r0) < kTcRows ? (n - r0) : kTcRows);
@@ -372,12 +439,15 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         tc_fence_after();
         if (!*ok) break;
         // the whole buffer: the ring is no longer read
-        relu_to_operand(lane_addr, A, gt,
-                        kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[1] + (r0 + gt) * kHidden) : nullptr);
+        uint64_t pos[kLayers];  // training: where H_l > 0
+        float y[3] = {0.f, 0.f, 0.f};
+        pos[1] = relu_to_operand<kTrain>(
+            lane_addr, A, gt, kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[1] + (r0 + gt) * kHidden) : nullptr);
         fence_async_smem();
         tc_fence_before();
         group_sync(group);
         tc_fence_after();
+#pragma unroll (kTrain ? kLayers : 1)
         for (int l = 1; l < kLayers; l++) {
             const int K = layer_in(l), N = tc_out(l);
             if (gt == 0) {
@@ -395,32 +465,91 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
             tc_fence_after();
             if (!*ok) break;
             if (l < kLayers - 1) {
-                relu_to_operand(lane_addr, A, gt,
-                                kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[l + 1] + (r0 + gt) * kHidden) : nullptr);
+                pos[l + 1] = relu_to_operand<kTrain>(
+                    lane_addr, A, gt,
+                    kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[l + 1] + (r0 + gt) * kHidden) : nullptr);
                 fence_async_smem();
             } else {
                 float v[16];
                 tmem_ld16(lane_addr, v);
                 tmem_wait_ld();
-                if (gt < rows) {
-                    if (kTrain) {
-                        float *o = a.y + (r0 + gt) * 3;
-                        o[0] = v[0];
-                        o[1] = v[1];
-                        o[2] = v[2];
-                    } else {
-                        float *o = a.rgb + (r0 + gt) * 3;
-                        o[0] = expf(fminf(v[0], 20.0f));
-                        o[1] = expf(fminf(v[1], 20.0f));
-                        o[2] = expf(fminf(v[2], 20.0f));
-                    }
+                if (kTrain) {
+                    y[0] = v[0];
+                    y[1] = v[1];
+                    y[2] = v[2];
+                } else if (gt < rows) {
+                    float *o = a.rgb + (r0 + gt) * 3;
+                    o[0] = expf(fminf(v[0], 20.0f));
+                    o[1] = expf(fminf(v[1], 20.0f));
+                    o[2] = expf(fminf(v[2], 20.0f));
                 }
             }
             tc_fence_before();
             group_sync(group);
             tc_fence_after();
         }
+        if (kTrain) {  // (a group whose wait ran out comes here too: nothing is issued for it)
+            if (!*ok) break;
+            const long long row = r0 + gt;
+            const bool own = gt < rows;
+            float dy[3] = {0.f, 0.f, 0.f};
+            if (own) {
+#pragma unroll
+                for (int c = 0; c < kOut; c++) {
+                    const float p = expf(fminf(y[c], 20.0f));
+                    const float diff = p - a.target[row * 3 + c];
+                    const float den = p * p + 0.01f;
+                    loss += diff * diff / den;
+                    dy[c] = y[c] < 20.0f ? 2.0f * diff / den * p * inv_n : 0.0f;
+                }
+            }
+            const uint4 d5 = make_uint4(pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], 0.0f), 0u, 0u);
+            *reinterpret_cast<uint4 *>(A + a_offset(gt, 0)) = d5;
+            *reinterpret_cast<uint4 *>(A + a_offset(gt, 8)) = make_uint4(0u, 0u, 0u, 0u);
+            if (own) *reinterpret_cast<uint4 *>(a.dz[kLayers - 1] + row * kOutPad) = d5;
+            fence_async_smem();
+            tc_fence_before();
+            group_sync(group);
+            tc_fence_after();
+#pragma unroll
+            for (int l = kLayers - 1; l >= 1; l--) {
+                const int K = tc_out(l), N = layer_in(l);
+                if (gt == 0) {
+                    if (l == kLayers - 1 && !mbar_wait(bar_wT, 0, a.wait_cycles)) {
+                        *ok = 0;  // the transposed weights have not come
+                    } else {
+                        const uint32_t a0 = saddr(A), b0 = saddr(WT + tcT_offset(l));
+                        const uint32_t idesc = idesc_bf16(kTcRows, N);
+                        for (int s2 = 0; s2 < K / 16; s2++)
+                            umma(tmem, sdesc(a0 + s2 * 2 * 2048, 2048, 128),
+                                 sdesc(b0 + s2 * 2 * (N / 8) * 128, (N / 8) * 128, 128), idesc, s2 > 0 ? 1u : 0u);
+                        umma_commit(bar_mma);
+                        mma_issued++;
+                        if (mbar_wait(bar_mma, (uint32_t)(mma_done & 1), a.wait_cycles)) mma_done++;
+                        else *ok = 0;
+                    }
+                }
+                group_sync(group);
+                tc_fence_after();
+                if (!*ok) {
+                    failed = true;
+                    break;
+                }
+                mask_to_operand(lane_addr, own ? pos[l] : 0ull, l > 1 ? A : nullptr, gt,
+                                own ? reinterpret_cast<uint4 *>(a.dz[l - 1] + row * kHidden) : nullptr);
+                fence_async_smem();
+                tc_fence_before();
+                group_sync(group);
+                tc_fence_after();
+            }
+            if (failed) break;
+        }
         buf = (buf + 1) % kRecBufs;
+    }
+    if (kTrain) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        if ((tid & 31) == 0 && a.loss) atomicAdd(a.loss, loss * inv_n);
     }
     if (gt == 0) {
         if (!*ok) atomicOr(a.err, kErrMlpWait);
@@ -433,6 +562,7 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         while (mma_done < mma_issued && mbar_wait(bar_mma, (uint32_t)(mma_done & 1))) mma_done++;
     }
     if (tid == 0 && w_pending) mbar_wait(bar_w, 0);  // the weights copy, if its wait ran out
+    if (kTrain && tid == 0) mbar_wait(bar_wT, 0);    // (complete but for a wait that ran out)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -471,190 +601,6 @@ __global__ void k_tcT_layout(const float *w, uint16_t *out) {
     out[i] = *reinterpret_cast<const uint16_t *>(&b);
 }
 
-// ---- training: backward pass ---------------------------------------------------------------------
-// One warpgroup per tile of 128 rows (six per CTA, as in the forward kernel). Row r of the tile is
-// thread r and TMEM lane r. The loss gradient of the row's three outputs (relative L2 loss
-// sum_c (p - t)^2 / (p^2 + 0.01), p = exp(y), the denominator not differentiated, scaled by
-// 1 / rows) is the K = 16 operand dZ_5 (columns 3..15 zero). Then for l = 5 .. 1 one product
-// dH_l = dZ_l W_l (M = 128, N = 64, K = 16 or 64, B = the transposed weights), and the epilogue
-// reads the row's 64 columns, keeps those where H_l > 0 (the forward pass's stored BF16 input of
-// layer l, i.e. relu(Z_{l-1})), rounds to BF16 and writes dZ_{l-1} to global memory and, but for
-// l = 1, into the operand buffer for the next product. Every dZ row is stored as the weight
-// gradient needs it.
-struct TcBackArgs {
-    const uint16_t *wT;  // transposed operand-layout weights of layers 1..5 (kTcTWeights bf16)
-    const float *y, *target;
-    const uint16_t *h[kLayers];
-    uint16_t *dz[kLayers];
-    float *loss;  // loss sum over the rows / rows (atomic), or nullptr
-    long long n_host;
-    const int *n_dev;
-    long long off, cap;
-    unsigned *err;
-    long long wait_cycles;
-};
-constexpr int kTcTWeightBytes = kTcTWeights * 2;  // 34816
-__host__ __device__ constexpr int tc_back_smem(int g) { return g * kABytes + kTcTWeightBytes + kTcBarBytes; }
-static_assert(tc_back_smem(kTcGroups) <= 232448 && kTcTWeightBytes % 16 == 0, "backward shared memory");
-constexpr int kTrainGroups = 1;  // warpgroups per CTA of the training passes
-
-__device__ __forceinline__ bool bf16_pos(uint32_t bits16) { return bits16 != 0u && !(bits16 & 0x8000u); }
-
-// dZ = dH * [H > 0] for this thread's 64 accumulator columns; H: the row's 64 BF16 values in
-// global memory (nullptr: a row past the end, all zero). Into the operand buffer (A != nullptr)
-// and to gout (!= nullptr).
-__device__ __forceinline__ void mask_to_operand(uint32_t lane_addr, const uint16_t *H, __nv_bfloat16 *A, int r,
-                                                uint4 *gout) {
-#pragma unroll
-    for (int c = 0; c < kHidden; c += 16) {
-        float v[16];
-        tmem_ld16(lane_addr + c, v);
-        tmem_wait_ld();
-        uint4 hv[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-        if (H) {
-            hv[0] = *reinterpret_cast<const uint4 *>(H + c);
-            hv[1] = *reinterpret_cast<const uint4 *>(H + c + 8);
-        }
-        const uint32_t hw[8] = {hv[0].x, hv[0].y, hv[0].z, hv[0].w, hv[1].x, hv[1].y, hv[1].z, hv[1].w};
-        uint32_t w[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float lo = bf16_pos(hw[j] & 0xffffu) ? v[2 * j] : 0.0f;
-            const float hi = bf16_pos(hw[j] >> 16) ? v[2 * j + 1] : 0.0f;
-            const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
-            w[j] = *reinterpret_cast<const uint32_t *>(&b);
-        }
-        if (A) {
-            *reinterpret_cast<uint4 *>(A + a_offset(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4 *>(A + a_offset(r, c + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
-        }
-        if (gout) {
-            gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
-            gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
-    }
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t *>(&b);
-}
-
-template <int kG>
-__global__ void __launch_bounds__(128 * kG, 1) k_mlp_backward_tc(TcBackArgs a) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    const int tid = threadIdx.x, group = tid >> 7, gt = tid & 127, warp_in_group = gt >> 5;
-    __nv_bfloat16 *A = reinterpret_cast<__nv_bfloat16 *>(smem + group * kABytes);
-    uint16_t *W = reinterpret_cast<uint16_t *>(smem + kG * kABytes);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kG * kABytes + kTcTWeightBytes);
-    uint64_t *bar_w = bars;                  // weights
-    uint64_t *bar_mma = bars + 1 + group;    // the group's products
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 1 + kG);
-    int *ok_w = reinterpret_cast<int *>(tmem_slot + 1);
-    int *ok = ok_w + 1 + group;
-    static_assert(8 * (1 + kG) + 4 + 4 * (1 + kG) <= kTcBarBytes, "barrier block");
-
-    const long long n = tc_rows(a.n_host, a.n_dev, a.off, a.cap);
-    const long long ntiles = (n + kTcRows - 1) / kTcRows;
-    if ((long long)blockIdx.x * kG >= ntiles) return;  // uniform per block: nothing allocated yet
-    if (tid == 0) {
-        mbar_init(bar_w, 1);
-        for (int g = 0; g < kG; g++) {
-            mbar_init(bars + 1 + g, 1);
-            ok_w[1 + g] = 1;
-        }
-        *ok_w = 1;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (tid < 32) tmem_alloc(tmem_slot, tc_tmem_cols(kG));
-    bool w_pending = false;
-    if (tid == 0) {
-        mbar_expect_tx(bar_w, kTcTWeightBytes);
-        bulk_load(W, a.wT, kTcTWeightBytes, bar_w);
-        if (!mbar_wait(bar_w, 0, a.wait_cycles)) {
-            *ok_w = 0;
-            w_pending = true;
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot + (uint32_t)(group * 64);
-    const uint32_t lane_addr = tmem + ((uint32_t)(warp_in_group * 32) << 16);
-    const bool weights_ok = *ok_w != 0;
-    if (!weights_ok && gt == 0) *ok = 0;
-    group_sync(group);
-    const float inv_n = 1.0f / (float)n;
-    float loss = 0.0f;
-    int mma_issued = 0, mma_done = 0;
-    const long long tstride = (long long)gridDim.x * kG;
-    for (long long tile = (long long)blockIdx.x * kG + group; weights_ok && tile < ntiles; tile += tstride) {
-        const long long r0 = tile * kTcRows, row = r0 + gt;
-        const bool own = row < n;
-        float dy[3] = {0.f, 0.f, 0.f};
-        if (own) {
-#pragma unroll
-            for (int c = 0; c < kOut; c++) {
-                const float yv = a.y[row * 3 + c];
-                const float p = expf(fminf(yv, 20.0f));
-                const float diff = p - a.target[row * 3 + c];
-                const float den = p * p + 0.01f;
-                loss += diff * diff / den;
-                dy[c] = yv < 20.0f ? 2.0f * diff / den * p * inv_n : 0.0f;
-            }
-        }
-        const uint4 d5 = make_uint4(pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], 0.0f), 0u, 0u);
-        *reinterpret_cast<uint4 *>(A + a_offset(gt, 0)) = d5;
-        *reinterpret_cast<uint4 *>(A + a_offset(gt, 8)) = make_uint4(0u, 0u, 0u, 0u);
-        if (own) *reinterpret_cast<uint4 *>(a.dz[kLayers - 1] + row * kOutPad) = d5;
-        fence_async_smem();
-        tc_fence_before();
-        group_sync(group);
-        tc_fence_after();
-        bool failed = false;
-        for (int l = kLayers - 1; l >= 1; l--) {
-            const int K = tc_out(l), N = layer_in(l);
-            if (gt == 0) {
-                const uint32_t a0 = saddr(A), b0 = saddr(W + tcT_offset(l));
-                const uint32_t idesc = idesc_bf16(kTcRows, N);
-                for (int s2 = 0; s2 < K / 16; s2++)
-                    umma(tmem, sdesc(a0 + s2 * 2 * 2048, 2048, 128), sdesc(b0 + s2 * 2 * (N / 8) * 128, (N / 8) * 128, 128),
-                         idesc, s2 > 0 ? 1u : 0u);
-                umma_commit(bar_mma);
-                mma_issued++;
-                if (mbar_wait(bar_mma, (uint32_t)(mma_done & 1), a.wait_cycles)) mma_done++;
-                else *ok = 0;
-            }
-            group_sync(group);
-            tc_fence_after();
-            if (!*ok) {
-                failed = true;
-                break;
-            }
-            mask_to_operand(lane_addr, own ? a.h[l] + row * kHidden : nullptr, l > 1 ? A : nullptr, gt,
-                            own ? reinterpret_cast<uint4 *>(a.dz[l - 1] + row * kHidden) : nullptr);
-            fence_async_smem();
-            tc_fence_before();
-            group_sync(group);
-            tc_fence_after();
-        }
-        if (failed) break;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-    if ((tid & 31) == 0 && a.loss) atomicAdd(a.loss, loss * inv_n);
-    if (gt == 0) {
-        if (!*ok) atomicOr(a.err, kErrMlpWait);
-        while (mma_done < mma_issued && mbar_wait(bar_mma, (uint32_t)(mma_done & 1))) mma_done++;
-    }
-    if (tid == 0 && w_pending) mbar_wait(bar_w, 0);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (tid < 32) tmem_free(*tmem_slot, tc_tmem_cols(kG));
-}
-
 // ---- training: weight gradients ------------------------------------------------------------------
 // dW_l = dZ_l^T H_l over the batch's rows: one CTA per chunk of rows and layer, a product with
 // M = 128 (the layer's outputs, zero beyond them), N = the layer's inputs (160 or 64) and K = the
@@ -670,11 +616,13 @@ constexpr int kWgMinRows = 256;  // rows per chunk: at least this, more for larg
 constexpr int kWgABytes = kTcRows * kTcRows * 2;  // 128 outputs x 128 rows
 constexpr int kWgBBytes = kIn * kTcRows * 2;      // up to 160 inputs x 128 rows
 constexpr int kWgSmem = kWgABytes + kWgBBytes + 256;
-// requested per CTA, so that at most two CTAs share an SM and their 256 TMEM columns each fit
-constexpr int kWgSmemReq = 80 * 1024;
-static_assert(kWgSmem <= kWgSmemReq && 3 * kWgSmemReq > 232448, "at most two CTAs per SM");
-constexpr int kWgTmemCols = 256;
-constexpr int kWgThreads = 512;  // staging threads; warps 0-3 also read the sums out of TMEM
+// Three CTAs to an SM: the 384 CTAs of a 16,384-row step then run in one round (two to an SM: 1.3
+// rounds), each waiting for its copies while the others work. TMEM: 256 columns for layer 0's 160
+// inputs, 64 for the others; the first CTAs of the grid, layer 0's, go to different SMs, and an
+// allocation that does not fit waits for a neighbour to end. 23 to 16 us a step of 16,384 rows.
+constexpr int kWgPerSm = 3;
+static_assert(kWgPerSm * (kWgSmem + 1024) <= 233472, "three CTAs per SM");
+constexpr int kWgThreads = 384;  // staging threads; warps 0-3 also read the sums out of TMEM
 
 struct TcWgradArgs {
     const uint16_t *h[kLayers];
@@ -688,7 +636,8 @@ struct TcWgradArgs {
     long long wait_cycles;
 };
 
-__global__ void __launch_bounds__(kWgThreads, 1) k_mlp_wgrad_tc(TcWgradArgs a) {
+__global__ void __launch_bounds__(kWgThreads, 3) k_mlp_wgrad_tc(TcWgradArgs a) {
+    chain_begin();
     extern __shared__ __align__(128) uint8_t smem[];
     uint16_t *As = reinterpret_cast<uint16_t *>(smem);
     uint16_t *Bs = reinterpret_cast<uint16_t *>(smem + kWgABytes);
@@ -712,7 +661,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_mlp_wgrad_tc(TcWgradArgs a) {
     for (int i = tid; i < kWgABytes / 16; i += kWgThreads)  // A columns beyond the outputs stay zero
         reinterpret_cast<uint4 *>(As)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    if (tid < 32) tmem_alloc(tmem_slot, kWgTmemCols);
+    const uint32_t tmem_cols = in > 64 ? 256u : 64u;
+    if (tid < 32) tmem_alloc(tmem_slot, tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -765,7 +715,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_mlp_wgrad_tc(TcWgradArgs a) {
             tmem_wait_ld();
             if (m < out)
 #pragma unroll
-                for (int j = 0; j < 16; j++) P[m * in + c + j] = v[j];
+                for (int j = 0; j < 16; j += 4)
+                    *reinterpret_cast<float4 *>(P + m * in + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
         }
     }
     if (tid == 0) {
@@ -775,7 +726,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_mlp_wgrad_tc(TcWgradArgs a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (tid < 32) tmem_free(*tmem_slot, kWgTmemCols);
+    if (tid < 32) tmem_free(*tmem_slot, tmem_cols);
 }
 
 tt_status tc_setup() {
@@ -783,18 +734,12 @@ tt_status tc_setup() {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mlp_forward_tc<true, kTrainGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 tc_smem(kTrainGroups));
+                                 tc_train_smem(kTrainGroups));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_forward_tc<true, kTcGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 tc_smem(kTcGroups));
+        e = cudaFuncSetAttribute(k_mlp_forward_tc<true, kTrainWideGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 tc_train_smem(kTrainWideGroups));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_backward_tc<kTrainGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 tc_back_smem(kTrainGroups));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_backward_tc<kTcGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 tc_back_smem(kTcGroups));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmemReq);
+        e = cudaFuncSetAttribute(k_mlp_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
     if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("tensor-core MLP setup: ") + cudaGetErrorString(e));
     return TT_OK;
 }
@@ -847,34 +792,21 @@ tt_status tc_train(const TcTrainArgs &t, cudaStream_t s) {
         f.enc.lo[i] = t.lo[i];
         f.enc.inv_ext[i] = t.inv_ext[i];
     }
-    f.y = t.y;
-    for (int l = 0; l < kLayers; l++) f.h[l] = t.h[l];
+    for (int l = 0; l < kLayers; l++) {
+        f.h[l] = t.h[l];
+        f.dz[l] = t.dz[l];
+    }
+    f.wT = t.w_tcT;
+    f.target = t.target;
+    f.loss = t.loss;
     f.err = t.err;
     f.wait_cycles = wc;
-    // A batch of fewer tiles than six per SM: one group per block, so that the tiles spread over
-    // every SM (two blocks fit an SM); larger ones: six groups per block, as inference runs.
-    const bool wide = (rows + kTcRows - 1) / kTcRows >= (long long)kTcGroups * t.num_sms;
-    const int grid = wide ? tc_grid(rows, kTcGroups, t.num_sms, 1) : tc_grid(rows, kTrainGroups, t.num_sms, 2);
-    if (wide) k_mlp_forward_tc<true, kTcGroups><<<grid, 128 * kTcGroups, tc_smem(kTcGroups), s>>>(f);
-    else k_mlp_forward_tc<true, kTrainGroups><<<grid, 128 * kTrainGroups, tc_smem(kTrainGroups), s>>>(f);
-    TcBackArgs b;
-    std::memset(&b, 0, sizeof(b));
-    b.wT = t.w_tcT;
-    b.y = t.y;
-    b.target = t.target;
-    for (int l = 0; l < kLayers; l++) {
-        b.h[l] = t.h[l];
-        b.dz[l] = t.dz[l];
-    }
-    b.loss = t.loss;
-    b.n_host = t.n_host;
-    b.n_dev = t.n_dev;
-    b.off = t.off;
-    b.cap = t.cap;
-    b.err = t.err;
-    b.wait_cycles = wc;
-    if (wide) k_mlp_backward_tc<kTcGroups><<<grid, 128 * kTcGroups, tc_back_smem(kTcGroups), s>>>(b);
-    else k_mlp_backward_tc<kTrainGroups><<<grid, 128 * kTrainGroups, tc_back_smem(kTrainGroups), s>>>(b);
+    // A batch of fewer tiles than five per SM: one group per block, so that the tiles spread over
+    // every SM (two blocks fit an SM); larger ones: five groups per block.
+    const bool wide = (rows + kTcRows - 1) / kTcRows >= (long long)kTrainWideGroups * t.num_sms;
+    const int groups = wide ? kTrainWideGroups : kTrainGroups;
+    launch_chained(wide ? k_mlp_forward_tc<true, kTrainWideGroups> : k_mlp_forward_tc<true, kTrainGroups>,
+                   tc_grid(rows, groups, t.num_sms, wide ? 1 : 2), 128 * groups, tc_train_smem(groups), s, f);
     TcWgradArgs w;
     std::memset(&w, 0, sizeof(w));
     for (int l = 0; l < kLayers; l++) {
@@ -889,7 +821,7 @@ tt_status tc_train(const TcTrainArgs &t, cudaStream_t s) {
     w.err = t.err;
     w.wait_cycles = wc;
     w.chunk_rows = tc_wgrad_rows(rows, t.num_sms);
-    k_mlp_wgrad_tc<<<dim3(tc_wgrad_chunks(rows, t.num_sms), kLayers), kWgThreads, kWgSmemReq, s>>>(w);
+    launch_chained(k_mlp_wgrad_tc, dim3(tc_wgrad_chunks(rows, t.num_sms), kLayers), kWgThreads, kWgSmem, s, w);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("tensor-core MLP training: ") + cudaGetErrorString(e));
     return TT_OK;

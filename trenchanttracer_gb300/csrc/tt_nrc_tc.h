@@ -31,8 +31,8 @@ void tcT_relayout(const float *w_f32, uint16_t *w_tcT, cudaStream_t s);
 int tc_wgrad_chunks(long long rows, int num_sms);
 
 // One training pass on the tensor cores over rows [0, rows) of the call (rows = clamp(*n_dev - off,
-// 0, cap) with n_dev set, else n_host): forward (storing each layer's input H_l and the raw
-// outputs y), backward (dZ_l, the loss) and the weight gradients, one partial per chunk of rows.
+// 0, cap) with n_dev set, else n_host): forward and backward (storing each layer's input H_l, the
+// loss gradients dZ_l and the loss) and the weight gradients, one partial per chunk of rows.
 struct TcTrainArgs {
     const uint16_t *w_tc, *w_tcT;
     const float *rec, *target;  // the pass's first row
@@ -40,7 +40,6 @@ struct TcTrainArgs {
     const int *n_dev;
     long long off, cap;
     float lo[3], inv_ext[3];
-    float *y;
     uint16_t *h[6], *dz[6];
     float *loss;
     float *partial;
