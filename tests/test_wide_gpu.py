@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from tests.test_wide_bvh import SCENES, rays_for, soup
-from trenchanttracer_gb300 import BVHCompact, DeviceBVH, Renderer, Scene, make_camera_meta, render_params, scenes
+from trenchanttracer_gb300 import BVHCompact, DeviceBVH, Renderer, Scene, make_camera_meta, render_meta, render_params, scenes
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -72,3 +72,34 @@ def test_ordered_queues_give_the_unordered_image(streamed):
         r.check()
         images.append(acc.cpu().numpy().view(np.uint32))
     assert np.array_equal(*images)
+
+
+@pytest.mark.parametrize("w,h,samples", [(16, 16, 1), (48, 32, 3), (333, 77, 2), (640, 352, 1)])
+def test_compat_frames_do_not_depend_on_overlap_or_size(w, h, samples):
+    """tt_render_compat hands its pixels to the warps that are there: every pixel of the whole 16 x 16 blocks gets
+    its value once a frame, and frames on two streams do not disturb each other."""
+    sc = Scene.from_mesh(scenes.cornell(2))
+    sc.set_env(np.ones((8, 16, 3), F))
+    r = Renderer(DeviceBVH(BVHCompact.build(sc, 1e-5, 1, 8)), sc)
+    away = make_camera_meta(w, h, [0.0, 0.0, 1.55], [0.0, 0.0, 1.0], fov=(45.0, 45.0))  # every ray meets the sky
+    box = make_camera_meta(w, h, [0.0, 0.0, 1.55], [0.0, 0.0, -1.0], fov=(45.0, 45.0))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    accs = [torch.zeros(h, w, 3, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    for k in (0, 1):
+        r.render_compat(box, render_meta(7, samples), accs[k], stream=streams[k].cuda_stream)
+    torch.cuda.synchronize()
+    r.render_compat(box, render_meta(7, samples), accs[2])
+    for _ in range(2):
+        r.render_compat(away, render_meta(7, samples), accs[3])
+    r.check()
+    a, b, c, sky = (x.cpu().numpy() for x in accs)
+    assert np.array_equal(a, b) and np.array_equal(a, c)
+    # rows count from the image's bottom; the blocks cover its top rows and left columns
+    inside = np.zeros((h, w), bool)
+    inside[h - h // 16 * 16:, :w // 16 * 16] = True
+    assert not a[~inside].any() and not sky[~inside].any()
+    one = F(0)
+    for _ in range(samples):  # the samples' sum as the kernel rounds it; the sky counts twice
+        one = F(np.float64(F(2.0)) * np.float64(F(1.0) / F(samples)) + np.float64(one))
+    assert (sky[inside] == one + one).all()

@@ -317,51 +317,45 @@ __device__ __forceinline__ void sample_material(const MaterialRec &m, int kind, 
     }
 }
 
-// renderKernel (src/core/RenderKernel.cu:27-95)
-__device__ V3 radiance(const CompatArgs &a, curandState *rs, RRay ray, uint32_t &err) {
-    V3 mask(1.0f, 1.0f, 1.0f);
-    V3 acc(0.0f, 0.0f, 0.0f);
-    for (int bounce = 0; bounce < 10; bounce++) {
-        const float4 r0 = make_float4(ray.o.x, ray.o.y, ray.o.z, ray.d.x);
-        const float4 r1 = make_float4(ray.d.y, ray.d.z, ray.tmin, ray.tmax);
-        WideStackOf<0, 1, true> stack;
-        const TraceResult tr = traverse_wide<true>(stack, a.bvh, r0, r1, err);
-        RHit hit;
-        hit.distance = tr.t;
-        hit.index = -1;
-        hit.mat = -1;
-        if (tr.addr >= 0) {
-            hit.index = __ldg(a.bvh.tri_idx + tr.addr);
-            hit.mat = (int)__ldg(a.bvh.mat_idx + tr.addr);
-            hit_normal(a.bvh, tr.addr, tr.u, tr.v, hit.normal.x, hit.normal.y, hit.normal.z);
-        }
-        RHit gh;
-        gh.index = -1;
-        gh.mat = -1;
-        gh.distance = ray.tmax;
-        for (int i = 0; i < a.num_geoms; i++) {
-            const GeomRec g = a.geoms[i];
-            if (g.kind == GEOM_SPHERE) gh = sphere_hit(g, ray.o, ray.d, ray.tmax);
-            else if (g.kind == GEOM_PLANE) gh = plane_hit(g, ray.o, ray.d, ray.tmax);
-            if (gh.distance < ray.tmax) {
-                gh.index = i;
-                if (hit_less(gh, hit)) {
-                    gh.mat = g.mat;
-                    hit = gh;
-                }
+// One pass of renderKernel's bounce loop (src/core/RenderKernel.cu:27-95) behind intersect(): whether
+// the path ends here.
+__device__ __forceinline__ bool bounce(const CompatArgs &a, curandState *rs, RRay &ray, const TraceResult &tr, V3 &mask,
+                                       V3 &acc) {
+    RHit hit;
+    hit.distance = tr.t;
+    hit.index = -1;
+    hit.mat = -1;
+    if (tr.addr >= 0) {
+        hit.index = __ldg(a.bvh.tri_idx + tr.addr);
+        hit.mat = (int)__ldg(a.bvh.mat_idx + tr.addr);
+        hit_normal(a.bvh, tr.addr, tr.u, tr.v, hit.normal.x, hit.normal.y, hit.normal.z);
+    }
+    RHit gh;
+    gh.index = -1;
+    gh.mat = -1;
+    gh.distance = ray.tmax;
+    for (int i = 0; i < a.num_geoms; i++) {
+        const GeomRec g = a.geoms[i];
+        if (g.kind == GEOM_SPHERE) gh = sphere_hit(g, ray.o, ray.d, ray.tmax);
+        else if (g.kind == GEOM_PLANE) gh = plane_hit(g, ray.o, ray.d, ray.tmax);
+        if (gh.distance < ray.tmax) {
+            gh.index = i;
+            if (hit_less(gh, hit)) {
+                gh.mat = g.mat;
+                hit = gh;
             }
         }
-        if ((double)hit.distance > 1e19) {
-            acc = r_madd(mask, env_lookup(a, ray.d), acc);
-            return acc;
-        }
-        hit_frame(hit, ray);
-        if (hit.mat < 0 || hit.mat >= a.num_materials) return acc;  // no material: stop the path
-        const MaterialRec m = a.materials[hit.mat];
-        acc = r_madd(mask, V3(m.emission[0], m.emission[1], m.emission[2]), acc);
-        sample_material(m, m.kind, rs, ray, hit, mask);
     }
-    return acc;
+    if ((double)hit.distance > 1e19) {
+        acc = r_madd(mask, env_lookup(a, ray.d), acc);
+        return true;
+    }
+    hit_frame(hit, ray);
+    if (hit.mat < 0 || hit.mat >= a.num_materials) return true;  // no material: stop the path
+    const MaterialRec m = a.materials[hit.mat];
+    acc = r_madd(mask, V3(m.emission[0], m.emission[1], m.emission[2]), acc);
+    sample_material(m, m.kind, rs, ray, hit, mask);
+    return false;
 }
 
 // The primary ray of one sample (src/core/RenderKernel.cu:131-197): jitter and, with an aperture,
@@ -408,30 +402,109 @@ __device__ __forceinline__ RRay camera_ray(const CompatArgs &a, int pixel_x, int
     return ray;
 }
 
-// pathTracingKernel (src/core/RenderKernel.cu:97-206): one thread per pixel, 16x16 blocks.
-__global__ void __launch_bounds__(256) render_compat_kernel(CompatArgs a) {
-    const unsigned x = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int width = a.cam.width;
-    const int height = a.cam.height;
-    const int thread_id = (int)((blockIdx.x + blockIdx.y * gridDim.x) * (blockDim.x * blockDim.y) +
-                                (threadIdx.y * blockDim.x) + threadIdx.x);
-    curandState rs;
-    curand_init((unsigned long long)(a.meta.hashed_frame + (unsigned)thread_id), 0, 0, &rs);
+constexpr int kCompatBounces = 10;  // the reference's bounce loop (src/core/RenderKernel.cu:33)
+constexpr int kCompatBlock = 128;
+constexpr unsigned kCompatChunk = 4;
+constexpr int kCompatBlocks = 5;  // resident blocks per SM it is compiled for (4: +5 %, 6: +2 %, 8: +7 %)
+constexpr int kCompatStack = 8;   // traversal stack entries per thread in shared memory
+
+// pathTracingKernel (src/core/RenderKernel.cu:97-206). The reference runs one thread per pixel in 16 x 16
+// blocks; its thread index seeds the pixel's curand stream, and each pixel's samples and bounces
+// follow one another on that stream. Here that index is a queue: a lane keeps a pixel, a warp
+// steps its lanes' rays together (as trace_queue does), and the lanes whose rays are finished shade them
+// together and go on with their next bounce, sample or pixel. One thread per pixel left 6 of 32
+// lanes busy, waiting for each other's rays, paths and samples: the Cornell box at 640 x 360 x 4 2.17 ms,
+// so 1.81. The shares are fixed (every warps-th run of kCompatChunk pixels; runs of 8, 16 and 32 take
+// 1.85, 1.93 and 2.15 ms), so frames of one renderer may overlap on several streams: a common
+// counter takes 1.76 but would be theirs together.
+__global__ void __launch_bounds__(kCompatBlock, kCompatBlocks) render_compat_kernel(CompatArgs a) {
+    __shared__ uint2 sh_stack[kCompatStack * kCompatBlock];
+    WideStackOf<kCompatStack, kCompatBlock, true> stack;
+    stack.sh = sh_stack + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int blocks_x = a.cam.width / 16;
+    const unsigned n = (unsigned)blocks_x * (unsigned)(a.cam.height / 16) * 256u;
     uint32_t err = 0;
-    V3 final_color(0.0f, 0.0f, 0.0f);
-    const int i = (int)((unsigned)(height - (int)y - 1) * (unsigned)width + x);
-    const int pixel_x = (int)x;
-    const int pixel_y = height - (int)y - 1;
-    for (int s = 0; s < a.meta.samples; s++) {
-        const RRay ray = camera_ray(a, pixel_x, pixel_y, &rs);
-        const V3 L = radiance(a, &rs, ray, err);
-        final_color = r_madd(L, __fdiv_rn(1.0f, (float)a.meta.samples), final_color);
+    // a warp's pixels: every warps-th run of kCompatChunk of them
+    const unsigned warps = gridDim.x * (kCompatBlock / 32), warp = blockIdx.x * (kCompatBlock / 32) + threadIdx.x / 32;
+    unsigned next = 0;
+    bool more = true;       // pixels may be left
+    int left = 0;           // samples of this lane's pixel still to do; 0: no pixel
+    int depth = 0, x = 0, y = 0;
+    curandState rs;
+    RRay ray;
+    V3 mask, acc, final_color;
+    WideState s;
+    s.ref = kWideIdle;
+    for (;;) {
+        const unsigned inner = __ballot_sync(0xffffffffu, s.ref < kWideMark);
+        if (__popc(inner) < kWideInner) {
+            if (__any_sync(0xffffffffu, (int)s.ref < 0)) {
+                if ((int)s.ref < 0) {
+                    wide_leaf<true>(s, a.bvh, make_float4(ray.o.x, ray.o.y, ray.o.z, ray.d.x),
+                                    make_float4(ray.d.y, ray.d.z, ray.tmin, ray.tmax));
+                    wide_pop<true>(s, stack);
+                }
+                continue;
+            }
+            bool fresh = false;  // a new sample starts
+            if (s.ref == kWideDone) {
+                s.ref = kWideIdle;
+                depth++;
+                if (bounce(a, &rs, ray, wide_result(s), mask, acc) || depth == kCompatBounces) {
+                    final_color = r_madd(acc, __fdiv_rn(1.0f, (float)a.meta.samples), final_color);
+                    fresh = true;
+                    if (--left == 0) {
+                        const int i = (int)((unsigned)(a.cam.height - y - 1) * (unsigned)a.cam.width + (unsigned)x);
+                        float *px = a.accum + 3ll * i;
+                        px[0] = __fadd_rn(px[0], final_color.x);
+                        px[1] = __fadd_rn(px[1], final_color.y);
+                        px[2] = __fadd_rn(px[2], final_color.z);
+                    }
+                }
+            }
+            __syncwarp();
+            const unsigned want = __ballot_sync(0xffffffffu, left == 0);
+            if (more && want) {
+                const unsigned j = next + __popc(want & ((1u << lane) - 1u));
+                next += __popc(want);
+                const unsigned id = (j / kCompatChunk * warps + warp) * kCompatChunk + j % kCompatChunk;
+                more = (next / kCompatChunk * warps + warp) * kCompatChunk < n;
+                if (left == 0 && id < n) {
+                    const int block = (int)(id / 256u), t = (int)(id % 256u);
+                    x = block % blocks_x * 16 + t % 16;
+                    y = block / blocks_x * 16 + t / 16;
+                    curand_init((unsigned long long)(a.meta.hashed_frame + id), 0, 0, &rs);
+                    final_color = V3(0.0f, 0.0f, 0.0f);
+                    left = a.meta.samples;
+                    fresh = true;
+                }
+            }
+            if (left > 0 && s.ref == kWideIdle) {
+                if (fresh) {
+                    ray = camera_ray(a, x, a.cam.height - y - 1, &rs);
+                    mask = V3(1.0f, 1.0f, 1.0f);
+                    acc = V3(0.0f, 0.0f, 0.0f);
+                    depth = 0;
+                }
+                const float4 r0 = make_float4(ray.o.x, ray.o.y, ray.o.z, ray.d.x);
+                const float4 r1 = make_float4(ray.d.y, ray.d.z, ray.tmin, ray.tmax);
+                if (!wide_start(s, a.bvh, r0, r1)) {
+                    const TraceResult tr = traverse_two_wide<true>(a.bvh, r0, r1, err);
+                    s.t = tr.t;
+                    s.u = tr.u;
+                    s.v = tr.v;
+                    s.addr = tr.addr;
+                    s.ref = kWideDone;
+                }
+            }
+            if (!__any_sync(0xffffffffu, left > 0)) break;
+        }
+        if (s.ref < kWideMark) {
+            wide_node<true>(s, stack, a.bvh);
+            wide_pop<true>(s, stack);
+        }
     }
-    float *px = a.accum + 3ll * i;
-    px[0] = __fadd_rn(px[0], final_color.x);
-    px[1] = __fadd_rn(px[1], final_color.y);
-    px[2] = __fadd_rn(px[2], final_color.z);
     if (err) atomicOr(a.err, err);
 }
 
@@ -594,9 +667,10 @@ tt_status tt_render_compat(tt_renderer *r, const tt_camera_meta *cam, const tt_r
     a.meta = *meta;
     a.accum = d_accum;
     a.err = r->err;
-    dim3 block(16, 16, 1);
-    dim3 grid(cam->width / 16, cam->height / 16, 1);
-    render_compat_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(a);
+    const long long pixels = (long long)(cam->width / 16) * (cam->height / 16) * 256;
+    const long long blocks = std::min<long long>((pixels + kCompatBlock - 1) / kCompatBlock,
+                                                 (long long)r->num_sms * kCompatBlocks);
+    render_compat_kernel<<<(unsigned)blocks, kCompatBlock, 0, (cudaStream_t)stream>>>(a);
     TT_CUDA_R(cudaGetLastError());
     return TT_OK;
 }
