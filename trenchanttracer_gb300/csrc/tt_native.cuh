@@ -51,16 +51,18 @@ struct ViewRec {
     float aperture, focal;  // thin lens (aperture <= 1e-5: pinhole)
 };
 
+// A path's state in two 16-byte words and the generator's two (one load and one store each; as seven
+// arrays of 4 to 12 bytes a path the shade stage spent its time on load and store instructions):
+//   bp   throughput, last BSDF pdf
+//   lf   radiance so far, depth and flags (pack_depth)
+//   rng  PCG32 state, stream increment
 struct PathSoA {
-    float *beta, *L;     // 3 per path
-    uint64_t *rng;       // PCG32 state
-    uint64_t *rng_inc;   // PCG32 stream increment
-    float *last_pdf;
-    int *depth, *flags;
+    float4 *bp, *lf;
+    ulonglong2 *rng;
     int *queue[2];       // path index per queue slot, by bounce parity
     float4 *ray[2];      // 2 float4 per queue slot, by bounce parity
-    float *hit_t, *hit_u, *hit_v;  // per slot of the queue being shaded
-    int *hit_prim;       // triangle slot >= 0, -(geometry+2) for analytic objects, -1 = miss
+    float4 *hit;         // t, u, v, primitive per slot of the queue being shaded: triangle slot >= 0,
+                         // -(geometry+2) for analytic objects, -1 = miss
     int *counts;         // [0] [1] queue lengths by parity, [2] shadow queue length,
                          // [3] extend work counter, [4] shadow work counter
     int *shadow_path;
@@ -119,12 +121,15 @@ struct ShadowOrderView {
 
 // Path state by index: the state slot of a path in waves, the queue slot in a streamed render.
 struct PathState {
-    float *beta, *L;  // 3 per path
-    float *last_pdf;
-    uint64_t *rng, *rng_inc;
-    int *depth, *flags;
+    float4 *bp, *lf;
+    ulonglong2 *rng;
     long long *g;     // streamed renders: the path's index
 };
+__device__ __forceinline__ float pack_depth(int depth, int flags) { return __int_as_float(depth << 4 | flags); }
+__device__ __forceinline__ void unpack_depth(float w, int &depth, int &flags) {
+    depth = __float_as_int(w) >> 4;
+    flags = __float_as_int(w) & 15;
+}
 
 // Streamed render: a pool of wave_paths queue slots that is refilled with the next paths of the
 // index space as paths end, so every bounce launch works on a full pool and the few long paths

@@ -15,6 +15,10 @@ namespace tt {
 
 using namespace pt;
 
+// trace_queue's lanes at inner nodes below which a warp turns to leaves and new rays: the Cornell box at
+// 512 x 512 x 16 takes 3.39 ms with 8, 3.33 with 10, 3.30 with 12; 12 views of a terrain 2.59, 2.58 and 2.65.
+constexpr int kQueueInner = 10;
+
 // kPrefix: the ordering covers only the queue's first *n_sorted slots (a streamed render's
 // survivors); the rest is traced in place. Without it an ordered queue is ordered whole.
 template <int kBlock, int kSh, bool kPrefix>
@@ -34,7 +38,7 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
     // an ordered queue prefix: hits by place, moved back by k_order_gather_hits
     const bool ordered = a.order.src && order_built(a.order.state);
     const int n_sorted = ordered ? (kPrefix ? *a.order.n_sorted : n) : 0;
-    trace_queue<true, kWideInner>(
+    trace_queue<true, kQueueInner>(
         stack, a.bvh, (unsigned)n, err,
         [&](int count) {
             int base = 0;
@@ -58,14 +62,9 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
                 const float4 r0 = a.ps.ray[cur][2 * (size_t)q], r1 = a.ps.ray[cur][2 * (size_t)q + 1];
                 analytic_hit(a, lanes, true, V3(r0.x, r0.y, r0.z), V3(r0.w, r1.x, r1.y), r1.z, t, prim, hu, hv, false);
             }
-            if (kPrefix ? (int)q < n_sorted : ordered) {
-                a.order.hits[a.order.pos[q]] = make_float4(t, hu, hv, __int_as_float(prim));
-            } else {
-                a.ps.hit_t[q] = t;
-                a.ps.hit_prim[q] = prim;
-                a.ps.hit_u[q] = hu;
-                a.ps.hit_v[q] = hv;
-            }
+            const float4 h = make_float4(t, hu, hv, __int_as_float(prim));
+            if (kPrefix ? (int)q < n_sorted : ordered) a.order.hits[a.order.pos[q]] = h;
+            else a.ps.hit[q] = h;
         });
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.stats + 0, (unsigned long long)n);
     if (err) atomicOr(a.err, err);
@@ -82,7 +81,7 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
     stack.sh = sh_stack + threadIdx.x;
     uint32_t err = 0;
     const bool ordered = a.shadow_order.src && order_built(a.shadow_order.state);
-    trace_queue<false, kWideInner>(
+    trace_queue<false, kQueueInner>(
         stack, a.bvh, (unsigned)n, err,
         [&](int count) {
             int base = 0;
@@ -109,14 +108,22 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
                 blocked = blocked || prim != -1;
             }
             if (!blocked) {
-                // a path's radiance: L[3 * t] for t >= 0, else (an ended path of a streamed
+                // a path's radiance: state slot t for t >= 0, else (an ended path of a streamed
                 // render) ring entry -1 - t
                 const int t = a.ps.shadow_path[j];
-                float *L = t >= 0 ? a.ps.L + 3ll * t : a.stream.ring + 3ll * (-1ll - t);
                 const float *c = a.ps.shadow_val + 3ll * j;
-                L[0] = PT_ADD(L[0], c[0]);
-                L[1] = PT_ADD(L[1], c[1]);
-                L[2] = PT_ADD(L[2], c[2]);
+                if (t >= 0) {
+                    float4 L = a.ps.lf[t];
+                    L.x = PT_ADD(L.x, c[0]);
+                    L.y = PT_ADD(L.y, c[1]);
+                    L.z = PT_ADD(L.z, c[2]);
+                    a.ps.lf[t] = L;
+                } else {
+                    float *L = a.stream.ring + 3ll * (-1ll - t);
+                    L[0] = PT_ADD(L[0], c[0]);
+                    L[1] = PT_ADD(L[1], c[1]);
+                    L[2] = PT_ADD(L[2], c[2]);
+                }
             }
         });
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.stats + 1, (unsigned long long)n);
@@ -131,13 +138,9 @@ __global__ void __launch_bounds__(256) k_order_gather_hits(NativeArgs a, int cur
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int p = __ldcs(a.order.pos + i);
         if ((unsigned)p < (unsigned)n) {
-            const float4 h = a.order.hits[p];
-            a.ps.hit_t[i] = h.x;
-            a.ps.hit_u[i] = h.y;
-            a.ps.hit_v[i] = h.z;
-            a.ps.hit_prim[i] = __float_as_int(h.w);
+            a.ps.hit[i] = a.order.hits[p];
         } else {  // not reachable with a consistent ordering: report, and let the path miss
-            a.ps.hit_prim[i] = -1;
+            a.ps.hit[i] = make_float4(1e20f, 0.0f, 0.0f, __int_as_float(-1));
             bad = 1;
         }
     }

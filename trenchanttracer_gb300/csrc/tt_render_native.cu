@@ -446,11 +446,12 @@ __global__ void __launch_bounds__(kShadeBlockMax) k_cache_resolve(NativeArgs a) 
     chain_begin();
     const int n = a.cache.counts[0];
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        float *L = a.ps.L + 3ll * a.cache.q_path[q];
+        float4 L = a.ps.lf[a.cache.q_path[q]];
         const float *b = a.cache.q_beta + 3ll * q, *c = a.cache.q_rgb + 3ll * q;
-        L[0] = PT_FMA(b[0], c[0], L[0]);
-        L[1] = PT_FMA(b[1], c[1], L[1]);
-        L[2] = PT_FMA(b[2], c[2], L[2]);
+        L.x = PT_FMA(b[0], c[0], L.x);
+        L.y = PT_FMA(b[1], c[1], L.y);
+        L.z = PT_FMA(b[2], c[2], L.z);
+        a.ps.lf[a.cache.q_path[q]] = L;
     }
 }
 
@@ -459,7 +460,8 @@ __global__ void __launch_bounds__(kShadeBlockMax) k_cache_targets(NativeArgs a) 
     chain_begin();
     const int n = min(a.cache.counts[1], a.cache.train_cap);
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const float *L = a.ps.L + 3ll * a.cache.t_path[s];
+        const float4 lf = a.ps.lf[a.cache.t_path[s]];
+        const float L[3] = {lf.x, lf.y, lf.z};
         for (int c = 0; c < 3; c++) {
             const float b = a.cache.t_beta[3ll * s + c];
             const float v = b > 0.0f ? PT_DIV(PT_SUB(L[c], a.cache.t_L[3ll * s + c]), b) : 0.0f;
@@ -517,20 +519,16 @@ __device__ __forceinline__ void camera_path(const NativeArgs &a, long long g, Ca
 }
 
 __device__ __forceinline__ PathState wave_state(const PathSoA &ps) {
-    return PathState{ps.beta, ps.L, ps.last_pdf, ps.rng, ps.rng_inc, ps.depth, ps.flags, nullptr};
+    return PathState{ps.bp, ps.lf, ps.rng, nullptr};
 }
 
 // A new path in state slot i, its camera ray in slot q of `rays`.
 __device__ __forceinline__ void start_path(const PathState &S, int i, float4 *rays, int q, const V3 &org,
                                            const V3 &dir, const Rng &rg, int flags) {
     put_ray(rays, q, org, dir);
-    st3(S.beta + 3ll * i, V3(1.f, 1.f, 1.f));
-    st3(S.L + 3ll * i, V3(0.f, 0.f, 0.f));
-    S.rng[i] = rg.state;
-    S.rng_inc[i] = rg.inc;
-    S.last_pdf[i] = 0.0f;
-    S.depth[i] = 0;
-    S.flags[i] = flags;
+    S.bp[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    S.lf[i] = make_float4(0.0f, 0.0f, 0.0f, pack_depth(0, flags));
+    S.rng[i] = make_ulonglong2(rg.state, rg.inc);
 }
 
 // Camera rays of the wave's paths into queue 0.
@@ -685,15 +683,17 @@ __device__ __forceinline__ void shade_queue(const NativeArgs &a, int cur) {
             i = kStream ? q : a.ps.queue[cur][q];
             if (kStream) pg = (cur ? a.stream.st[1].g : a.stream.st[0].g)[i];
             Rng g;
-            g.state = TT_ST(rng)[i];
-            g.inc = TT_ST(rng_inc)[i];
+            const ulonglong2 rng = TT_ST(rng)[i];
+            g.state = rng.x;
+            g.inc = rng.y;
             const float4 r0 = a.ps.ray[cur][2 * q], r1 = a.ps.ray[cur][2 * q + 1];
             const V3 o(r0.x, r0.y, r0.z), d(r0.w, r1.x, r1.y);
-            V3 beta = ld3(TT_ST(beta) + 3ll * i), L = ld3(TT_ST(L) + 3ll * i);
-            const int prim = a.ps.hit_prim[q];
-            int flags = TT_ST(flags)[i];
-            const float last_pdf = TT_ST(last_pdf)[i];
-            int depth = TT_ST(depth)[i];
+            const float4 bp = TT_ST(bp)[i], lf = TT_ST(lf)[i], hit = a.ps.hit[q];
+            V3 beta(bp.x, bp.y, bp.z), L(lf.x, lf.y, lf.z);
+            const float last_pdf = bp.w;
+            int depth, flags;
+            unpack_depth(lf.w, depth, flags);
+            const int prim = __float_as_int(hit.w);
             if (prim == -1) {
                 if (use_env) {
                     const int texel = env_texel(a.env, d);
@@ -706,12 +706,12 @@ __device__ __forceinline__ void shade_queue(const NativeArgs &a, int cur) {
                     L = madd(mul(beta, le), w, L);
                 }
             } else {
-                const float t = a.ps.hit_t[q];
+                const float t = hit.x;
                 const V3 p = madd(d, t, o);
                 V3 n;
                 int mat;
                 if (prim >= 0) {
-                    hit_normal(a.bvh, prim, a.ps.hit_u[q], a.ps.hit_v[q], n.x, n.y, n.z);
+                    hit_normal(a.bvh, prim, hit.y, hit.z, n.x, n.y, n.z);
                     mat = (int)__ldg(a.bvh.mat_idx + prim);
                 } else {
                     const GeomRec g2 = a.geoms[-prim - 2];
@@ -777,15 +777,8 @@ __device__ __forceinline__ void shade_queue(const NativeArgs &a, int cur) {
                         const V3 off = dot(bs.wi, nl) >= 0.0f ? nl : V3(-nl.x, -nl.y, -nl.z);
                         next_o = madd(off, eps, p);
                         next_d = bs.wi;
-                        if (kStream) {
-                            pdf_next = bs.pdf;
-                            flags_next = (flags & kFlagsKept) | ((bs.specular || !nee) ? kFlagSpecular : 0);
-                        } else {
-                            st3(TT_ST(beta) + 3ll * i, beta);
-                            TT_ST(last_pdf)[i] = bs.pdf;
-                            TT_ST(flags)[i] = (flags & kFlagsKept) | ((bs.specular || !nee) ? kFlagSpecular : 0);
-                            TT_ST(depth)[i] = depth;
-                        }
+                        pdf_next = bs.pdf;
+                        flags_next = (flags & kFlagsKept) | ((bs.specular || !nee) ? kFlagSpecular : 0);
                     }
                 }
             }
@@ -796,8 +789,9 @@ __device__ __forceinline__ void shade_queue(const NativeArgs &a, int cur) {
                 out_inc = g.inc;
                 out_depth = depth;
             } else {
-                st3(TT_ST(L) + 3ll * i, L);
-                TT_ST(rng)[i] = g.state;
+                if (alive) TT_ST(bp)[i] = make_float4(beta.x, beta.y, beta.z, pdf_next);
+                TT_ST(lf)[i] = make_float4(L.x, L.y, L.z, pack_depth(depth, flags_next));
+                TT_ST(rng)[i].x = g.state;
             }
         }
         const int slot = warp_append(a.ps.counts + (cur ^ 1), alive);
@@ -806,13 +800,9 @@ __device__ __forceinline__ void shade_queue(const NativeArgs &a, int cur) {
             put_ray(a.ps.ray[cur ^ 1], slot, next_o, next_d);
             if (kStream) {
                 const PathState &N = cur ? a.stream.st[0] : a.stream.st[1];
-                st3(N.beta + 3ll * slot, out_beta);
-                st3(N.L + 3ll * slot, out_L);
-                N.rng[slot] = out_rng;
-                N.rng_inc[slot] = out_inc;
-                N.last_pdf[slot] = pdf_next;
-                N.flags[slot] = flags_next;
-                N.depth[slot] = out_depth;
+                N.bp[slot] = make_float4(out_beta.x, out_beta.y, out_beta.z, pdf_next);
+                N.lf[slot] = make_float4(out_L.x, out_L.y, out_L.z, pack_depth(out_depth, flags_next));
+                N.rng[slot] = make_ulonglong2(out_rng, out_inc);
                 N.g[slot] = pg;
             }
         }
@@ -823,7 +813,7 @@ __device__ __forceinline__ void shade_queue(const NativeArgs &a, int cur) {
         }
         const int sslot = warp_append(a.ps.counts + 2, shadow);
         if (shadow) {
-            // the shadow stage adds to L[3 * t] of the state it is given for t >= 0, else to ring
+            // the shadow stage adds to slot t of the state it is given for t >= 0, else to ring
             // entry -1 - t
             a.ps.shadow_path[sslot] = !kStream ? i : (alive ? slot : (int)(-1 - ring_e));
             put_ray(a.ps.shadow_ray, sslot, sh_o, sh_d);
@@ -854,10 +844,9 @@ __global__ void __launch_bounds__(kShadeBlockMax) k_shade_stream(NativeArgs a, i
 // Adds the radiance of paths [first, first + n) to the views' accumulation blocks. The thread of
 // a pixel's first path in the range adds all of that pixel's paths in the range, in sample order,
 // so the sums do not depend on how a render is cut into ranges. kRing: path g's radiance is at
-// ring entry g mod ring_n, else at L[g - first].
+// ring entry g mod ring_n, else in state slot g - first.
 template <typename T, bool kRing>
-__device__ __forceinline__ void accumulate_range(const NativeArgs &a, T *accum, long long first, long long n,
-                                                 const float *L) {
+__device__ __forceinline__ void accumulate_range(const NativeArgs &a, T *accum, long long first, long long n) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const long long g = first + i;
@@ -868,10 +857,17 @@ __device__ __forceinline__ void accumulate_range(const NativeArgs &a, T *accum, 
         T *px = accum + vw.accum + 3 * pixel;
         T acc[3] = {px[0], px[1], px[2]};
         for (long long k = i, lk = l; k < n && lk < vw.paths; k += vw.npix, lk += vw.npix) {
-            const long long e = kRing ? (first + k) % a.stream.ring_n : k;
-            acc[0] += (T)L[3 * e];
-            acc[1] += (T)L[3 * e + 1];
-            acc[2] += (T)L[3 * e + 2];
+            if (kRing) {
+                const float *L = a.stream.ring + 3 * ((first + k) % a.stream.ring_n);
+                acc[0] += (T)L[0];
+                acc[1] += (T)L[1];
+                acc[2] += (T)L[2];
+            } else {
+                const float4 L = a.ps.lf[k];
+                acc[0] += (T)L.x;
+                acc[1] += (T)L.y;
+                acc[2] += (T)L.z;
+            }
         }
         px[0] = acc[0];
         px[1] = acc[1];
@@ -882,14 +878,14 @@ __device__ __forceinline__ void accumulate_range(const NativeArgs &a, T *accum, 
 template <typename T>
 __global__ void __launch_bounds__(kShadeBlockMax) k_accumulate(NativeArgs a, T *accum) {
     chain_begin();
-    accumulate_range<T, false>(a, accum, a.wave_first, a.wave_paths, a.ps.L);
+    accumulate_range<T, false>(a, accum, a.wave_first, a.wave_paths);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kShadeBlockMax) k_accumulate_stream(NativeArgs a, T *accum) {
     chain_begin();
     const long long lo = a.stream.plan->acc_lo, hi = a.stream.plan->acc_hi;
-    accumulate_range<T, true>(a, accum, lo, hi - lo, a.stream.ring);
+    accumulate_range<T, true>(a, accum, lo, hi - lo);
 }
 
 }  // namespace tt
@@ -1141,10 +1137,10 @@ void native_release(tt_renderer *r) {
 // the pointers, which captured graphs hold, change only when the allocation does).
 static tt_status ensure_paths(tt_renderer *r, int cap, PathSoA &ps) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    constexpr int kArrays = 21;
+    constexpr int kArrays = 14;
     auto layout = [&](size_t n, size_t *sizes) {
-        const size_t s[kArrays] = {12 * n, 12 * n, 8 * n, 8 * n,  4 * n,  4 * n, 4 * n, 4 * n, 4 * n, 32 * n, 32 * n,
-                                   4 * n,  4 * n,  4 * n, 4 * n, 64,     4 * n, 32 * n, 12 * n, 4 * n, 4 * n};
+        const size_t s[kArrays] = {16 * n, 16 * n, 16 * n, 4 * n, 4 * n,  32 * n, 32 * n,
+                                   16 * n, 64,     4 * n,  32 * n, 12 * n, 4 * n,  4 * n};
         size_t total = 0;
         for (int i = 0; i < kArrays; i++) {
             sizes[i] = s[i];
@@ -1183,27 +1179,20 @@ static tt_status ensure_paths(tt_renderer *r, int cap, PathSoA &ps) {
         v[i] = p;
         p += al(sizes[i]);
     }
-    ps.beta = (float *)v[0];
-    ps.L = (float *)v[1];
-    ps.rng = (uint64_t *)v[2];
-    ps.rng_inc = (uint64_t *)v[3];
-    ps.last_pdf = (float *)v[4];
-    ps.depth = (int *)v[5];
-    ps.flags = (int *)v[6];
-    ps.queue[0] = (int *)v[7];
-    ps.queue[1] = (int *)v[8];
-    ps.ray[0] = (float4 *)v[9];
-    ps.ray[1] = (float4 *)v[10];
-    ps.hit_t = (float *)v[11];
-    ps.hit_u = (float *)v[12];
-    ps.hit_v = (float *)v[13];
-    ps.hit_prim = (int *)v[14];
-    ps.counts = (int *)v[15];
-    ps.shadow_path = (int *)v[16];
-    ps.shadow_ray = (float4 *)v[17];
-    ps.shadow_val = (float *)v[18];
-    ps.a0 = (float *)v[19];
-    ps.spread = (float *)v[20];
+    ps.bp = (float4 *)v[0];
+    ps.lf = (float4 *)v[1];
+    ps.rng = (ulonglong2 *)v[2];
+    ps.queue[0] = (int *)v[3];
+    ps.queue[1] = (int *)v[4];
+    ps.ray[0] = (float4 *)v[5];
+    ps.ray[1] = (float4 *)v[6];
+    ps.hit = (float4 *)v[7];
+    ps.counts = (int *)v[8];
+    ps.shadow_path = (int *)v[9];
+    ps.shadow_ray = (float4 *)v[10];
+    ps.shadow_val = (float *)v[11];
+    ps.a0 = (float *)v[12];
+    ps.spread = (float *)v[13];
     return TT_OK;
 }
 
@@ -1448,10 +1437,9 @@ static long long stream_ring_entries(long long pool, int max_depth) {
 // indices.
 static tt_status ensure_stream(tt_renderer *r, const PathSoA &ps, long long pool, long long ring, StreamView &sv) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    constexpr int kArrays = 11;
+    constexpr int kArrays = 7;
     const size_t P = (size_t)pool;
-    const size_t sizes[kArrays] = {12ull * (size_t)ring, 12 * P, 12 * P, 4 * P, 8 * P, 8 * P, 4 * P, 4 * P,
-                                   8 * P, 8 * P, sizeof(StreamPlan)};
+    const size_t sizes[kArrays] = {12ull * (size_t)ring, 16 * P, 16 * P, 16 * P, 8 * P, 8 * P, sizeof(StreamPlan)};
     size_t need = 0;
     for (size_t x : sizes) need += al(x);
     if (r->stream_bytes < need) {
@@ -1471,10 +1459,9 @@ static tt_status ensure_stream(tt_renderer *r, const PathSoA &ps, long long pool
     }
     sv.ring = (float *)v[0];
     sv.ring_n = ring;
-    sv.st[0] = PathState{ps.beta, ps.L, ps.last_pdf, ps.rng, ps.rng_inc, ps.depth, ps.flags, (long long *)v[8]};
-    sv.st[1] = PathState{(float *)v[1], (float *)v[2], (float *)v[3], (uint64_t *)v[4], (uint64_t *)v[5],
-                         (int *)v[6], (int *)v[7], (long long *)v[9]};
-    sv.plan = (StreamPlan *)v[10];
+    sv.st[0] = PathState{ps.bp, ps.lf, ps.rng, (long long *)v[4]};
+    sv.st[1] = PathState{(float4 *)v[1], (float4 *)v[2], (ulonglong2 *)v[3], (long long *)v[5]};
+    sv.plan = (StreamPlan *)v[6];
     return TT_OK;
 }
 
@@ -1530,7 +1517,7 @@ static tt_status issue_stream(NativeArgs a, long long total, const Launch &L, co
             if (st != TT_OK) return st;
         }
         NativeArgs as = a;  // shadow rays of survivors add to their state in the next queue
-        as.ps.L = sv.st[c ^ 1].L;
+        as.ps.lf = sv.st[c ^ 1].lf;
         launch_chained(L.tk.shadow, L.grid_trace, L.block, 0, s, as);
     }
     TT_CUDA_N(cudaGetLastError());
