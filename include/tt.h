@@ -225,10 +225,10 @@ tt_status tt_trace(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_hit *
 /* as tt_trace, writing the full hit record (material index and interpolated normal). */
 tt_status tt_trace_ext(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_hit_ext *d_hits,
                        int32_t closest, void *stream);
-/* as tt_trace with HOST buffers: copies rays in, traces and copies hits out on `stream`
- * through a device staging area owned by `bvh`, and synchronises the stream before returning
- * (page-locked host buffers get full copy bandwidth). Returns the device error word like
- * tt_dbvh_check. */
+/* as tt_trace with HOST buffers; synchronises the stream before returning. Page-locked, device-mapped
+ * buffers (rays 16-byte, hits 8-byte aligned) are read and written by the trace itself across the
+ * host link; others are copied through a device staging area owned by `bvh`. Returns the device
+ * error word like tt_dbvh_check. */
 tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_hit *h_hits,
                         int32_t closest, void *stream);
 /* Synchronises `stream`, then reads and clears the device error word that tt_trace /

@@ -103,3 +103,22 @@ def test_compat_frames_do_not_depend_on_overlap_or_size(w, h, samples):
     for _ in range(samples):  # the samples' sum as the kernel rounds it; the sky counts twice
         one = F(np.float64(F(2.0)) * np.float64(F(1.0) / F(samples)) + np.float64(one))
     assert (sky[inside] == one + one).all()
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_page_locked_host_rays(offset):
+    """Page-locked rays and hits go through the mapped buffers, rays and hits that start off a 16- or 8-byte
+    boundary through staging; the hits are those of device rays either way."""
+    sc, alpha, leaf, extent = SCENES["spheres"]()
+    dbvh = DeviceBVH(BVHCompact.build(sc, alpha, 1, leaf))
+    for n in (1, 33, 5000, 70001):
+        rays = rays_for(extent, 21, n)
+        h_rays = torch.empty(8 * n + 4).pin_memory().numpy()[offset:offset + 8 * n].reshape(n, 8)
+        h_hits = torch.empty(2 * n + 4, dtype=torch.int32).pin_memory().numpy()[offset:offset + 2 * n].reshape(n, 2)
+        h_rays[:] = rays
+        for closest in (True, False):
+            h_hits[:] = 77
+            dbvh.intersect_host(h_rays, h_hits, closest=closest)
+            want = hits(dbvh, torch.from_numpy(rays).cuda(), DeviceBVH.VARIANT_DYNAMIC, closest, False)
+            dbvh.set_variant(DeviceBVH.VARIANT_SORTED)
+            assert np.array_equal(h_hits, want), (n, closest)

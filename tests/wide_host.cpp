@@ -12,6 +12,7 @@
 struct float4 { float x, y, z, w; };
 struct uint4 { uint32_t x, y, z, w; };
 struct uint2 { uint32_t x, y; };
+static inline float4 make_float4(float a, float b, float c, float d) { return float4{a, b, c, d}; }
 static inline uint2 make_uint2(uint32_t a, uint32_t b) { return uint2{a, b}; }
 template <class T> static inline T __ldg(const T *p) { return *p; }
 static inline int __float_as_int(float f) { int i; memcpy(&i, &f, 4); return i; }

@@ -34,12 +34,13 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
     const int lane = threadIdx.x & 31;
     WideStackOf<kSh, kBlock, true> stack;
     stack.sh = sh_stack + threadIdx.x;
+    WideRays<0> rays;
     uint32_t err = 0;
     // an ordered queue prefix: hits by place, moved back by k_order_gather_hits
     const bool ordered = a.order.src && order_built(a.order.state);
     const int n_sorted = ordered ? (kPrefix ? *a.order.n_sorted : n) : 0;
     trace_queue<true, kQueueInner>(
-        stack, a.bvh, (unsigned)n, err,
+        stack, rays, a.bvh, (unsigned)n, err,
         [&](int count) {
             int base = 0;
             if (lane == 0) base = atomicAdd(a.ps.counts + 3, count);
@@ -79,10 +80,11 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
     const int lane = threadIdx.x & 31;
     WideStackOf<kSh, kBlock, false> stack;
     stack.sh = sh_stack + threadIdx.x;
+    WideRays<0> rays;
     uint32_t err = 0;
     const bool ordered = a.shadow_order.src && order_built(a.shadow_order.state);
     trace_queue<false, kQueueInner>(
-        stack, a.bvh, (unsigned)n, err,
+        stack, rays, a.bvh, (unsigned)n, err,
         [&](int count) {
             int base = 0;
             if (lane == 0) base = atomicAdd(a.ps.counts + 4, count);

@@ -268,27 +268,6 @@ int order_origin_bits(int64_t n) {
     return ob < kOrderMinOriginBits ? kOrderMinOriginBits : ob;
 }
 
-bool host_rays_coherent(const float *rays, int64_t n, const float lo[3], const float hi[3]) {
-    const int64_t warps = n / 32;
-    if (warps <= 0) return true;
-    const OrderGrid g = order_grid(lo, hi, order_origin_bits(n));
-    const int64_t samples = warps < 64 ? warps : 64;
-    int uniform = 0;
-    for (int64_t k = 0; k < samples; k++) {
-        const float *w = rays + 8 * 32 * (k * warps / samples);
-        auto key = [&](int lane) {
-            const float *r = w + 8 * lane;
-            return order_key(make_float4(r[0], r[1], r[2], r[3]), make_float4(r[4], r[5], r[6], r[7]), g);
-        };
-        // lanes 1, 7, 13, 19, 25 and 31 against lane 0: enough to choose a schedule
-        const unsigned k0 = key(0);
-        int lane = 1;
-        while (lane < 32 && key(lane) == k0) lane += 6;
-        uniform += lane >= 32;
-    }
-    return 2 * uniform > samples;
-}
-
 static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 size_t reorder_state_offset(int64_t n) {

@@ -81,11 +81,6 @@ __host__ __device__ inline unsigned order_key(const float4 r0, const float4 r1, 
 int order_origin_bits(int64_t n);
 OrderGrid order_grid(const float lo[3], const float hi[3], int origin_bits);
 
-// Whether 64 warps of 32 consecutive rays (8 floats each, host memory), evenly spaced over the n,
-// are mostly uniform in key (six lanes of each compared with its first): the host-side twin of
-// the device probe, for callers that still hold the rays on the host.
-bool host_rays_coherent(const float *rays, int64_t n, const float lo[3], const float hi[3]);
-
 // Device scratch for ordering n rays: key + rank, the ray of each sorted slot, the sorted slot of
 // each ray, 16 B per ray for a caller's hits in sorted order, 2^21 counts, the scan's chunk totals and
 // the 256-byte state block (which must be zero when the scratch is new).

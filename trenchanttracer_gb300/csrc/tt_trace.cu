@@ -51,7 +51,8 @@ enum TraceVariant : int {
     VARIANT_SORTED_OCC = 7,
     NUM_VARIANTS = 8,
     VARIANT_TWO_WIDE = 8,  // internal: the two-wide tree, for trees without a four-wide form
-    kNumKernels = 9
+    VARIANT_HOST = 9,      // internal: SORTED's shape over host rays in their own order
+    kNumKernels = 10
 };
 constexpr int64_t kMaxLaunchRays = (int64_t)1 << 30;
 constexpr int kOccBlocks = 12;  // resident blocks per SM the *_OCC variants are compiled for
@@ -75,7 +76,7 @@ struct DeviceBVH {
     unsigned long long *scratch = nullptr;  // [0] work counter, [1] error word (low 32 bits)
     int device = 0;
     int num_sms = 0;
-    int blocks_per_sm[kNumKernels] = {1, 1, 1, 1, 1, 1, 1, 1, 1};
+    int blocks_per_sm[kNumKernels] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
     int variant = VARIANT_SORTED;
     // L2 access-policy window over the node array for the trace launches (0 bytes: none), set up
     // at the first trace launch (the persisting set-aside shrinks the L2 left to other work, so a
@@ -138,9 +139,10 @@ __device__ __forceinline__ void store_hit(const TraceArgs &a, void *hits, int64_
     }
 }
 
-// The four-wide tree (kPerm: in the rays' order, when the ordering built one). kSh
+// The four-wide tree (kPerm: in the rays' order, when the ordering built one; kHost: rays and hits in
+// page-locked host memory). kSh
 // stack entries live in shared memory.
-template <bool kClosest, bool kExt, int kSh, bool kPerm, int kMinBlocks>
+template <bool kClosest, bool kExt, int kSh, bool kPerm, int kMinBlocks, bool kHost = false>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(TraceArgs a) {
     chain_begin();
     __shared__ typename WideEntry<kClosest>::type sh_stack[(kSh > 0 ? kSh : 1) * kTraceBlock];
@@ -148,10 +150,13 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
     uint32_t err = 0;
     WideStackOf<kSh, kTraceBlock, kClosest> stack;
     stack.sh = sh_stack + threadIdx.x;
+    __shared__ float sh_rays[kHost ? 6 * kTraceBlock : 1];
+    WideRays<kHost ? kTraceBlock : 0> rays;
+    rays.sh = sh_rays + (kHost ? threadIdx.x : 0);
     const bool use_perm = kPerm && a.order_state && order_built(a.order_state);
     unsigned *queue = reinterpret_cast<unsigned *>(a.counter);  // the next ray; blocks done
     trace_queue<kClosest, kWideInner>(
-        stack, a.bvh, (unsigned)a.n, err,
+        stack, rays, a.bvh, (unsigned)a.n, err,
         [&](int count) {
             unsigned b = 0;
             if (lane == 0) b = atomicAdd(queue, (unsigned)count);
@@ -259,6 +264,8 @@ static const void *kernel_for(int variant) {
         case VARIANT_SORTED: return (const void *)trace_wide_kernel<kClosest, kExt, kSortedStack, true, kSortedBlocks>;
         case VARIANT_SH16_OCC: return (const void *)trace_wide_kernel<kClosest, kExt, 16, false, kOccBlocks>;
         case VARIANT_SORTED_OCC: return (const void *)trace_wide_kernel<kClosest, kExt, 16, true, kOccBlocks>;
+        case VARIANT_HOST:
+            return (const void *)trace_wide_kernel<kClosest, kExt, kSortedStack, false, kSortedBlocks, true>;
         case VARIANT_TWO_WIDE: return (const void *)trace_warp_kernel<kClosest, kExt, false, 16, true>;
         default: return (const void *)trace_warp_kernel<kClosest, kExt, true, 0>;
     }
@@ -400,9 +407,9 @@ static void setup_l2_window(DeviceBVH &d) {
     cudaGetLastError();
 }
 
-// unordered = true traces a SORTED / SORTED_OCC variant's rays in their own order.
+// host_rays = true: rays and hits in mapped host memory, traced in their own order.
 static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n, void *d_hits, bool closest,
-                              bool ext, cudaStream_t stream, int counter_slot = 0, bool unordered = false) {
+                              bool ext, cudaStream_t stream, int counter_slot = 0, bool host_rays = false) {
     if (n < 0 || n > ((int64_t)1 << 40)) return fail(TT_ERR_INVALID, "ray count out of range");
     if (n == 0) return TT_OK;
     if (!d_rays || !d_hits) return fail(TT_ERR_INVALID, "null ray or hit buffer");
@@ -411,7 +418,7 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     // the kernels count rays in 32 bits: a longer set is traced in parts, one after the other
     for (; n > kMaxLaunchRays; n -= kMaxLaunchRays) {
         const tt_status st =
-            launch_trace(d, d_rays, kMaxLaunchRays, d_hits, closest, ext, stream, counter_slot, unordered);
+            launch_trace(d, d_rays, kMaxLaunchRays, d_hits, closest, ext, stream, counter_slot, host_rays);
         if (st != TT_OK) return st;
         d_rays = static_cast<const char *>(d_rays) + 32 * kMaxLaunchRays;
         d_hits = static_cast<char *>(d_hits) + (ext ? sizeof(tt_hit_ext) : sizeof(tt_hit)) * kMaxLaunchRays;
@@ -430,7 +437,8 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     int variant = d.variant;
     // too few rays cannot pay for the ordering
     const bool order_rays =
-        (variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC) && !unordered && n >= kOrderMinRays;
+        (variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC) && !host_rays && n >= kOrderMinRays;
+    if (host_rays) variant = VARIANT_HOST;
     if (!d.view.wide_nodes && variant != VARIANT_DYNAMIC && variant != VARIANT_WARP_VOTE) variant = VARIANT_TWO_WIDE;
     if (order_rays) {
         // one scratch per work-counter slot, so the pipeline streams never share one
@@ -649,15 +657,21 @@ tt_status tt_trace_ext(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_h
     return launch_trace(bvh->d, d_rays, n, d_hits, closest != 0, true, (cudaStream_t)stream);
 }
 
-// The device address of page-locked host memory mapped into the device's address space, or
-// nullptr (pageable memory, device memory, or an error, which is cleared).
-static const void *mapped_host_pointer(const void *p) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+// The device address of a range of page-locked host memory mapped into the device's address space, or
+// nullptr (pageable memory, device memory, a range that is not mapped as one, or an error, which is
+// cleared).
+static const void *mapped_host_range(const void *p, size_t bytes) {
+    cudaPointerAttributes first, last;
+    const char *end = static_cast<const char *>(p) + (bytes - 1);
+    if (cudaPointerGetAttributes(&first, p) != cudaSuccess || cudaPointerGetAttributes(&last, end) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer) return nullptr;
+    return static_cast<const char *>(last.devicePointer) - static_cast<const char *>(first.devicePointer) ==
+                   (ptrdiff_t)(bytes - 1)
+               ? first.devicePointer
+               : nullptr;
 }
 
 tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_hit *h_hits, int32_t closest,
@@ -666,22 +680,19 @@ tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_
     if (n == 0) return TT_OK;
     DeviceBVH &d = const_cast<tt_dbvh *>(bvh)->d;
     cudaStream_t s = (cudaStream_t)stream;
-    // Coherent rays (a sample of the host buffer decides, as the device probe would) are bound by
-    // the transfer in, incoherent ones by the trace.
-    const bool sorted_variant = d.variant == VARIANT_SORTED || d.variant == VARIANT_SORTED_OCC;
-    const bool coherent = !sorted_variant || n < (int64_t)(1 << 21) ||
-                          host_rays_coherent(reinterpret_cast<const float *>(h_rays), n, d.lo, d.hi);
-    // Coherent rays in page-locked, device-mapped host buffers: one trace launch that reads the rays
-    // and writes the hits across the host link itself (about 208 / 192 GB/s each way on a GB300,
-    // the rate the copy engines reach too), so the transfer overlaps traversal with no staging.
-    if (coherent && n >= (int64_t)(1 << 21)) {
-        const void *dr_mapped = mapped_host_pointer(h_rays), *dh_mapped = mapped_host_pointer(h_hits);
-        if (dr_mapped && dh_mapped) {
-            tt_status st = launch_trace(d, dr_mapped, n, const_cast<void *>(dh_mapped), closest != 0, false, s, 0, true);
-            if (st != TT_OK) return st;
-            TT_CUDA(cudaStreamSynchronize(s));
-            return read_error_word(d, s);
-        }
+    // Page-locked, device-mapped host buffers: one trace launch reads the rays and writes the hits across
+    // the host link itself (about 208 / 192 GB/s each way on a GB300, the rate the copy engines reach
+    // too), so the transfer overlaps traversal with no staging. Staged chunks that overlap their copies
+    // take longer for every set: 2M / 4M cosine bounces on a 524,288-triangle terrain 0.65 / 1.15 ms
+    // against 0.50 / 0.85, 4M camera rays 0.85 against 0.72, 1,000 rays 73 us against 61.
+    const void *dr_mapped = mapped_host_range(h_rays, 32ull * n), *dh_mapped = mapped_host_range(h_hits, 8ull * n);
+    if (dr_mapped && dh_mapped && !(reinterpret_cast<uintptr_t>(dr_mapped) & 15) &&
+        !(reinterpret_cast<uintptr_t>(dh_mapped) & 7) && d.view.wide_nodes && d.variant != VARIANT_DYNAMIC &&
+        d.variant != VARIANT_WARP_VOTE) {
+        tt_status st = launch_trace(d, dr_mapped, n, const_cast<void *>(dh_mapped), closest != 0, false, s, 0, true);
+        if (st != TT_OK) return st;
+        TT_CUDA(cudaStreamSynchronize(s));
+        return read_error_word(d, s);
     }
     const size_t rb = 32ull * n, hb = 8ull * n;
     if (d.d_stage_bytes < rb + hb) {
@@ -701,13 +712,9 @@ tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_
     }
     char *dr = static_cast<char *>(d.d_stage);
     char *dh = dr + rb;
-    // Otherwise chunks rotate over three streams so that the copy in of chunk i+1, the trace of
-    // chunk i and the copy out of chunk i-1 overlap; everything is ordered after prior work on
-    // `stream`. Coherent rays: 1M-ray chunks, traced in their own order. Incoherent ones: chunks of
-    // n/16, 3n/16, 6n/16 and the rest, each ordered when the variant orders, so that the trace
-    // starts early and the later chunks are large enough for ordering to pay (measured on 4M
-    // terrain rays: 2.04 ms against 2.32 ms for 1M chunks).
-    const int64_t sched[4] = {n / 16, 3 * (n / 16), 6 * (n / 16), 0};
+    // Otherwise chunks of 1M rays rotate over three streams so that the copy in of chunk i+1, the trace
+    // of chunk i and the copy out of chunk i-1 overlap; everything is ordered after prior work on
+    // `stream`.
     // The first failing call stops the issue, but every stream used is still drained before the
     // return, so no copy of the caller's buffers is in flight once the call has returned.
     tt_status st = TT_OK;
@@ -718,10 +725,7 @@ tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_
     int used = 0;
     if (cu(cudaEventRecord(d.pipe_start, s), "cudaEventRecord(pipeline start)")) {
         for (int64_t off = 0, k = 0, m = 0; off < n; off += m, k++) {
-            if (n < (int64_t)(1 << 21)) m = n;
-            else if (coherent) m = (int64_t)(1 << 20);
-            else m = k < 3 ? sched[k] : n - off;
-            if (m > n - off) m = n - off;
+            m = std::min<int64_t>(n < (int64_t)(1 << 21) ? n : (int64_t)(1 << 20), n - off);
             const int p = (int)(k % 3);
             cudaStream_t ps = d.pipe[p];
             if (k < 3) {
@@ -732,8 +736,7 @@ tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_
                                     cudaMemcpyHostToDevice, ps),
                     "cudaMemcpyAsync(rays to the device)"))
                 break;
-            st = launch_trace(d, dr + 32 * off, m, dh + 8 * off, closest != 0, false, ps, kScratchPipe + p,
-                              coherent && n >= (int64_t)(1 << 21));
+            st = launch_trace(d, dr + 32 * off, m, dh + 8 * off, closest != 0, false, ps, kScratchPipe + p);
             if (st != TT_OK) break;
             if (!cu(cudaMemcpyAsync(reinterpret_cast<char *>(h_hits) + 8 * off, dh + 8 * off, 8ull * m,
                                     cudaMemcpyDeviceToHost, ps),
