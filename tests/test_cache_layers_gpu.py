@@ -1,4 +1,5 @@
-"""The radiance cache's encoding on the GPU for arguments of any size."""
+"""The radiance cache's encoding and layers on the GPU where their arithmetic changes form: arguments of
+any size in the encoding, and tile, group and CTA edges of the tcgen05 kernel."""
 import numpy as np
 import pytest
 
@@ -37,3 +38,19 @@ def test_encoding_of_positions_in_and_far_outside_the_box(scale):
         for o, ref in ((0, np.sin(turn)), (1, np.cos(turn))):
             err = np.abs(got[:, [24 * i + 2 * k + o for i in range(3)]] - ref)
             assert np.all(err <= 2.0 ** -8 * np.abs(ref) + 2e-6), (k, o, err.max())
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 5 * 128 + 1, 152 * 5 * 128 + 130])
+def test_tcgen05_inference_matches_mma_sync(n):
+    """Radiance of both kernels from the same BF16 weights and inputs; sums in another order move a BF16
+    activation by a step (2^-8) now and then, as between any two of the cache's kernels."""
+    w = nrc.init_weights(5)
+    rec = torch.from_numpy(_records(n, 4)).cuda()
+    out = []
+    for kind in (0, 1):
+        c = Cache(LO, HI, batch=4096, mma_kind=kind)
+        c.set_weights(w)
+        out.append(c.infer(rec).cpu().numpy())
+        c.check()
+    rel = np.abs(out[0] - out[1]) / np.abs(out[1])
+    assert out[0].shape == (n, 3) and np.median(rel) < 1e-3 and np.quantile(rel, 0.999) < 5e-2

@@ -19,11 +19,20 @@
 //   layers   one thread of the group issues the layer's tcgen05.mma (M = 128, N = 64 or 16, K = 16
 //            each) and a tcgen05.commit to the group's mbarrier; after the wait every warp of the
 //            group reads its 32 TMEM lanes (tcgen05.ld 32x32b), applies ReLU, rounds to BF16 and
-//            writes the next layer's A (the 64 hidden columns fill the whole buffer)
+//            writes the next layer's A: the 64 hidden columns fill the whole buffer; in training
+//            they go back into TMEM (tcgen05.st), where the products read them, to 32 columns more
 //   output   exp of the first three columns of the last layer
 // A warpgroup synchronises on its own named barrier, so the groups advance independently.
 //
-// Operand layout: no swizzle, K-major, 8 x 16-byte core matrices. A (128 x K): core (m8, k8) at
+// What bounds it: each tile's chain of ten dependent steps (encode or ReLU, barrier, products,
+// wait), tensor pipe 21 % and issue slots 54 % of the time. 1M records: 116.4 us with the loop over the
+// layers rolled (its offsets computed by the thread that issues the products, on the chain), 114.2
+// unrolled. With the hidden activations in TMEM there is room for five groups only (96 columns each),
+// 115.8 us; training has five at most, and its steps, one tile to a CTA, are shorter that way (four of
+// 16,384 rows 222 to 214 us). Three groups that encode the next tile during a tile's products: 138 us.
+//
+// Operand layout: A in TMEM: row r in lane r, two BF16 values to a column. In shared memory: no
+// swizzle, K-major, 8 x 16-byte core matrices. A (128 x K): core (m8, k8) at
 // byte (k8 * 16 + m8) * 128, so the stride between 8-row groups (SBO) is 128 and between the two
 // K halves of one instruction (LBO) 2048; a ring slot holds k8 = 0..3 of its 32 columns. Weights
 // W_l (N x K): core (n8, k8) at (k8 * N/8 + n8) * 128 from the layer's base: SBO 128, LBO N/8 *
@@ -31,9 +40,9 @@
 // the barriers, so that every operand address the descriptors can form (with either of the two
 // byte offsets applied along either dimension) lies inside the CTA's own allocation.
 //
-// Every wait is bounded (a clock budget of about a second): one thread waits, the outcome goes
-// to all threads through shared memory and a block barrier, so a failure is uniform; it is
-// reported in the error word, and the TMEM columns are freed on every path.
+// Every wait is bounded (a clock budget of about a second); an outcome goes to the whole group or block
+// through shared memory and a barrier, so that its threads leave together; it is reported in the
+// error word, and the TMEM columns are freed on every path.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -50,17 +59,18 @@ namespace nrc {
 constexpr int kTcRows = 128;
 constexpr int kTcGroups = 6;                         // warpgroups (tiles in flight) per CTA
 constexpr int kTcThreads = 128 * kTcGroups;
-constexpr int kTmemCols = 512;                       // 64 per group, allocated as a power of two
+constexpr int kTmemCols = 512;                       // of an SM; allocated as a power of two
+constexpr int kOperandCol = kHidden;                 // a group's columns: 64 of accumulators; training: then
+__host__ __device__ constexpr int group_cols(bool train) { return kHidden + (train ? kHidden / 2 : 0); }  // the next A
 constexpr int kFillCols = 32;                        // encoded columns per ring slot (two K = 16 steps)
 constexpr int kFills = kIn / kFillCols;              // 5 slot fills per tile
 constexpr int kSlotBytes = kTcRows * kFillCols * 2;  // 8192
-constexpr int kABytes = 2 * kSlotBytes;              // 16384: the ring, later the hidden activations
+constexpr int kABytes = 2 * kSlotBytes;              // 16384: the ring, in inference later the hidden activations
 constexpr int kRecBytes = kTcRows * kRec * 4;        // 8192
 constexpr int kRecBufs = 1;                          // record buffers per group
 constexpr long long kWaitCycles = 2000000000ll;      // ~1 s at 2 GHz
 constexpr unsigned kErrMlpWait = 8u;                 // error word bit: a tensor-core wait ran out
 static_assert(kIn % kFillCols == 0 && kFillCols % 8 == 0, "whole encoding chunks per slot");
-static_assert(kABytes == kTcRows * kHidden * 2, "the hidden activations fill the operand buffer");
 
 constexpr int kTcWeightBytes = kTcWeights * 2;        // 55296
 // weights barrier; per group 2 record, 2 ring-slot and 1 product barriers; TMEM slot; flags
@@ -70,8 +80,8 @@ constexpr int kTcBarBytes = 512;
 __host__ __device__ constexpr int tc_smem(int g) {
     return g * (kABytes + kRecBufs * kRecBytes) + kTcWeightBytes + kTcBarBytes;
 }
-__host__ __device__ constexpr int tc_tmem_cols(int g) {
-    return 64 * g <= 32 ? 32 : (64 * g <= 64 ? 64 : (64 * g <= 128 ? 128 : (64 * g <= 256 ? 256 : 512)));
+__host__ __device__ constexpr int tc_tmem_cols(bool train, int g) {
+    return group_cols(train) * g <= 128 ? 128 : (group_cols(train) * g <= 256 ? 256 : 512);
 }
 constexpr int kTcSmem = tc_smem(kTcGroups);
 // Training: the transposed weights of layers 1..5 as well; five groups per CTA at most.
@@ -82,7 +92,9 @@ __host__ __device__ constexpr int tc_train_smem(int g) { return tc_smem(g) + kTc
 static_assert(tc_train_smem(kTrainWideGroups) <= 232448 && kTcTWeightBytes % 16 == 0, "training shared memory");
 static_assert(kTcSmem <= 232448, "fits the 227 KB a CTA may use");
 static_assert(kTcWeightBytes % 16 == 0 && kABytes % 16 == 0 && kRecBytes % 16 == 0, "bulk copy sizes");
-static_assert(kTmemCols >= 64 * kTcGroups, "64 accumulator columns per group");
+static_assert(kTmemCols >= group_cols(false) * kTcGroups && kTmemCols >= group_cols(true) * kTrainWideGroups,
+              "accumulator and operand columns of every group");
+static_assert(kABytes == kTcRows * kHidden * 2, "the hidden activations fill the operand buffer");
 
 
 // ---- PTX helpers ------------------------------------------------------------------------------
@@ -146,6 +158,14 @@ __device__ __forceinline__ void umma(uint32_t dtmem, uint64_t adesc, uint64_t bd
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
         : "memory");
 }
+// the same with A in tensor memory (row r in lane r, two BF16 values to a column)
+__device__ __forceinline__ void umma_ta(uint32_t dtmem, uint32_t atmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(
+            dtmem),
+        "r"(atmem), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar))
                  : "memory");
@@ -162,6 +182,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
+// 8 consecutive 32-bit TMEM columns of this thread's lane
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t w[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(w[0]),
+                 "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---- the A operand ----------------------------------------------------------------------------
@@ -193,34 +220,46 @@ __device__ __forceinline__ void encode_fill(const EncInputs &in, const float *re
 
 __device__ __forceinline__ bool bf16_pos(uint32_t bits16) { return bits16 != 0u && !(bits16 & 0x8000u); }
 
-// ReLU of this thread's 64 accumulator columns, rounded to BF16, into its row of the next A (and,
+// ReLU of this thread's 64 accumulator columns, rounded to BF16, into its lane of the next A (and,
 // training, into the row of that layer's input H in global memory, gout; the result: a bit per
 // column where H > 0).
 template <bool kTrain>
 __device__ __forceinline__ uint64_t relu_to_operand(uint32_t lane_addr, __nv_bfloat16 *A, int r, uint4 *gout) {
     uint64_t pos = 0;
+    constexpr int kBatch = 32;  // columns in flight
 #pragma unroll
-    for (int c = 0; c < kHidden; c += 16) {
-        float v[16];
-        tmem_ld16(lane_addr + c, v);
+    for (int c0 = 0; c0 < kHidden; c0 += kBatch) {
+        float v[kBatch];
+#pragma unroll
+        for (int c = 0; c < kBatch; c += 16) tmem_ld16(lane_addr + c0 + c, v + c);
         tmem_wait_ld();
-        uint32_t w[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const __nv_bfloat162 b = __floats2bfloat162_rn(fmaxf(v[2 * j], 0.f), fmaxf(v[2 * j + 1], 0.f));
-            w[j] = *reinterpret_cast<const uint32_t *>(&b);
+        for (int c = c0; c < c0 + kBatch; c += 16) {
+            uint32_t w[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float *q = v + (c - c0) + 2 * j;
+                const __nv_bfloat162 b = __floats2bfloat162_rn(fmaxf(q[0], 0.f), fmaxf(q[1], 0.f));
+                w[j] = *reinterpret_cast<const uint32_t *>(&b);
+                if (kTrain) {
+                    if (bf16_pos(w[j] & 0xffffu)) pos |= 1ull << (c + 2 * j);
+                    if (bf16_pos(w[j] >> 16)) pos |= 1ull << (c + 2 * j + 1);
+                }
+            }
             if (kTrain) {
-                if (bf16_pos(w[j] & 0xffffu)) pos |= 1ull << (c + 2 * j);
-                if (bf16_pos(w[j] >> 16)) pos |= 1ull << (c + 2 * j + 1);
+                tmem_st8(lane_addr + kOperandCol + c / 2, w);
+            } else {
+                *reinterpret_cast<uint4 *>(A + a_offset(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<uint4 *>(A + a_offset(r, c + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
+            }
+            if (kTrain && gout) {
+                gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
+                gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
             }
         }
-        *reinterpret_cast<uint4 *>(A + a_offset(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4 *>(A + a_offset(r, c + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
-        if (kTrain && gout) {
-            gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
-            gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
     }
+    if (kTrain) tmem_wait_st();
+    else fence_async_smem();
     return pos;
 }
 
@@ -230,8 +269,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // Training: dZ = dH * [H > 0] for this thread's 64 accumulator columns (pos: a bit per column; 0 for
-// a row past the end), into the operand buffer (A != nullptr) and to gout (!= nullptr).
-__device__ __forceinline__ void mask_to_operand(uint32_t lane_addr, uint64_t pos, __nv_bfloat16 *A, int r, uint4 *gout) {
+// a row past the end), into the operand columns (operand) and to gout (!= nullptr).
+__device__ __forceinline__ void mask_to_operand(uint32_t lane_addr, uint64_t pos, bool operand, uint4 *gout) {
 #pragma unroll
     for (int c = 0; c < kHidden; c += 16) {
         float v[16];
@@ -241,15 +280,13 @@ __device__ __forceinline__ void mask_to_operand(uint32_t lane_addr, uint64_t pos
 #pragma unroll
         for (int j = 0; j < 8; j++)
             w[j] = pack_bf16(pos >> (c + 2 * j) & 1 ? v[2 * j] : 0.0f, pos >> (c + 2 * j + 1) & 1 ? v[2 * j + 1] : 0.0f);
-        if (A) {
-            *reinterpret_cast<uint4 *>(A + a_offset(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4 *>(A + a_offset(r, c + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
-        }
+        if (operand) tmem_st8(lane_addr + kOperandCol + c / 2, w);
         if (gout) {
             gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
             gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
     }
+    if (operand) tmem_wait_st();
 }
 
 struct TcArgs {
@@ -307,8 +344,8 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
     uint64_t *bar_wT = bars + 1 + 5 * kG;          // training: transposed weights
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 + 5 * kG);
     int *ok_w = reinterpret_cast<int *>(tmem_slot + 1);  // the weights arrived
-    int *ok = ok_w + 1 + group;                          // this group's waits all ended
-    static_assert(8 * (2 + 5 * kG) + 4 + 4 * (1 + kG) <= kTcBarBytes, "barrier block");
+    int *ok = ok_w + 1 + 2 * group;                      // this group's waits all ended, in turns
+    static_assert(8 * (2 + 5 * kG) + 4 + 4 * (1 + 2 * kG) <= kTcBarBytes, "barrier block");
 
     const long long n = tc_rows(a.n_host, a.n_dev, a.off, a.cap);
     const long long ntiles = (n + kTcRows - 1) / kTcRows;
@@ -319,18 +356,18 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         mbar_init(bar_wT, 1);
         for (int g = 0; g < kG; g++) {
             for (int k = 0; k < 5; k++) mbar_init(bars + 1 + 5 * g + k, 1);
-            ok_w[1 + g] = 1;
+            ok_w[1 + 2 * g] = ok_w[2 + 2 * g] = 1;
         }
         *ok_w = 1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (tid < 32) tmem_alloc(tmem_slot, tc_tmem_cols(kG));
-    // Asynchronous operations of this group, counted by its issuing thread (gt == 0): the k-th
-    // completion of a barrier is awaited with parity k & 1, and whatever was issued and not yet
-    // awaited is drained (bounded) before the block exits.
-    int rec_issued[2] = {0, 0}, rec_done[2] = {0, 0}, ring_issued[2] = {0, 0}, ring_done[2] = {0, 0};
-    int mma_issued = 0, mma_done = 0;
+    if (tid < 32) tmem_alloc(tmem_slot, tc_tmem_cols(kTrain, kG));
+    // Asynchronous operations of this group, a bit for each of its five barriers (at most one operation
+    // is in flight on each): the parity a thread awaits next, and for the issuing thread (gt == 0)
+    // what it has issued and not seen complete, which it drains (bounded) before the block exits.
+    constexpr int kRec0 = 0, kRing0 = 2, kMma = 4;
+    uint32_t parity = 0, in_flight = 0;
     const long long tstride = (long long)gridDim.x * kG;
     const long long first = (long long)blockIdx.x * kG + group;
     if (gt == 0 && first < ntiles) {  // the group's first records, while the weights come in
@@ -338,7 +375,7 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         const uint32_t bytes = (uint32_t)((n - r0) < kTcRows ? (n - r0) : kTcRows) * kRec * 4;
         mbar_expect_tx(bar_rec, bytes);
         bulk_load(R, a.rec + r0 * kRec, bytes, bar_rec);
-        rec_issued[0]++;
+        in_flight |= 1u << kRec0;
     }
     bool w_pending = false;  // tid 0: the weights copy was issued and not seen complete
     if (tid == 0) {
@@ -356,55 +393,58 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot + (uint32_t)(group * 64);
+    const uint32_t tmem = *tmem_slot + (uint32_t)(group * group_cols(kTrain));
     const uint32_t lane_addr = tmem + ((uint32_t)(warp_in_group * 32) << 16);
-    // *ok_w is not written after the block barrier above; *ok is read by the group only right after
-    // a group barrier that follows the issuing thread's write and precedes its next one
+    // *ok_w is not written after the block barrier above
     const bool weights_ok = *ok_w != 0;
-    if (!weights_ok && gt == 0) *ok = 0;
-    group_sync(group);
+    // Every thread waits for the products and copies it depends on itself. dead: one of this thread's waits ran out. The
+    // group learns of it at its next checkpoint, a barrier behind which all of its threads read the
+    // same flag: the two flags take turns, so a flag is next written only when all have read it.
+    bool dead = !weights_ok && gt == 0, failed = false;
+    int turn = 0;
+    auto wait = [&](int k) {
+        if (mbar_wait(bar_rec + k, parity >> k & 1u, a.wait_cycles)) {
+            parity ^= 1u << k;
+            in_flight &= ~(1u << k);
+        } else {
+            dead = true;
+        }
+        __syncwarp();  // the TMEM loads behind a wait are the whole warp's
+        tc_fence_after();
+    };
+    auto checkpoint = [&]() {
+        if (dead) ok[turn] = 0;
+        tc_fence_before();
+        group_sync(group);
+        tc_fence_after();
+        failed = ok[turn] == 0;
+        turn ^= 1;
+        return !failed;
+    };
     int buf = 0;
     const float inv_n = 1.0f / (float)n;
     float loss = 0.0f;
-    for (long long tile = first; weights_ok && tile < ntiles; tile += tstride) {
+    for (long long tile = first; weights_ok && !failed && tile < ntiles; tile += tstride) {
         const long long r0 = tile * kTcRows;
         const int rows = (int)((n - r0) < kTcRows ? (n - r0) : kTcRows);
         const float *rec = R + buf * kTcRows * kRec + gt * kRec;
-        if (gt == 0) {
-            if (mbar_wait(bar_rec + buf, (uint32_t)(rec_done[buf] & 1), a.wait_cycles)) rec_done[buf]++;
-            else *ok = 0;
-        }
-        group_sync(group);
-        if (!*ok) break;
+        wait(kRec0 + buf);
         // layer 0 through the ring: encode a slot, issue its products, encode the other slot meanwhile
         EncInputs in{};
         if (gt < rows) in = enc_inputs(rec, a.enc.lo, a.enc.inv_ext);
-        bool failed = false;
 #pragma unroll
         for (int f = 0; f < kFills; f++) {
             const int slot = f & 1;
             __nv_bfloat16 *S = A + slot * (kSlotBytes / 2);
-            if (f >= 2) {  // the slot's previous products have read it
-                if (gt == 0) {
-                    if (mbar_wait(bar_ring + slot, (uint32_t)(ring_done[slot] & 1), a.wait_cycles)) ring_done[slot]++;
-                    else *ok = 0;
-                }
-                group_sync(group);
-                if (!*ok) {
-                    failed = true;
-                    break;
-                }
-            }
+            if (f >= 2) wait(kRing0 + slot);  // the slot's previous products have read it
             if (gt < rows) {
                 encode_fill(in, rec, S, gt, f, kTrain ? reinterpret_cast<uint4 *>(a.h[0] + (r0 + gt) * kIn) : nullptr);
             } else {
                 for (int k = 0; k < kFillCols; k += 8)
                     *reinterpret_cast<uint4 *>(S + a_offset(gt, k)) = make_uint4(0u, 0u, 0u, 0u);
             }
-            fence_async_smem();
-            tc_fence_before();
-            group_sync(group);  // the slot is encoded (after the last fill the records are free too)
-            tc_fence_after();
+            fence_async_smem();        // this thread's stores, before the products that read them
+            if (!checkpoint()) break;  // the slot is encoded (after the last fill the records are free too)
             if (gt == 0) {
                 const uint32_t s0 = saddr(S), b0 = saddr(W + tc_offset(0));
                 constexpr int N = tc_out(0);
@@ -414,61 +454,47 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
                          idesc_bf16(kTcRows, N), ks > 0 ? 1u : 0u);
                 }
                 umma_commit(bar_ring + slot);
-                ring_issued[slot]++;
+                in_flight |= 1u << (kRing0 + slot);
             }
         }
         if (failed) break;
-        if (gt == 0) {
-            if (tile + tstride < ntiles) {  // the next tile's records (every encoding read is done)
-                const int nb = (buf + 1) % kRecBufs;
-                const long long nr0 = (tile + tstride) * kTcRows;
-                const uint32_t bytes = (uint32_t)((n - nr0) < kTcRows ? (n - nr0) : kTcRows) * kRec * 4;
-                mbar_expect_tx(bar_rec + nb, bytes);
-                bulk_load(R + nb * kTcRows * kRec, a.rec + nr0 * kRec, bytes, bar_rec + nb);
-                rec_issued[nb]++;
-            }
-            // layer 0 is complete when the last fill of each slot is
-            for (int b = 0; b < 2; b++) {
-                if (ring_done[b] < ring_issued[b]) {
-                    if (mbar_wait(bar_ring + b, (uint32_t)(ring_done[b] & 1), a.wait_cycles)) ring_done[b]++;
-                    else *ok = 0;
-                }
-            }
+        if (gt == 0 && tile + tstride < ntiles) {  // the next tile's records (every encoding read is done)
+            const int nb = (buf + 1) % kRecBufs;
+            const long long nr0 = (tile + tstride) * kTcRows;
+            const uint32_t bytes = (uint32_t)((n - nr0) < kTcRows ? (n - nr0) : kTcRows) * kRec * 4;
+            mbar_expect_tx(bar_rec + nb, bytes);
+            bulk_load(R + nb * kTcRows * kRec, a.rec + nr0 * kRec, bytes, bar_rec + nb);
+            in_flight |= 1u << (kRec0 + nb);
         }
-        group_sync(group);
-        tc_fence_after();
-        if (!*ok) break;
-        // the whole buffer: the ring is no longer read
+        // layer 0 is complete when the last fill of each slot is
+        wait(kRing0 + 1);
+        wait(kRing0 + 0);
         uint64_t pos[kLayers];  // training: where H_l > 0
         float y[3] = {0.f, 0.f, 0.f};
         pos[1] = relu_to_operand<kTrain>(
             lane_addr, A, gt, kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[1] + (r0 + gt) * kHidden) : nullptr);
-        fence_async_smem();
-        tc_fence_before();
-        group_sync(group);
-        tc_fence_after();
-#pragma unroll (kTrain ? kLayers : 1)
+        if (!checkpoint()) break;
+#pragma unroll
         for (int l = 1; l < kLayers; l++) {
             const int K = layer_in(l), N = tc_out(l);
             if (gt == 0) {
-                const uint32_t a0 = saddr(A), b0 = saddr(W + tc_offset(l));
+                const uint32_t b0 = saddr(W + tc_offset(l));
                 const uint32_t idesc = idesc_bf16(kTcRows, N);
-                for (int s = 0; s < K / 16; s++)
-                    umma(tmem, sdesc(a0 + s * 2 * 2048, 2048, 128), sdesc(b0 + s * 2 * (N / 8) * 128, (N / 8) * 128, 128),
-                         idesc, s > 0 ? 1u : 0u);
+                const uint32_t a0 = saddr(A);
+                for (int s = 0; s < K / 16; s++) {
+                    const uint64_t b = sdesc(b0 + s * 2 * (N / 8) * 128, (N / 8) * 128, 128);
+                    if (kTrain) umma_ta(tmem, tmem + kOperandCol + 8 * s, b, idesc, s > 0 ? 1u : 0u);
+                    else umma(tmem, sdesc(a0 + s * 2 * 2048, 2048, 128), b, idesc, s > 0 ? 1u : 0u);
+                }
                 umma_commit(bar_mma);
-                mma_issued++;
-                if (mbar_wait(bar_mma, (uint32_t)(mma_done & 1), a.wait_cycles)) mma_done++;
-                else *ok = 0;
+                in_flight |= 1u << kMma;
             }
-            group_sync(group);
-            tc_fence_after();
-            if (!*ok) break;
+            wait(kMma);
             if (l < kLayers - 1) {
                 pos[l + 1] = relu_to_operand<kTrain>(
                     lane_addr, A, gt,
                     kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[l + 1] + (r0 + gt) * kHidden) : nullptr);
-                fence_async_smem();
+                if (!checkpoint()) break;
             } else {
                 float v[16];
                 tmem_ld16(lane_addr, v);
@@ -477,19 +503,16 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
                     y[0] = v[0];
                     y[1] = v[1];
                     y[2] = v[2];
-                } else if (gt < rows) {
+                } else if (gt < rows && !dead) {
                     float *o = a.rgb + (r0 + gt) * 3;
                     o[0] = expf(fminf(v[0], 20.0f));
                     o[1] = expf(fminf(v[1], 20.0f));
                     o[2] = expf(fminf(v[2], 20.0f));
                 }
             }
-            tc_fence_before();
-            group_sync(group);
-            tc_fence_after();
         }
-        if (kTrain) {  // (a group whose wait ran out comes here too: nothing is issued for it)
-            if (!*ok) break;
+        if (failed) break;
+        if (kTrain) {
             const long long row = r0 + gt;
             const bool own = gt < rows;
             float dy[3] = {0.f, 0.f, 0.f};
@@ -504,45 +527,30 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
                 }
             }
             const uint4 d5 = make_uint4(pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], 0.0f), 0u, 0u);
-            *reinterpret_cast<uint4 *>(A + a_offset(gt, 0)) = d5;
-            *reinterpret_cast<uint4 *>(A + a_offset(gt, 8)) = make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t d5w[8] = {d5.x, d5.y, 0u, 0u, 0u, 0u, 0u, 0u};
+            __syncwarp();
+            tmem_st8(lane_addr + kOperandCol, d5w);
+            tmem_wait_st();
             if (own) *reinterpret_cast<uint4 *>(a.dz[kLayers - 1] + row * kOutPad) = d5;
-            fence_async_smem();
-            tc_fence_before();
-            group_sync(group);
-            tc_fence_after();
+            if (gt == 0 && !mbar_wait(bar_wT, 0, a.wait_cycles)) dead = true;  // the transposed weights
+            if (!checkpoint()) break;
 #pragma unroll
             for (int l = kLayers - 1; l >= 1; l--) {
                 const int K = tc_out(l), N = layer_in(l);
                 if (gt == 0) {
-                    if (l == kLayers - 1 && !mbar_wait(bar_wT, 0, a.wait_cycles)) {
-                        *ok = 0;  // the transposed weights have not come
-                    } else {
-                        const uint32_t a0 = saddr(A), b0 = saddr(WT + tcT_offset(l));
-                        const uint32_t idesc = idesc_bf16(kTcRows, N);
-                        for (int s2 = 0; s2 < K / 16; s2++)
-                            umma(tmem, sdesc(a0 + s2 * 2 * 2048, 2048, 128),
-                                 sdesc(b0 + s2 * 2 * (N / 8) * 128, (N / 8) * 128, 128), idesc, s2 > 0 ? 1u : 0u);
-                        umma_commit(bar_mma);
-                        mma_issued++;
-                        if (mbar_wait(bar_mma, (uint32_t)(mma_done & 1), a.wait_cycles)) mma_done++;
-                        else *ok = 0;
-                    }
+                    const uint32_t b0 = saddr(WT + tcT_offset(l));
+                    const uint32_t idesc = idesc_bf16(kTcRows, N);
+                    for (int s2 = 0; s2 < K / 16; s2++)
+                        umma_ta(tmem, tmem + kOperandCol + 8 * s2,
+                                sdesc(b0 + s2 * 2 * (N / 8) * 128, (N / 8) * 128, 128), idesc, s2 > 0 ? 1u : 0u);
+                    umma_commit(bar_mma);
+                    in_flight |= 1u << kMma;
                 }
-                group_sync(group);
-                tc_fence_after();
-                if (!*ok) {
-                    failed = true;
-                    break;
-                }
-                mask_to_operand(lane_addr, own ? pos[l] : 0ull, l > 1 ? A : nullptr, gt,
+                wait(kMma);
+                mask_to_operand(lane_addr, own ? pos[l] : 0ull, l > 1,
                                 own ? reinterpret_cast<uint4 *>(a.dz[l - 1] + row * kHidden) : nullptr);
-                fence_async_smem();
-                tc_fence_before();
-                group_sync(group);
-                tc_fence_after();
+                if (l > 1 && !checkpoint()) break;
             }
-            if (failed) break;
         }
         buf = (buf + 1) % kRecBufs;
     }
@@ -551,22 +559,18 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
         if ((tid & 31) == 0 && a.loss) atomicAdd(a.loss, loss * inv_n);
     }
+    if (dead) atomicOr(a.err, kErrMlpWait);
     if (gt == 0) {
-        if (!*ok) atomicOr(a.err, kErrMlpWait);
         // drain what this group issued and did not see complete (bounded again), before TMEM is freed
-        for (int b = 0; b < 2; b++) {
-            while (rec_done[b] < rec_issued[b] && mbar_wait(bar_rec + b, (uint32_t)(rec_done[b] & 1))) rec_done[b]++;
-            while (ring_done[b] < ring_issued[b] && mbar_wait(bar_ring + b, (uint32_t)(ring_done[b] & 1)))
-                ring_done[b]++;
-        }
-        while (mma_done < mma_issued && mbar_wait(bar_mma, (uint32_t)(mma_done & 1))) mma_done++;
+        for (int k = 0; k < 5; k++)
+            if (in_flight >> k & 1u) mbar_wait(bar_rec + k, parity >> k & 1u);
     }
     if (tid == 0 && w_pending) mbar_wait(bar_w, 0);  // the weights copy, if its wait ran out
     if (kTrain && tid == 0) mbar_wait(bar_wT, 0);    // (complete but for a wait that ran out)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (tid < 32) tmem_free(*tmem_slot, tc_tmem_cols(kG));
+    if (tid < 32) tmem_free(*tmem_slot, tc_tmem_cols(kTrain, kG));
 }
 
 __global__ void k_tc_layout(const float *w, uint16_t *out) {
