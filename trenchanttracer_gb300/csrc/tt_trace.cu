@@ -22,6 +22,7 @@
 //   TT_VARIANT_SH16_OCC,  WARP_SH16 and SORTED (16 entries) compiled for 12 resident blocks per SM (40
 //   TT_VARIANT_SORTED_OCC registers and spilled values), trading spills for more warps.
 // All but WARP_VOTE return the per-ray result of the reference's algorithm, bit for bit.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -658,20 +659,35 @@ tt_status tt_trace_ext(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_h
 }
 
 // The device address of a range of page-locked host memory mapped into the device's address space, or
-// nullptr (pageable memory, device memory, a range that is not mapped as one, or an error, which is
-// cleared).
+// nullptr: pageable memory, device memory, a range that is not all of one page-locked allocation
+// (its ends alone do not tell: two registered ranges may have pageable memory between them), or
+// an error, which is cleared.
 static const void *mapped_host_range(const void *p, size_t bytes) {
-    cudaPointerAttributes first, last;
-    const char *end = static_cast<const char *>(p) + (bytes - 1);
-    if (cudaPointerGetAttributes(&first, p) != cudaSuccess || cudaPointerGetAttributes(&last, end) != cudaSuccess) {
+    using GetAttribute = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const GetAttribute get = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &found) !=
+                cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<GetAttribute>(fn);
+    }();
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer) return nullptr;
-    return static_cast<const char *>(last.devicePointer) - static_cast<const char *>(first.devicePointer) ==
-                   (ptrdiff_t)(bytes - 1)
-               ? first.devicePointer
-               : nullptr;
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer || !get) return nullptr;
+    const CUdeviceptr first = reinterpret_cast<CUdeviceptr>(at.devicePointer);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, first) != CUDA_SUCCESS ||
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, first) != CUDA_SUCCESS)
+        return nullptr;
+    return first >= start && first - start <= size && bytes <= size - (first - start) ? at.devicePointer : nullptr;
 }
 
 tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_hit *h_hits, int32_t closest,
