@@ -9,7 +9,7 @@
 // hit still goes to its own slot, and traversal has per-ray semantics, so the results do not
 // depend on the order.
 //
-// Kernels, in stream order: (1) clear the key counts and probe every 16th warp of rays (a
+// Kernels, in stream order: (1) clear the key counts and probe a 16th of the warps of rays (a
 // warp is uniform when its 32 keys are equal); when more than half of the sampled warps are
 // uniform the rays are already coherent and every later kernel returns at once, leaving the rays
 // in their own order. (2) Keys, and for each ray its rank among the rays of its key, from one
@@ -35,7 +35,7 @@ namespace tt {
 constexpr int kOrderBlock = 256;
 constexpr int kScanChunk = 2048;  // counts per scan chunk: 256 threads x 8
 constexpr int kNumChunks = (1 << kOrderBits) / kScanChunk;
-constexpr int kProbeStride = 16;  // the coherence probe looks at every 16th warp of rays
+constexpr int kProbeStride = 16;  // the coherence probe looks at one warp of rays in 16
 static_assert(kScanChunk == 8 * kOrderBlock && kNumChunks == 4 * kOrderBlock, "scan shapes");
 static_assert(((1 << (kOrderDirBits + kOrderMinOriginBits)) / kScanChunk) % 4 == 0, "whole uint4 of chunk totals");
 
@@ -111,7 +111,11 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
     __syncthreads();
     const int64_t warps = (n + 31) / 32;
     unsigned uniform = 0, full = 0;
-    for (int64_t w = (tid >> 5) * kProbeStride; w < warps; w += (nthreads >> 5) * kProbeStride) {
+    for (int64_t j = tid >> 5; j * kProbeStride < warps; j += nthreads >> 5) {
+        // one warp of every kProbeStride, each time another one: a fixed one meets the same columns in every
+        // row of an image (1,024 wide: two, the centre's among them, where directions change their
+        // cells, so camera rays were ordered to no use: 1M on the 2,097,152-triangle terrain 282 us, so 219)
+        const int64_t w = j * kProbeStride + (((unsigned)j * 0x9e3779b1u) >> 28) % kProbeStride;
         if (w * 32 + 32 > n) continue;  // only full warps count; w is the same in every lane
         const int64_t i = w * 32 + lane;
         const unsigned key = order_key(a.rays[2 * i], a.rays[2 * i + 1], a.g);

@@ -8,7 +8,7 @@
 // minima and maxima, because the signs of the direction pick the entered and the left planes by
 // address. Leaves hold their triangles in pairs, so one pass of the packed instructions tests two.
 // 4M rays on the 2,097,152-triangle terrain, two-wide to four-wide (both sets through the ordering):
-// camera rays 0.64 to 0.49 ms, cosine bounces 1.18 to 0.87 ms.
+// camera rays 0.64 to 0.49 ms, cosine bounces 1.18 to 0.83 ms.
 //
 // Why the result is the same. The two-wide loop at a node A tests A's children B and C against the
 // current hit distance t, goes to the one with the smaller entry distance (B when equal) and
