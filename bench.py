@@ -63,16 +63,16 @@ METRIC = "Mrays/s closest-hit; time to relMSE 0.01, cached vs plain tracer, 1 GB
 UNIT = "Mrays/s"
 L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of the trace kernel of
-# this workload (the default, ray-ordered variant), the mean of the primary (293.1 MB) and
-# incoherent (328.8 MB) launches ncu captured of `bench.py --steps 2 --warmup 3` on a GB300; the
-# ordering kernels around them add 8 MB (primary: the probe only) and 523 MB (incoherent: probe,
-# keys, scan, ordered copy, hit gather). bench.py cannot run ncu itself.
-TRACE_DRAM_BYTES_PER_LAUNCH = 311_000_000
-# L2 of the same GB300 from one ncu capture of the incoherent trace launch (1M rays, the current
-# 10-block build): 74.89 sectors/ns were 6.59 % of the sustained peak, i.e. 1,136 sectors/ns x 32 B;
-# the launch's own L2 traffic was that 6.6 % of it
+# this workload (the default, ray-ordered variant), the mean of a launch of 4M camera rays (318.2
+# MB) and one of 4M cosine rays (897.9 MB: rays read through an index, hits written to their own
+# places) that ncu captured on a GB300 on this terrain; the ordering kernels around them add 8 MB
+# (camera rays: the probe only) and 215 MB (probe, keys, scan, index). bench.py cannot run ncu itself.
+TRACE_DRAM_BYTES_PER_LAUNCH = 608_000_000
+# L2 of the same GB300 from one ncu capture of an incoherent trace launch (1M rays): 132.0 sectors/ns
+# were 11.67 % of the sustained peak, i.e. 1,131 sectors/ns x 32 B (an earlier capture: 1,136, kept);
+# the launch's own L2 traffic was that 11.7 % of it
 TRACE_L2_PEAK_GBS = 36_370.0
-TRACE_L2_TRAFFIC_PCT = 6.6
+TRACE_L2_TRAFFIC_PCT = 11.7
 
 
 def load_peaks() -> dict:
@@ -85,7 +85,7 @@ def load_peaks() -> dict:
 
 # the SIMD efficiency and the L2 figures of the trace kernel from the same committed ncu capture
 # (profiles/trace_kernel_terrain_closest.md, incoherent launch): threads per executed instruction
-TRACE_THREADS_PER_INST = 9.06
+TRACE_THREADS_PER_INST = 16.89
 
 
 def terrain_config(n_rays: int) -> dict:
@@ -461,8 +461,8 @@ def run_ours(args) -> None:
         "any_hit": dict(any_hit, light=SHADOW_LIGHT),
         "e2e": {"value": round(e2e_val, 2), "unit": UNIT, "h2d_bytes_per_step": int(n_rays * 32),
                 "d2h_bytes_per_step": int(n_rays * 8)},
-        "roofline": {"binding": "issue and latency of divergent traversal: DRAM at 4 % of its peak, real L2 traffic "
-                                f"at {TRACE_L2_TRAFFIC_PCT} % of its peak, issue on 59 % of cycles with "
+        "roofline": {"binding": "latency and issue of divergent traversal: DRAM at 10 % of its peak, real L2 traffic "
+                                f"at {TRACE_L2_TRAFFIC_PCT} % of its peak, issue on 49 % of cycles with "
                                 f"{TRACE_THREADS_PER_INST} of 32 lanes per instruction (ncu, incoherent launch)",
                      "l2": {"frac": round(achieved / TRACE_L2_PEAK_GBS, 4), "achieved": round(achieved, 1),
                             "peak": TRACE_L2_PEAK_GBS, "unit": "GB/s", "l2_traffic_pct_of_peak": TRACE_L2_TRAFFIC_PCT,
@@ -478,7 +478,7 @@ def run_ours(args) -> None:
                                        "workload (mean of the primary and incoherent launches)",
                      "peak_source": f"{peaks['source']} hbm_gbs (MEASURED_PEAKS.json)" if peaks["source"] == "measured"
                      else "fallback 6.8 TB/s", "bytes_per_ray": round(bpr, 1),
-                     "kernel": "tt_trace: ray ordering + trace_warp_kernel<closest> (avg per ray set)",
+                     "kernel": "tt_trace: ray ordering + trace_wide_kernel<closest> (avg per ray set)",
                      "avg_launch_ms": round(float(kernel_ms), 4)},
         "ref_kernel": ref_kernel,
         "cache": cache_line,
