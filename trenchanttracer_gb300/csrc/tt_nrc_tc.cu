@@ -87,6 +87,7 @@ constexpr int kTcSmem = tc_smem(kTcGroups);
 // Training: the transposed weights of layers 1..5 as well; five groups per CTA at most.
 constexpr int kTcTWeightBytes = kTcTWeights * 2;  // 34816
 constexpr int kTrainGroups = 1;                   // few tiles: spread over the SMs
+constexpr int kTrainSplit = 2;                    // threads to a row then (k_mlp_forward_tc)
 constexpr int kTrainWideGroups = 5;
 __host__ __device__ constexpr int tc_train_smem(int g) { return tc_smem(g) + kTcTWeightBytes; }
 static_assert(tc_train_smem(kTrainWideGroups) <= 232448 && kTcTWeightBytes % 16 == 0, "training shared memory");
@@ -200,38 +201,54 @@ __device__ __forceinline__ int kmajor_offset(int r, int k, int R) {
     return ((k >> 3) * (R >> 3) + (r >> 3)) * 64 + (r & 7) * 8 + (k & 7);
 }
 
+// 32 bytes of a row in one store (p 32-byte aligned): a store of 16 bytes of each of 32 rows takes the
+// same 32 cache-line accesses
+__device__ __forceinline__ void store32(uint4 *p, uint4 a, uint4 b) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+
 struct TcEncoding {
     float lo[3], inv_ext[3];
 };
 
 // Encoding values [32 f, 32 f + 32) of one row (tt_nrc.cuh) into ring slot S: four chunks of 8
 // BF16 values, each one 16-byte store (the 32 rows of a warp write 512 contiguous bytes per
-// chunk). f must be a compile-time constant after unrolling.
+// chunk). f must be a compile-time constant after unrolling. With kSplit threads to a row, thread
+// `part` of the row makes its share of the chunks (part is the same in all lanes of a warp).
 // gout (training): the row of H_0 in global memory, which gets the same values.
-__device__ __forceinline__ void encode_fill(const EncInputs &in, const float *rec, __nv_bfloat16 *S, int r, int f,
-                                            uint4 *gout) {
+template <int kSplit>
+__device__ __forceinline__ void encode_fill(const EncInputs &in, const float *rec, __nv_bfloat16 *S, int r, int part,
+                                            int f, uint4 *gout) {
+    constexpr int kChunks = kFillCols / 8;
+    static_assert(kChunks % (2 * kSplit) == 0, "whole chunks for each thread of a row");
 #pragma unroll
-    for (int j = 0; j < kFillCols / 8; j++) {
-        const uint4 v = enc_chunk(in, rec, f * (kFillCols / 8) + j);
+    for (int j = 0; j < kChunks; j += 2) {
+        if (kSplit > 1 && j / (kChunks / kSplit) != part) continue;
+        const uint4 v = enc_chunk(in, rec, f * kChunks + j), w = enc_chunk(in, rec, f * kChunks + j + 1);
         *reinterpret_cast<uint4 *>(S + a_offset(r, 8 * j)) = v;
-        if (gout) gout[f * (kFillCols / 8) + j] = v;
+        *reinterpret_cast<uint4 *>(S + a_offset(r, 8 * j + 8)) = w;
+        if (gout) store32(gout + f * kChunks + j, v, w);
     }
 }
 
 __device__ __forceinline__ bool bf16_pos(uint32_t bits16) { return bits16 != 0u && !(bits16 & 0x8000u); }
 
-// ReLU of this thread's 64 accumulator columns, rounded to BF16, into its lane of the next A (and,
-// training, into the row of that layer's input H in global memory, gout; the result: a bit per
-// column where H > 0).
-template <bool kTrain>
-__device__ __forceinline__ uint64_t relu_to_operand(uint32_t lane_addr, __nv_bfloat16 *A, int r, uint4 *gout) {
+// ReLU of this thread's 64 / kSplit accumulator columns from col on, rounded to BF16, into its lane of
+// the next A (and, training, into the row of that layer's input H in global memory, gout; the result:
+// a bit per column where H > 0).
+template <bool kTrain, int kSplit>
+__device__ __forceinline__ uint64_t relu_to_operand(uint32_t lane_addr, int col, __nv_bfloat16 *A, int r, uint4 *gout) {
+    static_assert(kTrain || kSplit == 1, "the shared-memory operand is written by one thread a row");
     uint64_t pos = 0;
-    constexpr int kBatch = 32;  // columns in flight
+    constexpr int kCols = kHidden / kSplit, kBatch = kCols < 32 ? kCols : 32;  // columns in flight
+    if (gout) gout += col / 8;
 #pragma unroll
-    for (int c0 = 0; c0 < kHidden; c0 += kBatch) {
+    for (int c0 = 0; c0 < kCols; c0 += kBatch) {
         float v[kBatch];
 #pragma unroll
-        for (int c = 0; c < kBatch; c += 16) tmem_ld16(lane_addr + c0 + c, v + c);
+        for (int c = 0; c < kBatch; c += 16) tmem_ld16(lane_addr + col + c0 + c, v + c);
         tmem_wait_ld();
 #pragma unroll
         for (int c = c0; c < c0 + kBatch; c += 16) {
@@ -247,14 +264,13 @@ __device__ __forceinline__ uint64_t relu_to_operand(uint32_t lane_addr, __nv_bfl
                 }
             }
             if (kTrain) {
-                tmem_st8(lane_addr + kOperandCol + c / 2, w);
+                tmem_st8(lane_addr + kOperandCol + (col + c) / 2, w);
             } else {
                 *reinterpret_cast<uint4 *>(A + a_offset(r, c)) = make_uint4(w[0], w[1], w[2], w[3]);
                 *reinterpret_cast<uint4 *>(A + a_offset(r, c + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
             }
             if (kTrain && gout) {
-                gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
-                gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
+                store32(gout + c / 8, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
             }
         }
     }
@@ -268,23 +284,22 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<const uint32_t *>(&b);
 }
 
-// Training: dZ = dH * [H > 0] for this thread's 64 accumulator columns (pos: a bit per column; 0 for
-// a row past the end), into the operand columns (operand) and to gout (!= nullptr).
-__device__ __forceinline__ void mask_to_operand(uint32_t lane_addr, uint64_t pos, bool operand, uint4 *gout) {
+// Training: dZ = dH * [H > 0] for this thread's 64 / kSplit accumulator columns from col on (pos: a bit
+// per column; 0 for a row past the end), into the operand columns (operand) and to gout (!= nullptr).
+template <int kSplit>
+__device__ __forceinline__ void mask_to_operand(uint32_t lane_addr, int col, uint64_t pos, bool operand, uint4 *gout) {
+    if (gout) gout += col / 8;
 #pragma unroll
-    for (int c = 0; c < kHidden; c += 16) {
+    for (int c = 0; c < kHidden / kSplit; c += 16) {
         float v[16];
-        tmem_ld16(lane_addr + c, v);
+        tmem_ld16(lane_addr + col + c, v);
         tmem_wait_ld();
         uint32_t w[8];
 #pragma unroll
         for (int j = 0; j < 8; j++)
             w[j] = pack_bf16(pos >> (c + 2 * j) & 1 ? v[2 * j] : 0.0f, pos >> (c + 2 * j + 1) & 1 ? v[2 * j + 1] : 0.0f);
-        if (operand) tmem_st8(lane_addr + kOperandCol + c / 2, w);
-        if (gout) {
-            gout[c / 8] = make_uint4(w[0], w[1], w[2], w[3]);
-            gout[c / 8 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
+        if (operand) tmem_st8(lane_addr + kOperandCol + (col + c) / 2, w);
+        if (gout) store32(gout + c / 8, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
     }
     if (operand) tmem_wait_st();
 }
@@ -312,8 +327,9 @@ __device__ __forceinline__ long long tc_rows(long long n_host, const int *n_dev,
     return n < 0 ? 0 : (n > cap ? cap : n);
 }
 
-__device__ __forceinline__ void group_sync(int group) {  // the 128 threads of one warpgroup
-    asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+template <int kThreads>
+__device__ __forceinline__ void group_sync(int group) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kThreads) : "memory");
 }
 
 // kTrain: also writes every layer's input H_l, and goes back through the layers before the next tile.
@@ -325,11 +341,19 @@ __device__ __forceinline__ void group_sync(int group) {  // the 128 threads of o
 // the operand buffer. Where H_l > 0 stays in registers, 64 bits a layer: a backward kernel of its own
 // loaded its weights, the outputs and every H_l again, one dependent cache access after another
 // (four steps of 16,384 rows, the cache's batch, with the host's copies 257 to 225 us).
-template <bool kTrain, int kG>
-__global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
+//
+// kSplit: threads to a row. A group's warps w, w + 4, ... read the same TMEM lanes, each its share of the
+// columns. Training with one tile to a CTA takes two: with 32-byte stores of H and dZ (a warp's store meets
+// 32 lines whatever its width, and these stores are a tenth of the step) four steps take 209 us, with one
+// thread to a row 216, with four and 16-byte stores 226 (two: 215).
+template <bool kTrain, int kG, int kSplit>
+__global__ void __launch_bounds__(128 * kG * kSplit, 1) k_mlp_forward_tc(TcArgs a) {
     chain_begin();
     extern __shared__ __align__(128) uint8_t smem[];
-    const int tid = threadIdx.x, group = tid >> 7, gt = tid & 127, warp_in_group = gt >> 5;
+    constexpr int kGroupThreads = kTcRows * kSplit;
+    // gt: the thread of its group; gr: its row of the tile; part: its share of the row
+    const int tid = threadIdx.x, group = tid / kGroupThreads, gt = tid % kGroupThreads, gr = gt % kTcRows;
+    const int part = kSplit > 1 ? gt / kTcRows : 0, col = part * (kHidden / kSplit);
     __nv_bfloat16 *A = reinterpret_cast<__nv_bfloat16 *>(smem + group * kABytes);
     uint16_t *W = reinterpret_cast<uint16_t *>(smem + kG * kABytes);
     constexpr int kWBytes = kTcWeightBytes + (kTrain ? kTcTWeightBytes : 0);
@@ -343,9 +367,9 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
     uint64_t *bar_mma = bar_rec + 4;               // the group's hidden and output layers
     uint64_t *bar_wT = bars + 1 + 5 * kG;          // training: transposed weights
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 + 5 * kG);
-    int *ok_w = reinterpret_cast<int *>(tmem_slot + 1);  // the weights arrived
-    int *ok = ok_w + 1 + 2 * group;                      // this group's waits all ended, in turns
-    static_assert(8 * (2 + 5 * kG) + 4 + 4 * (1 + 2 * kG) <= kTcBarBytes, "barrier block");
+    int *flags = reinterpret_cast<int *>(tmem_slot + 1);
+    int *ok = flags + 2 * group;  // this group's waits all ended, in turns
+    static_assert(8 * (2 + 5 * kG) + 4 + 4 * 2 * kG <= kTcBarBytes, "barrier block");
 
     const long long n = tc_rows(a.n_host, a.n_dev, a.off, a.cap);
     const long long ntiles = (n + kTcRows - 1) / kTcRows;
@@ -356,9 +380,8 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         mbar_init(bar_wT, 1);
         for (int g = 0; g < kG; g++) {
             for (int k = 0; k < 5; k++) mbar_init(bars + 1 + 5 * g + k, 1);
-            ok_w[1 + 2 * g] = ok_w[2 + 2 * g] = 1;
+            flags[2 * g] = flags[2 * g + 1] = 1;
         }
-        *ok_w = 1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -377,30 +400,27 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         bulk_load(R, a.rec + r0 * kRec, bytes, bar_rec);
         in_flight |= 1u << kRec0;
     }
-    bool w_pending = false;  // tid 0: the weights copy was issued and not seen complete
+    bool dead = false;
     if (tid == 0) {
         mbar_expect_tx(bar_w, kTcWeightBytes);
         bulk_load(W, a.w, kTcWeightBytes, bar_w);
         if (kTrain) {  // comes in while the forward pass runs
             mbar_expect_tx(bar_wT, kTcTWeightBytes);
             bulk_load(WT, a.wT, kTcTWeightBytes, bar_wT);
-        }
-        if (!mbar_wait(bar_w, 0, a.wait_cycles)) {
-            *ok_w = 0;
-            w_pending = true;
+        } else if (!mbar_wait(bar_w, 0, a.wait_cycles)) {
+            dead = true;
         }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot + (uint32_t)(group * group_cols(kTrain));
-    const uint32_t lane_addr = tmem + ((uint32_t)(warp_in_group * 32) << 16);
-    // *ok_w is not written after the block barrier above
-    const bool weights_ok = *ok_w != 0;
-    // Every thread waits for the products and copies it depends on itself. dead: one of this thread's waits ran out. The
-    // group learns of it at its next checkpoint, a barrier behind which all of its threads read the
-    // same flag: the two flags take turns, so a flag is next written only when all have read it.
-    bool dead = !weights_ok && gt == 0, failed = false;
+    const uint32_t lane_addr = tmem + ((uint32_t)(gr & ~31) << 16);
+    // Every thread waits for the products and copies it depends on itself. dead: one of this thread's waits
+    // ran out. The group learns of it at its next checkpoint, a barrier behind which all of its threads
+    // read the same flag: the two flags take turns, so a flag is next written only when all have
+    // read it.
+    bool failed = false;
     int turn = 0;
     auto wait = [&](int k) {
         if (mbar_wait(bar_rec + k, parity >> k & 1u, a.wait_cycles)) {
@@ -415,7 +435,7 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
     auto checkpoint = [&]() {
         if (dead) ok[turn] = 0;
         tc_fence_before();
-        group_sync(group);
+        group_sync<kGroupThreads>(group);
         tc_fence_after();
         failed = ok[turn] == 0;
         turn ^= 1;
@@ -424,26 +444,28 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
     int buf = 0;
     const float inv_n = 1.0f / (float)n;
     float loss = 0.0f;
-    for (long long tile = first; weights_ok && !failed && tile < ntiles; tile += tstride) {
+    for (long long tile = first; !failed && tile < ntiles; tile += tstride) {
         const long long r0 = tile * kTcRows;
         const int rows = (int)((n - r0) < kTcRows ? (n - r0) : kTcRows);
-        const float *rec = R + buf * kTcRows * kRec + gt * kRec;
+        const float *rec = R + buf * kTcRows * kRec + gr * kRec;
         wait(kRec0 + buf);
         // layer 0 through the ring: encode a slot, issue its products, encode the other slot meanwhile
         EncInputs in{};
-        if (gt < rows) in = enc_inputs(rec, a.enc.lo, a.enc.inv_ext);
+        if (gr < rows) in = enc_inputs(rec, a.enc.lo, a.enc.inv_ext);
 #pragma unroll
         for (int f = 0; f < kFills; f++) {
             const int slot = f & 1;
             __nv_bfloat16 *S = A + slot * (kSlotBytes / 2);
             if (f >= 2) wait(kRing0 + slot);  // the slot's previous products have read it
-            if (gt < rows) {
-                encode_fill(in, rec, S, gt, f, kTrain ? reinterpret_cast<uint4 *>(a.h[0] + (r0 + gt) * kIn) : nullptr);
+            if (gr < rows) {
+                encode_fill<kSplit>(in, rec, S, gr, part, f,
+                                    kTrain ? reinterpret_cast<uint4 *>(a.h[0] + (r0 + gr) * kIn) : nullptr);
             } else {
-                for (int k = 0; k < kFillCols; k += 8)
-                    *reinterpret_cast<uint4 *>(S + a_offset(gt, k)) = make_uint4(0u, 0u, 0u, 0u);
+                for (int k = part * (kFillCols / kSplit); k < (part + 1) * (kFillCols / kSplit); k += 8)
+                    *reinterpret_cast<uint4 *>(S + a_offset(gr, k)) = make_uint4(0u, 0u, 0u, 0u);
             }
-            fence_async_smem();        // this thread's stores, before the products that read them
+            fence_async_smem();  // this thread's stores, before the products that read them
+            if (f == 0 && gt == 0 && tile == first && !mbar_wait(bar_w, 0, a.wait_cycles)) dead = true;  // the weights
             if (!checkpoint()) break;  // the slot is encoded (after the last fill the records are free too)
             if (gt == 0) {
                 const uint32_t s0 = saddr(S), b0 = saddr(W + tc_offset(0));
@@ -471,8 +493,9 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         wait(kRing0 + 0);
         uint64_t pos[kLayers];  // training: where H_l > 0
         float y[3] = {0.f, 0.f, 0.f};
-        pos[1] = relu_to_operand<kTrain>(
-            lane_addr, A, gt, kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[1] + (r0 + gt) * kHidden) : nullptr);
+        pos[1] = relu_to_operand<kTrain, kSplit>(
+            lane_addr, col, A, gr,
+            kTrain && gr < rows ? reinterpret_cast<uint4 *>(a.h[1] + (r0 + gr) * kHidden) : nullptr);
         if (!checkpoint()) break;
 #pragma unroll
         for (int l = 1; l < kLayers; l++) {
@@ -491,11 +514,11 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
             }
             wait(kMma);
             if (l < kLayers - 1) {
-                pos[l + 1] = relu_to_operand<kTrain>(
-                    lane_addr, A, gt,
-                    kTrain && gt < rows ? reinterpret_cast<uint4 *>(a.h[l + 1] + (r0 + gt) * kHidden) : nullptr);
+                pos[l + 1] = relu_to_operand<kTrain, kSplit>(
+                    lane_addr, col, A, gr,
+                    kTrain && gr < rows ? reinterpret_cast<uint4 *>(a.h[l + 1] + (r0 + gr) * kHidden) : nullptr);
                 if (!checkpoint()) break;
-            } else {
+            } else if (part == 0) {
                 float v[16];
                 tmem_ld16(lane_addr, v);
                 tmem_wait_ld();
@@ -503,8 +526,8 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
                     y[0] = v[0];
                     y[1] = v[1];
                     y[2] = v[2];
-                } else if (gt < rows && !dead) {
-                    float *o = a.rgb + (r0 + gt) * 3;
+                } else if (gr < rows && !dead) {
+                    float *o = a.rgb + (r0 + gr) * 3;
                     o[0] = expf(fminf(v[0], 20.0f));
                     o[1] = expf(fminf(v[1], 20.0f));
                     o[2] = expf(fminf(v[2], 20.0f));
@@ -513,10 +536,10 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         }
         if (failed) break;
         if (kTrain) {
-            const long long row = r0 + gt;
-            const bool own = gt < rows;
+            const long long row = r0 + gr;
+            const bool own = gr < rows;
             float dy[3] = {0.f, 0.f, 0.f};
-            if (own) {
+            if (own && part == 0) {
 #pragma unroll
                 for (int c = 0; c < kOut; c++) {
                     const float p = expf(fminf(y[c], 20.0f));
@@ -529,9 +552,11 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
             const uint4 d5 = make_uint4(pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], 0.0f), 0u, 0u);
             const uint32_t d5w[8] = {d5.x, d5.y, 0u, 0u, 0u, 0u, 0u, 0u};
             __syncwarp();
-            tmem_st8(lane_addr + kOperandCol, d5w);
-            tmem_wait_st();
-            if (own) *reinterpret_cast<uint4 *>(a.dz[kLayers - 1] + row * kOutPad) = d5;
+            if (part == 0) {
+                tmem_st8(lane_addr + kOperandCol, d5w);
+                tmem_wait_st();
+            }
+            if (own && part == 0) *reinterpret_cast<uint4 *>(a.dz[kLayers - 1] + row * kOutPad) = d5;
             if (gt == 0 && !mbar_wait(bar_wT, 0, a.wait_cycles)) dead = true;  // the transposed weights
             if (!checkpoint()) break;
 #pragma unroll
@@ -547,7 +572,7 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
                     in_flight |= 1u << kMma;
                 }
                 wait(kMma);
-                mask_to_operand(lane_addr, own ? pos[l] : 0ull, l > 1,
+                mask_to_operand<kSplit>(lane_addr, col, own ? pos[l] : 0ull, l > 1,
                                 own ? reinterpret_cast<uint4 *>(a.dz[l - 1] + row * kHidden) : nullptr);
                 if (l > 1 && !checkpoint()) break;
             }
@@ -565,8 +590,9 @@ __global__ void __launch_bounds__(128 * kG, 1) k_mlp_forward_tc(TcArgs a) {
         for (int k = 0; k < 5; k++)
             if (in_flight >> k & 1u) mbar_wait(bar_rec + k, parity >> k & 1u);
     }
-    if (tid == 0 && w_pending) mbar_wait(bar_w, 0);  // the weights copy, if its wait ran out
-    if (kTrain && tid == 0) mbar_wait(bar_wT, 0);    // (complete but for a wait that ran out)
+    // the weights' copies: complete but for a wait that ran out
+    if (tid == 0) mbar_wait(bar_w, 0);
+    if (kTrain && tid == 0) mbar_wait(bar_wT, 0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -734,13 +760,13 @@ __global__ void __launch_bounds__(kWgThreads, 3) k_mlp_wgrad_tc(TcWgradArgs a) {
 }
 
 tt_status tc_setup() {
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_forward_tc<false, kTcGroups>,
+    cudaError_t e = cudaFuncSetAttribute(k_mlp_forward_tc<false, kTcGroups, 1>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_forward_tc<true, kTrainGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(k_mlp_forward_tc<true, kTrainGroups, kTrainSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  tc_train_smem(kTrainGroups));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_forward_tc<true, kTrainWideGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(k_mlp_forward_tc<true, kTrainWideGroups, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  tc_train_smem(kTrainWideGroups));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mlp_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
@@ -809,8 +835,9 @@ tt_status tc_train(const TcTrainArgs &t, cudaStream_t s) {
     // every SM (two blocks fit an SM); larger ones: five groups per block.
     const bool wide = (rows + kTcRows - 1) / kTcRows >= (long long)kTrainWideGroups * t.num_sms;
     const int groups = wide ? kTrainWideGroups : kTrainGroups;
-    launch_chained(wide ? k_mlp_forward_tc<true, kTrainWideGroups> : k_mlp_forward_tc<true, kTrainGroups>,
-                   tc_grid(rows, groups, t.num_sms, wide ? 1 : 2), 128 * groups, tc_train_smem(groups), s, f);
+    launch_chained(wide ? k_mlp_forward_tc<true, kTrainWideGroups, 1> : k_mlp_forward_tc<true, kTrainGroups, kTrainSplit>,
+                   tc_grid(rows, groups, t.num_sms, wide ? 1 : 2), kTcRows * groups * (wide ? 1 : kTrainSplit),
+                   tc_train_smem(groups), s, f);
     TcWgradArgs w;
     std::memset(&w, 0, sizeof(w));
     for (int l = 0; l < kLayers; l++) {
@@ -850,7 +877,7 @@ tt_status tc_infer(const uint16_t *w_tc, const float *rec, long long n_host, con
     a.err = err;
     const long long rows = n_dev ? cap : n_host;
     const int grid = tc_grid(rows, kTcGroups, num_sms, 1);
-    k_mlp_forward_tc<false, kTcGroups><<<grid, kTcThreads, kTcSmem, s>>>(a);
+    k_mlp_forward_tc<false, kTcGroups, 1><<<grid, kTcThreads, kTcSmem, s>>>(a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(TT_ERR_CUDA, std::string("tensor-core MLP: ") + cudaGetErrorString(e));
     return TT_OK;
