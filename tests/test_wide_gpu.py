@@ -122,3 +122,34 @@ def test_page_locked_host_rays(offset):
             want = hits(dbvh, torch.from_numpy(rays).cuda(), DeviceBVH.VARIANT_DYNAMIC, closest, False)
             dbvh.set_variant(DeviceBVH.VARIANT_SORTED)
             assert np.array_equal(h_hits, want), (n, closest)
+
+
+@pytest.mark.parametrize("n", [33, 5000, (1 << 20) + 1])
+def test_calls_captured_calls_and_streams_in_any_order(n):
+    """Direct calls, replays of a captured call and calls on other streams use work counters of their own."""
+    sc, alpha, leaf, extent = SCENES["spheres"]()
+    dbvh = DeviceBVH(BVHCompact.build(sc, alpha, 1, leaf))
+    rays = torch.from_numpy(rays_for(extent, 6, n)).cuda()
+    few = rays[:17].contiguous()
+    ref, ref_few = hits(dbvh, rays, DeviceBVH.VARIANT_DYNAMIC, True, False), hits(dbvh, few, DeviceBVH.VARIANT_DYNAMIC, True, False)
+    dbvh.set_variant(DeviceBVH.VARIANT_SORTED)
+    h, g, o = (torch.full((k, 2), 77, dtype=torch.int32, device="cuda") for k in (n, n, 17))
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    dbvh.intersect(rays, h)  # allocates what the call needs
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        dbvh.intersect(rays, g, stream=side.cuda_stream)
+    for k in range(7):
+        for t in (h, g, o):
+            t.fill_(77)
+        torch.cuda.synchronize()
+        for _ in range(k % 3):
+            dbvh.intersect(few, o)
+        graph.replay()
+        dbvh.intersect(rays, h)
+        torch.cuda.synchronize()
+        dbvh.intersect(few, o, stream=side.cuda_stream)
+        side.synchronize()
+        dbvh.check()
+        assert np.array_equal(h.cpu().numpy(), ref) and np.array_equal(g.cpu().numpy(), ref), k
+        assert np.array_equal(o.cpu().numpy(), ref_few), k

@@ -74,7 +74,8 @@ struct DeviceBVH {
     void *wide = nullptr;          // the four-wide form: nodes, then triangle pairs
     size_t bytes = 0;
     uint32_t num_nodes = 0, num_verts = 0;
-    unsigned long long *scratch = nullptr;  // [0] work counter, [1] error word (low 32 bits)
+    unsigned long long *scratch = nullptr;  // work counters and the error word (kScratch...)
+    unsigned turn[4] = {0, 0, 0, 0};        // of the four-wide launches' counters, per work-counter slot
     int device = 0;
     int num_sms = 0;
     int blocks_per_sm[kNumKernels] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
@@ -101,9 +102,14 @@ struct DeviceBVH {
 };
 
 // Scratch words (64-bit) of a DeviceBVH: [0] work counter of the caller-stream launches,
-// [1] error word shared by all launches, [2..4] work counters of the three pipeline streams.
+// [1] error word shared by all launches, [2..4] work counters of the three pipeline streams: each set to 0
+// in front of the launch that uses it. The four-wide launches outside stream capture do without that
+// operation (1.6 us of a small call): every work-counter slot has kTurns counters from kScratchTurns on, a
+// launch takes the next one and sets to 0 the one whose turn comes two launches later.
 constexpr int kScratchErr = 1;
 constexpr int kScratchPipe = 2;
+constexpr int kScratchTurns = 8;
+constexpr unsigned kTurns = 4;
 
 struct TraceArgs {
     BvhView bvh;
@@ -111,6 +117,7 @@ struct TraceArgs {
     int64_t n;
     void *hits;
     unsigned long long *counter;
+    unsigned long long *clear;  // a counter to set to 0 for a later launch, or nullptr
     unsigned int *err;
     // TT_VARIANT_SORTED, when order_built(order_state): the ray in each place of the order
     const int *order_src;
@@ -155,7 +162,8 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
     WideRays<kHost ? kTraceBlock : 0> rays;
     rays.sh = sh_rays + (kHost ? threadIdx.x : 0);
     const bool use_perm = kPerm && a.order_state && order_built(a.order_state);
-    unsigned *queue = reinterpret_cast<unsigned *>(a.counter);  // the next ray; blocks done
+    unsigned *queue = reinterpret_cast<unsigned *>(a.counter);  // the next ray
+    if (a.clear && blockIdx.x == 0 && threadIdx.x == 0) *a.clear = 0ull;
     trace_queue<kClosest, kWideInner>(
         stack, rays, a.bvh, (unsigned)a.n, err,
         [&](int count) {
@@ -170,15 +178,6 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
         },
         [&](unsigned, unsigned i, const TraceResult &tr) { store_hit<kExt>(a, a.hits, i, tr); });
     if (err) atomicOr(a.err, err);
-    // the last block to finish leaves the counter at 0 for the next launch (every claim is made by then)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(queue + 1, 1u) == gridDim.x - 1) {
-            queue[0] = 0u;
-            queue[1] = 0u;
-        }
-    }
 }
 
 // The two-wide tree: each warp claims 32 consecutive rays. kSpec: with the reference's warp vote.
@@ -431,6 +430,7 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     a.n = n;
     a.hits = d_hits;
     a.counter = d.scratch + counter_slot;
+    a.clear = nullptr;
     a.err = reinterpret_cast<unsigned int *>(d.scratch + kScratchErr);
     a.order_src = nullptr;
     a.order_state = nullptr;
@@ -441,11 +441,11 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
         (variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC) && !host_rays && n >= kOrderMinRays;
     if (host_rays) variant = VARIANT_HOST;
     if (!d.view.wide_nodes && variant != VARIANT_DYNAMIC && variant != VARIANT_WARP_VOTE) variant = VARIANT_TWO_WIDE;
+    // per work-counter slot: the ordering scratch, so the pipeline streams never share one, and the turns
+    const int k = counter_slot == 0 ? 0 : 1 + (counter_slot - kScratchPipe) % 3;
+    DeviceBVH &dm = const_cast<DeviceBVH &>(d);
     if (order_rays) {
-        // one scratch per work-counter slot, so the pipeline streams never share one
-        const int k = counter_slot == 0 ? 0 : 1 + (counter_slot - kScratchPipe) % 3;
         const size_t need = reorder_scratch_bytes(n);
-        DeviceBVH &dm = const_cast<DeviceBVH &>(d);
         if (dm.order_bytes[k] < need) {
             if (dm.order[k]) cudaFree(dm.order[k]);
             dm.order[k] = nullptr;
@@ -472,17 +472,27 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     int64_t blocks = (int64_t)d.num_sms * d.blocks_per_sm[variant];
     if (blocks > max_useful) blocks = max_useful;
     if (blocks < 1) blocks = 1;
-    // the four-wide kernels find their counter at 0 and leave it so
-    const bool counts_up = variant == VARIANT_TWO_WIDE || variant == VARIANT_DYNAMIC || variant == VARIANT_WARP_VOTE;
-    if (counts_up) TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
+    const bool two_wide = variant == VARIANT_TWO_WIDE || variant == VARIANT_DYNAMIC || variant == VARIANT_WARP_VOTE;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!two_wide && stream && stream != cudaStreamLegacy && cudaStreamIsCapturing(stream, &capture) != cudaSuccess)
+        cudaGetLastError();  // (the legacy stream cannot be captured)
+    // a captured launch runs again without the launches around it, so its counter is set to 0 with it
+    const bool turns = !two_wide && capture == cudaStreamCaptureStatusNone;
+    if (turns) {
+        unsigned long long *c = d.scratch + kScratchTurns + kTurns * k;
+        a.counter = c + dm.turn[k] % kTurns;
+        a.clear = c + (dm.turn[k] + 2) % kTurns;
+    } else {
+        TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
+    }
     cudaError_t le;
-    const bool chained = order_rays && !counts_up;
+    const bool chained = order_rays && turns;
     if (closest) le = ext ? launch_variant<true, true>(d, variant, (unsigned)blocks, chained, stream, a)
                           : launch_variant<true, false>(d, variant, (unsigned)blocks, chained, stream, a);
     else le = ext ? launch_variant<false, true>(d, variant, (unsigned)blocks, chained, stream, a)
                   : launch_variant<false, false>(d, variant, (unsigned)blocks, chained, stream, a);
     TT_CUDA(le);
-    if (counts_up) TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
+    if (turns) dm.turn[k]++;
     return TT_OK;
 }
 
