@@ -13,7 +13,7 @@
 // tree) and the bounds of tt_wide.h; costs from the bottom up, the second child to arrive going on
 // with the parent; which nodes are wide nodes, their depth and their triangle pairs; their places,
 // the tree's top levels first and breadth first, the rest in about the file's depth-first order;
-// the records. The host reads totals twice, then allocates the records. Everything
+// the records. The host reads the totals once, then allocates the records. Everything
 // moves at memory speed: uploading the 2,097,152-triangle terrain (765,188 two-wide nodes), arrays and
 // conversion, takes 3.0 ms (a conversion on one host thread took 59 ms by itself).
 #include <cuda_runtime.h>
@@ -28,6 +28,9 @@ namespace tt {
 namespace {
 
 constexpr uint32_t kNoParent = 0xffffffffu;
+// A scene of some thousand nodes meets more SMs than with 256 (uploading 20,492 triangles, one read-back
+// less as well: 368 to 344 us; 131,072 triangles 550 to 513; 64: 353 and 533).
+constexpr int kBuildBlock = 128;
 constexpr int kDepths = 128;  // depth buckets; deeper trees stay two-wide anyway (kWideStack)
 
 struct Totals {
@@ -40,6 +43,11 @@ struct Totals {
     uint32_t cursor[kDepths];  // places given out, by bucket
     uint32_t pair_cursor;
 };
+
+// No fault found and every node met, below the stack's depth.
+__host__ __device__ inline bool convertible(const Totals &t, uint32_t count) {
+    return !t.bad && t.done == count && t.need <= (uint32_t)kWideStack;
+}
 
 struct Build {
     const float4 *nodes, *verts;
@@ -71,7 +79,7 @@ __device__ __forceinline__ float area(const Box &a, const Box &b) {
 }
 
 // (1) parents; bounds of the planes
-__global__ void __launch_bounds__(256) k_wide_parents(Build b) {
+__global__ void __launch_bounds__(kBuildBlock) k_wide_parents(Build b) {
     bool bad = false, neg = false;
     for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < b.count; n += gridDim.x * blockDim.x) {
         Box box[2];
@@ -100,7 +108,7 @@ __global__ void __launch_bounds__(256) k_wide_parents(Build b) {
 }
 
 // (2) costs, from the nodes without inner children up
-__global__ void __launch_bounds__(256) k_wide_costs(Build b) {
+__global__ void __launch_bounds__(kBuildBlock) k_wide_costs(Build b) {
     if (b.tot->bad) return;
     uint32_t done = 0;
     for (uint32_t start = blockIdx.x * blockDim.x + threadIdx.x; start < b.count; start += gridDim.x * blockDim.x) {
@@ -205,9 +213,9 @@ __device__ __forceinline__ void wide_slots(const Build &b, uint32_t n, int32_t r
 
 // (3) wide nodes, their depths and pairs. index: 1 for a wide node, else 0. A node is taken in when
 // its parent is a wide node and takes it; up a chain of taken links wide nodes alternate.
-__global__ void __launch_bounds__(256) k_wide_roots(Build b) {
+__global__ void __launch_bounds__(kBuildBlock) k_wide_roots(Build b) {
     __shared__ uint32_t s_depth[kDepths];
-    if (b.tot->bad) return;
+    if (!convertible(*b.tot, b.count)) return;
     for (int d = threadIdx.x; d < kDepths; d += blockDim.x) s_depth[d] = 0;
     __syncthreads();
     unsigned long long pairs = 0;
@@ -249,7 +257,7 @@ struct Buckets {
 };
 
 // (4) places
-__global__ void __launch_bounds__(256) k_wide_places(Build b, Buckets k) {
+__global__ void __launch_bounds__(kBuildBlock) k_wide_places(Build b, Buckets k) {
     for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < b.count; n += gridDim.x * blockDim.x) {
         if (!b.index[n]) continue;
         const uint32_t q = k.bucket[b.depth[n]];
@@ -264,7 +272,7 @@ __global__ void __launch_bounds__(256) k_wide_places(Build b, Buckets k) {
 }
 
 // (5) records; the leaves' pairs in the order the threads ask for them
-__global__ void __launch_bounds__(256) k_wide_records(Build b, char *nodes, uint32_t num_nodes, char *pairs,
+__global__ void __launch_bounds__(kBuildBlock) k_wide_records(Build b, char *nodes, uint32_t num_nodes, char *pairs,
                                                       uint32_t num_pairs) {
     for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < b.count; n += gridDim.x * blockDim.x) {
         const uint32_t place = b.index[n];
@@ -332,23 +340,21 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
     b.depth = reinterpret_cast<uint8_t *>(take(align(n)));
     b.need = reinterpret_cast<uint16_t *>(take(align(2 * n)));
     b.tot = reinterpret_cast<Totals *>(take(align(sizeof(Totals))));
-    const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)num_sms * 8);
+    const unsigned grid = (unsigned)std::min<size_t>((n + kBuildBlock - 1) / kBuildBlock, (size_t)num_sms * 2048 / kBuildBlock);
     Totals t;
     auto run = [&]() -> cudaError_t {
         cudaError_t c = cudaMemsetAsync(b.parent, 0xff, words, nullptr);
         if (c == cudaSuccess) c = cudaMemsetAsync(b.arrived, 0, words, nullptr);
         if (c == cudaSuccess) c = cudaMemsetAsync(b.tot, 0, sizeof(Totals), nullptr);
         if (c != cudaSuccess) return c;
-        k_wide_parents<<<grid, 256>>>(b);
-        k_wide_costs<<<grid, 256>>>(b);
+        k_wide_parents<<<grid, kBuildBlock>>>(b);
+        k_wide_costs<<<grid, kBuildBlock>>>(b);
+        k_wide_roots<<<grid, kBuildBlock>>>(b);
         c = cudaMemcpy(&t, b.tot, sizeof t, cudaMemcpyDeviceToHost);
         if (c != cudaSuccess) return c;
-        if (t.bad || t.done != b.count || t.need > (uint32_t)kWideStack) return cudaSuccess;  // stays two-wide
-        k_wide_roots<<<grid, 256>>>(b);
-        c = cudaMemcpy(&t, b.tot, sizeof t, cudaMemcpyDeviceToHost);
-        if (c != cudaSuccess) return c;
+        if (!convertible(t, b.count)) return cudaSuccess;  // stays two-wide
         // shared leaves could multiply the triangles
-        if (t.bad || t.pairs > num_verts || t.pairs > kWideIndex || t.depth[kDepths - 1]) return cudaSuccess;
+        if (t.pairs > num_verts || t.pairs > kWideIndex || t.depth[kDepths - 1]) return cudaSuccess;
         // buckets: every depth its own while they fit in top_bytes, then one for all the rest
         const size_t top_nodes = std::max<size_t>(1, top_bytes / kWideNodeBytes);
         Buckets k{};
@@ -367,8 +373,8 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
         c = cudaMalloc(&out.base, nb + pb);
         if (c != cudaSuccess) return c;
         char *nodes = static_cast<char *>(out.base), *pairs = nodes + nb;
-        k_wide_places<<<grid, 256>>>(b, k);
-        k_wide_records<<<grid, 256>>>(b, nodes, (uint32_t)wide, pairs, (uint32_t)t.pairs);
+        k_wide_places<<<grid, kBuildBlock>>>(b, k);
+        k_wide_records<<<grid, kBuildBlock>>>(b, nodes, (uint32_t)wide, pairs, (uint32_t)t.pairs);
         c = cudaGetLastError();
         if (c == cudaSuccess) c = cudaStreamSynchronize(nullptr);
         if (c != cudaSuccess) return c;
