@@ -1,0 +1,81 @@
+"""The device passes that make the four-wide tree at upload, run on the CPU (tests/wide_passes_host.cpp): what they make
+of a tree gives the two-wide traversal's hits, and trees they must leave two-wide are refused before a pass that
+relies on what they lack."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from tests.test_wide_bvh import SCENES, rays_for, soup
+from trenchanttracer_gb300 import BVHCompact, build
+
+ROOT = Path(__file__).resolve().parents[1]
+F = np.float32
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    so = tmp_path_factory.mktemp("passes") / "wide_passes_host.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC",
+                    f"-I{ROOT / 'trenchanttracer_gb300' / 'csrc'}", f"-I{ROOT / 'include'}",
+                    f"-I{build._cuda_home() / 'include'}", str(ROOT / "tests" / "wide_passes_host.cpp"), "-o", str(so)],
+                   check=True)
+    lib = C.CDLL(str(so))
+    lib.wide_passes_trace.restype = C.c_longlong
+    return lib
+
+
+def convert(lib, arrays, rays, closest=1, two_wide=0, top=50):
+    """(wide nodes, stage of refusal, hit slots, t u v as words, error word)"""
+    n = rays.shape[0]
+    addr, tuv = np.empty(n, np.int32), np.empty((n, 3), F)
+    err, stage = C.c_uint(0), C.c_int(0)
+    p = lambda a: C.c_void_p(a.ctypes.data)
+    nodes, verts = np.ascontiguousarray(arrays["nodes"]), np.ascontiguousarray(arrays["vertices"])
+    wide = lib.wide_passes_trace(p(nodes), C.c_longlong(len(nodes)), p(verts), C.c_longlong(len(verts)),
+                                 C.c_longlong(top), p(rays), C.c_longlong(n), C.c_int(closest), C.c_int(two_wide),
+                                 p(addr), p(tuv), C.byref(err), C.byref(stage))
+    return wide, stage.value, addr, tuv.view(np.uint32), err.value
+
+
+@pytest.mark.parametrize("name", sorted(SCENES))
+@pytest.mark.parametrize("top", [1, 50, 1 << 20])
+def test_converted_trees_give_the_two_wide_hits(host, name, top):
+    sc, alpha, leaf, extent = SCENES[name]()
+    arrays = BVHCompact.build(sc, alpha, 1, leaf).arrays()
+    rays = rays_for(extent, 17, 5000)
+    for closest in (1, 0):
+        wide, stage, *got = convert(host, arrays, rays, closest, 0, top)
+        *_, a, b, c = convert(host, arrays, rays, closest, 1)
+        assert wide > 0 and stage == 0
+        assert np.array_equal(got[0], a) and np.array_equal(got[1], b) and got[2] == c
+
+
+def with_node(arrays, left, right):
+    """The tree with one node more, that no other node refers to."""
+    out = {k: v.copy() for k, v in arrays.items()}
+    node = out["nodes"][-4:].copy()
+    node[3, 0], node[3, 1] = left, right
+    out["nodes"] = np.concatenate([out["nodes"], node])
+    return out
+
+
+def test_trees_with_a_node_that_no_node_refers_to_stay_two_wide(host):
+    """Alone, with leaves or with one more such node below it: the passes that follow a node's links to the root
+    must not run."""
+    rays = rays_for(3.0, 5, 2000)
+    base = BVHCompact.build(soup(60, 7, 0.5, 2.0), 1e-5, 1, 1).arrays()
+    leaf = int(base["nodes"][-1, 0]) if base["nodes"][-1, 0] < 0 else ~0
+    n = len(base["nodes"])
+    two = BVHCompact.build(soup(2, 4, 1.0, 3.0), 1e-5, 1, 1).arrays()  # one inner node
+    small = with_node(two, int(two["nodes"][3, 0]), int(two["nodes"][3, 1]))
+    alone = with_node(base, leaf, leaf)
+    over_a_leaf_node = with_node(alone, n, leaf)          # refers to the node that `alone` added
+    ring = with_node(base, n, leaf)                       # refers to itself
+    for arrays in (small, alone, over_a_leaf_node, ring):
+        wide, stage, *got = convert(host, arrays, rays)
+        assert wide == 0 and stage in (1, 2)
+        *_, a, b, c = convert(host, arrays, rays, 1, 1)
+        assert np.array_equal(got[0], a) and np.array_equal(got[1], b) and got[2] == c

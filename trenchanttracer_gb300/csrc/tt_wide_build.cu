@@ -36,7 +36,7 @@ constexpr int kDepths = 128;  // depth buckets; deeper trees stay two-wide anywa
 struct Totals {
     uint32_t bad;       // not a tree, or outside the bounds
     uint32_t neg_zero;  // a box plane at -0.0
-    uint32_t done;      // nodes whose cost is known
+    uint32_t done;      // nodes whose cost is known and which are the root or have a parent
     uint32_t need;      // stack entries the root's traversal may need
     unsigned long long pairs;
     uint32_t depth[kDepths];   // wide nodes by depth
@@ -157,13 +157,17 @@ __global__ void __launch_bounds__(kBuildBlock) k_wide_costs(Build b) {
             b.take[n] = taken;
             const uint32_t need = min(below + slots - 1, 60000u);
             b.need[n] = (uint16_t)need;
-            done++;
             if (n == 0) {
+                done++;
                 b.tot->need = need;
                 break;
             }
+            // A node that no node refers to does not count, so the tree is refused before the passes that
+            // follow every node's links up to the root. (Nodes in a ring never get here: each waits for
+            // the next.)
             const uint32_t up = b.parent[n];
-            if (up == kNoParent) break;  // not reachable from the root (done stays short of count)
+            if (up == kNoParent) break;
+            done++;
             n = up / 2;
             load_node(b.nodes + 4 * (size_t)n, box, ch);
             if (ch[0] >= 0 && ch[1] >= 0) {
@@ -256,6 +260,24 @@ struct Buckets {
     uint32_t bucket[kDepths];  // bucket of each depth
 };
 
+// Buckets: every depth its own while they fit in top_nodes, then one for all the rest. The number of wide
+// nodes.
+inline size_t plan_places(const Totals &t, size_t top_nodes, Buckets &k) {
+    k = Buckets{};
+    size_t wide = 0;
+    int rest = -1;
+    for (int d = 0; d < kDepths; d++) {
+        if (rest < 0 && wide + t.depth[d] > top_nodes) {
+            rest = d;
+            k.first[d] = (uint32_t)wide;
+        }
+        k.bucket[d] = (uint32_t)(rest < 0 ? d : rest);
+        if (rest < 0) k.first[d] = (uint32_t)wide;
+        wide += t.depth[d];
+    }
+    return wide;
+}
+
 // (4) places
 __global__ void __launch_bounds__(kBuildBlock) k_wide_places(Build b, Buckets k) {
     for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < b.count; n += gridDim.x * blockDim.x) {
@@ -311,6 +333,7 @@ __global__ void __launch_bounds__(kBuildBlock) k_wide_records(Build b, char *nod
 
 }  // namespace
 
+#if defined(__CUDACC__)  // the passes above also build as plain C++, for the tests that run them on the CPU
 cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_verts, size_t top_bytes, int num_sms,
                        WideBVH &out) {
     out = WideBVH();
@@ -355,20 +378,9 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
         if (!convertible(t, b.count)) return cudaSuccess;  // stays two-wide
         // shared leaves could multiply the triangles
         if (t.pairs > num_verts || t.pairs > kWideIndex || t.depth[kDepths - 1]) return cudaSuccess;
-        // buckets: every depth its own while they fit in top_bytes, then one for all the rest
         const size_t top_nodes = std::max<size_t>(1, top_bytes / kWideNodeBytes);
-        Buckets k{};
-        size_t wide = 0;
-        int rest = -1;
-        for (int d = 0; d < kDepths; d++) {
-            if (rest < 0 && wide + t.depth[d] > top_nodes) {
-                rest = d;
-                k.first[d] = (uint32_t)wide;
-            }
-            k.bucket[d] = (uint32_t)(rest < 0 ? d : rest);
-            if (rest < 0) k.first[d] = (uint32_t)wide;
-            wide += t.depth[d];
-        }
+        Buckets k;
+        const size_t wide = plan_places(t, top_nodes, k);
         const size_t nb = align(wide * kWideNodeBytes), pb = (size_t)t.pairs * kWidePairBytes;
         c = cudaMalloc(&out.base, nb + pb);
         if (c != cudaSuccess) return c;
@@ -396,5 +408,6 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
     }
     return e;
 }
+#endif
 
 }  // namespace tt
