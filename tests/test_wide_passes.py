@@ -15,14 +15,17 @@ ROOT = Path(__file__).resolve().parents[1]
 F = np.float32
 
 
+def host_library(tmp_path_factory, source, *flags):
+    so = tmp_path_factory.mktemp("host") / (source + ".so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", *flags, f"-I{ROOT / 'tests'}",
+                    f"-I{ROOT / 'trenchanttracer_gb300' / 'csrc'}", f"-I{ROOT / 'include'}",
+                    f"-I{build._cuda_home() / 'include'}", str(ROOT / "tests" / source), "-o", str(so)], check=True)
+    return C.CDLL(str(so))
+
+
 @pytest.fixture(scope="module")
 def host(tmp_path_factory):
-    so = tmp_path_factory.mktemp("passes") / "wide_passes_host.so"
-    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC",
-                    f"-I{ROOT / 'trenchanttracer_gb300' / 'csrc'}", f"-I{ROOT / 'include'}",
-                    f"-I{build._cuda_home() / 'include'}", str(ROOT / "tests" / "wide_passes_host.cpp"), "-o", str(so)],
-                   check=True)
-    lib = C.CDLL(str(so))
+    lib = host_library(tmp_path_factory, "wide_passes_host.cpp")
     lib.wide_passes_trace.restype = C.c_longlong
     return lib
 

@@ -81,14 +81,16 @@ static void trace(const BvhView &v, const float *rays, long long n, int *addr, f
     }
 }
 
-extern "C" {
-// Converts a compact tree (float4 nodes and vertices) and traces n rays through what the passes made, or
-// through the two-wide tree. Returns the number of four-wide nodes, 0 when the tree must stay
-// two-wide, -1 when the passes let one through whose later passes would read out of range. stage: the pass
-// (1 to 5) after which a tree was refused, 0 for none.
-long long wide_passes_trace(const float *nodes, long long num_nodes, const float *verts, long long num_verts,
-                            long long top_nodes, const float *rays, long long n, int closest, int two_wide, int *addr,
-                            float *tuv, unsigned *err, int *stage) {
+struct Form {
+    std::vector<char> nodes, pairs;
+    uint32_t flags = 0;
+    long long wide = 0;  // nodes; 0: refused after pass `stage`; -1: see below
+    int stage = 0;
+};
+
+static Form convert(const float *nodes, long long num_nodes, const float *verts, long long num_verts,
+                    long long top_nodes) {
+    Form f;
     Build b{};
     b.nodes = reinterpret_cast<const float4 *>(nodes);
     b.verts = reinterpret_cast<const float4 *>(verts);
@@ -107,40 +109,67 @@ long long wide_passes_trace(const float *nodes, long long num_nodes, const float
     b.depth = depth.data();
     b.need = need.data();
     b.tot = &t;
-    BvhView v{};
-    v.nodes = b.nodes;
-    v.verts = b.verts;
-    std::vector<char> wide_nodes, wide_pairs;
-    long long wide = 0;
-    *stage = 0;
-    if (!two_wide) {
-        const unsigned blocks = 7;
-        run(blocks, [&] { k_wide_parents(b); });
-        if (t.bad) *stage = 1;
-        run(blocks, [&] { k_wide_costs(b); });
-        if (!*stage && !convertible(t, b.count)) *stage = 2;
-        if (!*stage)  // the third pass follows every node's links up to the root
-            for (uint32_t k = 1; k < b.count; k++)
-                if (parent[k] / 2 >= b.count) return -1;
-        if (!*stage) run(blocks, [&] { k_wide_roots(b); });
-        if (!*stage && (t.bad || t.pairs > b.num_verts || t.depth[kDepths - 1])) *stage = 3;
-        if (!*stage) {
-            Buckets k;
-            wide = (long long)plan_places(t, (size_t)top_nodes, k);
-            wide_nodes.resize((size_t)wide * kWideNodeBytes);
-            wide_pairs.resize((size_t)t.pairs * kWidePairBytes);
-            run(blocks, [&] { k_wide_places(b, k); });
-            run(blocks, [&] {
-                k_wide_records(b, wide_nodes.data(), (uint32_t)wide, wide_pairs.data(), (uint32_t)t.pairs);
-            });
-            if (t.pair_cursor != t.pairs) *stage = 5;
-            v.wide_nodes = wide_nodes.data();
-            v.wide_pairs = wide_pairs.data();
-            v.wide_flags = t.neg_zero ? kWideNegZero : 0u;
+    const unsigned blocks = 7;
+    run(blocks, [&] { k_wide_parents(b); });
+    f.stage = 1;
+    if (t.bad) return f;
+    run(blocks, [&] { k_wide_costs(b); });
+    f.stage = 2;
+    if (!convertible(t, b.count)) return f;
+    for (uint32_t k = 1; k < b.count; k++)  // the third pass follows every node's links up to the root
+        if (parent[k] / 2 >= b.count) {
+            f.wide = -1;
+            return f;
         }
+    run(blocks, [&] { k_wide_roots(b); });
+    f.stage = 3;
+    if (t.bad || t.pairs > b.num_verts || t.depth[kDepths - 1]) return f;
+    Buckets k;
+    f.wide = (long long)plan_places(t, (size_t)top_nodes, k);
+    f.nodes.resize((size_t)f.wide * kWideNodeBytes);
+    f.pairs.resize((size_t)t.pairs * kWidePairBytes);
+    run(blocks, [&] { k_wide_places(b, k); });
+    run(blocks, [&] { k_wide_records(b, f.nodes.data(), (uint32_t)f.wide, f.pairs.data(), (uint32_t)t.pairs); });
+    f.stage = t.pair_cursor == t.pairs ? 0 : 5;
+    f.flags = t.neg_zero ? kWideNegZero : 0u;
+    return f;
+}
+
+extern "C" {
+// Converts a compact tree (float4 nodes and vertices) and traces n rays through what the passes made, or
+// through the two-wide tree. Returns the number of four-wide nodes, 0 when the tree must stay
+// two-wide, -1 when the passes let one through whose later passes would read out of range. stage: the pass
+// (1 to 5) after which a tree was refused, 0 for none.
+long long wide_passes_trace(const float *nodes, long long num_nodes, const float *verts, long long num_verts,
+                            long long top_nodes, const float *rays, long long n, int closest, int two_wide, int *addr,
+                            float *tuv, unsigned *err, int *stage) {
+    Form f;
+    if (!two_wide) f = convert(nodes, num_nodes, verts, num_verts, top_nodes);
+    *stage = f.stage;
+    if (f.wide < 0) return f.wide;
+    BvhView v{};
+    v.nodes = reinterpret_cast<const float4 *>(nodes);
+    v.verts = reinterpret_cast<const float4 *>(verts);
+    if (f.wide) {
+        v.wide_nodes = f.nodes.data();
+        v.wide_pairs = f.pairs.data();
+        v.wide_flags = f.flags;
     }
     if (closest) trace<true>(v, rays, n, addr, tuv, err);
     else trace<false>(v, rays, n, addr, tuv, err);
-    return wide;
+    return f.wide;
+}
+
+// The four-wide form alone; out[0] nodes, out[1] pairs (kept until the next call), sizes in bytes, flags.
+long long wide_passes_form(const float *nodes, long long num_nodes, const float *verts, long long num_verts,
+                           long long top_nodes, const char **out, long long *bytes, unsigned *flags) {
+    static Form f;
+    f = convert(nodes, num_nodes, verts, num_verts, top_nodes);
+    out[0] = f.nodes.data();
+    out[1] = f.pairs.data();
+    bytes[0] = (long long)f.nodes.size();
+    bytes[1] = (long long)f.pairs.size();
+    *flags = f.flags;
+    return f.wide;
 }
 }

@@ -16,7 +16,9 @@
 namespace tt {
 
 __device__ __forceinline__ void chain_begin() {
+#if defined(__CUDACC__)
     asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
 }
 
 template <class... P, class... A>

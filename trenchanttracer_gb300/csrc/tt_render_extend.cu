@@ -48,9 +48,7 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
         },
         [&](unsigned place) {
             const bool srt = kPrefix ? (int)place < n_sorted : ordered;
-            if (!srt) return place;
-            const unsigned q = (unsigned)a.order.src[place];
-            return q < (unsigned)n ? q : place;  // (always, with a consistent ordering)
+            return srt ? ordered_slot(a.order.src, place, (unsigned)n_sorted, err) : place;
         },
         [&](unsigned q, float4 &r0, float4 &r1) {
             r0 = a.ps.ray[cur][2 * (size_t)q];
@@ -64,8 +62,14 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
                 analytic_hit(a, lanes, true, V3(r0.x, r0.y, r0.z), V3(r0.w, r1.x, r1.y), r1.z, t, prim, hu, hv, false);
             }
             const float4 h = make_float4(t, hu, hv, __int_as_float(prim));
-            if (kPrefix ? (int)q < n_sorted : ordered) a.order.hits[a.order.pos[q]] = h;
-            else a.ps.hit[q] = h;
+            if (kPrefix ? (int)q < n_sorted : ordered) {
+                const int p = a.order.pos[q];
+                // (k_order_gather_hits lets a path whose place is out of range miss)
+                if ((unsigned)p < (unsigned)n_sorted) a.order.hits[p] = h;
+                else err |= kErrOrder;
+            } else {
+                a.ps.hit[q] = h;
+            }
         });
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.stats + 0, (unsigned long long)n);
     if (err) atomicOr(a.err, err);
@@ -91,9 +95,7 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
             return (unsigned)__shfl_sync(0xffffffffu, base, 0);
         },
         [&](unsigned place) {
-            if (!ordered) return place;
-            const unsigned j = (unsigned)a.shadow_order.src[place];
-            return j < (unsigned)n ? j : place;  // (always, with a consistent ordering)
+            return ordered ? ordered_slot(a.shadow_order.src, place, (unsigned)n, err) : place;
         },
         [&](unsigned j, float4 &r0, float4 &r1) {
             r0 = a.ps.shadow_ray[2 * (size_t)j];

@@ -30,7 +30,7 @@ constexpr int64_t kOrderMinRays = 1 << 20;
 // pool) take 3.35 ms, from 2M on 2.88, from 4M on 2.65; 960 x 540 x 16 samples of 400 spheres 15.5, 15.2
 // and 15.2 ms.
 constexpr int64_t kOrderMinQueue = 1 << 22;
-// Error-word bit: a sorted slot came out of range (the ray's hit is then left unwritten).
+// Error-word bit: a slot of the order came out of range (see ordered_slot, and k_order_scatter).
 constexpr uint32_t kErrOrder = 4u;
 
 // The origin grid: q_k = clamp((o_k - lo_k) * scale_k, 0, cells_k - 1), and bit j of q_k goes to
@@ -115,5 +115,16 @@ tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const fl
 // equal keys (the rays are coherent already: camera rays share one origin cell and neighbouring
 // pixels one direction cell) or too few rays came; they are then traced in their own order.
 __device__ __forceinline__ bool order_built(const unsigned long long *state) { return state[3] == 1ull; }
+
+// The ray in a place of the order of rays 0 .. n - 1, for the kernels that take their rays through it. An order
+// that is no permutation (two calls that overlap on one scratch make one, and places that the scatter left out
+// hold what was there) is reported, and such a place keeps its own ray: a ray it leaves out has its hit
+// unwritten, and no access goes beyond the caller's buffers.
+__host__ __device__ inline unsigned ordered_slot(const int *src, unsigned place, unsigned n, uint32_t &err) {
+    const unsigned i = (unsigned)src[place];
+    if (i < n) return i;
+    err |= kErrOrder;
+    return place;
+}
 
 }  // namespace tt

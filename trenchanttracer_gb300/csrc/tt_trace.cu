@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
             if (lane == 0) b = atomicAdd(queue, (unsigned)count);
             return __shfl_sync(0xffffffffu, b, 0);
         },
-        [&](unsigned place) { return use_perm ? (unsigned)a.order_src[place] : place; },
+        [&](unsigned place) { return use_perm ? ordered_slot(a.order_src, place, (unsigned)a.n, err) : place; },
         [&](unsigned i, float4 &r0, float4 &r1) {
             r0 = __ldg(a.rays + 2 * (size_t)i);
             r1 = __ldg(a.rays + 2 * (size_t)i + 1);
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kTraceBlock) trace_warp_kernel(TraceArgs a) {
         if ((int64_t)base >= a.n) break;
         const int64_t slot = (int64_t)base + lane;
         if (slot < a.n) {
-            const int64_t i = use_perm ? (int64_t)__ldg(a.order_src + slot) : slot;
+            const int64_t i = use_perm ? (int64_t)ordered_slot(a.order_src, (unsigned)slot, (unsigned)a.n, err) : slot;
             const float4 r0 = __ldg(a.rays + 2 * i), r1 = __ldg(a.rays + 2 * i + 1);
             TravState s;
             trav_init(s, stack, r0, r1);

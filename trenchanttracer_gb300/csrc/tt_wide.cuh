@@ -474,7 +474,7 @@ __device__ __forceinline__ TraceResult traverse_wide(Stack &stack, const BvhView
     return wide_result(s);
 }
 
-#if defined(__CUDACC__)
+#if defined(__CUDACC__) || defined(TT_WARP_ON_HOST)  // (tests run it on emulated warps)
 // Lanes at inner nodes below which a warp turns to its leaves and to new rays: 4M camera rays / 4M
 // bounces on the 2,097,152-triangle terrain take 0.52 / 0.98 ms with 2, 0.50 / 0.90 with 4, 0.49 / 0.86
 // with 8, 0.50 / 0.86 with 10, 0.53 / 0.89 with 16.
