@@ -82,3 +82,43 @@ def test_trees_with_a_node_that_no_node_refers_to_stay_two_wide(host):
         assert wide == 0 and stage in (1, 2)
         *_, a, b, c = convert(host, arrays, rays, 1, 1)
         assert np.array_equal(got[0], a) and np.array_equal(got[1], b) and got[2] == c
+
+
+def run_of(triangles, g):
+    """`triangles` triangles behind one another and the terminator, as vertex words."""
+    v = np.zeros((3 * triangles + 1, 4), np.int32)
+    v[:-1, :3] = g.normal(size=(3 * triangles, 3)).astype(F).view(np.int32)
+    v[-1, 0] = -2**31
+    return v
+
+
+@pytest.mark.parametrize("leaves,triangles", [(2, 1), (2, 40), (300, 2000)])
+def test_trees_whose_leaves_overlap_stay_two_wide(host, leaves, triangles):
+    """Leaf addresses of a file may point into one another's triangles. A pass that walked each from its address to
+    its end would take leaves times triangles steps, so the first triangle met twice ends it."""
+    g = np.random.default_rng(3)
+    base = BVHCompact.build(soup(leaves, 7, 0.5, 2.0), 1e-5, 1, 1).arrays()
+    child = base["nodes"][3::4, :2]  # a view: the children's addresses
+    at = np.arange((child < 0).sum(), dtype=np.int32)
+    base["vertices"] = run_of(triangles, g)
+    child[child < 0] = ~(3 * (at % triangles))
+    base["nodes"] = base["nodes"].copy()
+    rays = rays_for(3.0, 5, 200)
+    wide, stage, *got = convert(host, base, rays)
+    assert wide == 0 and stage == 3
+    *_, a, b, c = convert(host, base, rays, 1, 1)
+    assert np.array_equal(got[0], a) and np.array_equal(got[1], b) and got[2] == c
+
+
+@pytest.mark.parametrize("triangles,accepted", [(8192, True), (8193, False)])
+def test_a_leaf_of_very_many_triangles_stays_two_wide(host, triangles, accepted):
+    """One thread walks a leaf, so its length is bounded."""
+    g = np.random.default_rng(4)
+    base = BVHCompact.build(soup(2, 4, 1.0, 3.0), 1e-5, 1, 1).arrays()
+    base["vertices"] = np.concatenate([run_of(triangles, g), run_of(1, g)])
+    base["nodes"][3, :2] = [~0, ~(3 * triangles + 1)]
+    rays = rays_for(3.0, 5, 50)
+    wide, stage, *got = convert(host, base, rays)
+    assert (wide > 0 and stage == 0) if accepted else (wide == 0 and stage == 3)
+    *_, a, b, c = convert(host, base, rays, 1, 1)
+    assert np.array_equal(got[0], a) and np.array_equal(got[1], b) and got[2] == c

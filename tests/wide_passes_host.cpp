@@ -100,6 +100,7 @@ static Form convert(const float *nodes, long long num_nodes, const float *verts,
     std::vector<float> cost(b.count, -1.0f);
     std::vector<uint8_t> take(b.count, 0xee), depth(b.count, 0xee);
     std::vector<uint16_t> need(b.count, 0xeeee);
+    std::vector<uint32_t> met(leaf_words(b.num_verts), 0);
     Totals t{};
     b.parent = parent.data();
     b.arrived = arrived.data();
@@ -108,6 +109,7 @@ static Form convert(const float *nodes, long long num_nodes, const float *verts,
     b.take = take.data();
     b.depth = depth.data();
     b.need = need.data();
+    b.met = met.data();
     b.tot = &t;
     const unsigned blocks = 7;
     run(blocks, [&] { k_wide_parents(b); });

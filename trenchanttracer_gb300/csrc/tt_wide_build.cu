@@ -31,6 +31,7 @@ constexpr uint32_t kNoParent = 0xffffffffu;
 // A scene of some thousand nodes meets more SMs than with 256 (uploading 20,492 triangles, one read-back
 // less as well: 368 to 344 us; 131,072 triangles 550 to 513; 64: 353 and 533).
 constexpr int kBuildBlock = 128;
+constexpr uint32_t kLeafTriangles = 8192;  // of a leaf; a tree with a longer one stays two-wide
 constexpr int kDepths = 128;  // depth buckets; deeper trees stay two-wide anyway (kWideStack)
 
 struct Totals {
@@ -57,8 +58,10 @@ struct Build {
     uint32_t *arrived, *index;
     uint8_t *take, *depth;
     uint16_t *need;
+    uint32_t *met;  // a bit per vertex slot: the triangle that starts there is in a leaf already
     Totals *tot;
 };
+__host__ __device__ inline size_t leaf_words(uint32_t num_verts) { return (size_t)num_verts / 32 + 1; }
 
 struct Box {
     float lo[3], hi[3];
@@ -182,16 +185,21 @@ __global__ void __launch_bounds__(kBuildBlock) k_wide_costs(Build b) {
 
 __device__ __forceinline__ bool is_terminator(const float4 &v) { return __float_as_uint(v.x) == 0x80000000u; }
 
-// Pairs of the leaf at slot `slot`; 0 for one that is not closed or outside the bounds.
+// Pairs of the leaf at slot `slot`; 0 for one that is not closed or outside the bounds, and, first time round,
+// for one that shares a triangle with another leaf or is longer than one thread should walk. Leaves of
+// a file may overlap: without the marks the walks would take leaves times triangles steps.
+template <bool kFirst>
 __device__ uint32_t leaf_pairs(const Build &b, uint32_t slot) {
     uint32_t tris = 0;
     for (; slot < b.num_verts; slot += 3, tris++) {
         const float4 v0 = b.verts[slot];
         if (is_terminator(v0)) return max(1u, (tris + 1) / 2);
+        if (kFirst && tris == kLeafTriangles) return 0;
         if (slot + 3 >= b.num_verts) return 0;
         const float4 v1 = b.verts[slot + 1], v2 = b.verts[slot + 2];
         for (float c : {v0.x, v0.y, v0.z, v1.x, v1.y, v1.z, v2.x, v2.y, v2.z})
             if (!(fabsf(c) <= kWideCoordMax)) return 0;
+        if (kFirst && (atomicOr(b.met + slot / 32, 1u << slot % 32) >> slot % 32 & 1u)) return 0;
     }
     return 0;
 }
@@ -243,7 +251,7 @@ __global__ void __launch_bounds__(kBuildBlock) k_wide_roots(Build b) {
         wide_slots(b, n, ref, box);
         for (int s = 0; s < 4; s++)
             if (ref[s] < 0) {
-                const uint32_t p = leaf_pairs(b, (uint32_t)~ref[s]);
+                const uint32_t p = leaf_pairs<true>(b, (uint32_t)~ref[s]);
                 bad |= p == 0;
                 pairs += p;
             }
@@ -305,7 +313,7 @@ __global__ void __launch_bounds__(kBuildBlock) k_wide_records(Build b, char *nod
         float *w = reinterpret_cast<float *>(nodes + (size_t)(place - 1) * kWideNodeBytes);
         uint32_t own[4], sum = 0;
         for (int s = 0; s < 4; s++) {
-            own[s] = ref[s] < 0 ? leaf_pairs(b, (uint32_t)~ref[s]) : 0u;
+            own[s] = ref[s] < 0 ? leaf_pairs<false>(b, (uint32_t)~ref[s]) : 0u;
             sum += own[s];
         }
         uint32_t first = sum ? atomicAdd(&b.tot->pair_cursor, sum) : 0u;
@@ -344,9 +352,9 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
     b.num_verts = num_verts;
     if (b.count == 0 || num_nodes % 4 || b.count > kWideIndex) return cudaSuccess;
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t n = b.count, words = align(4 * n);
+    const size_t n = b.count, words = align(4 * n), met = align(4 * leaf_words(num_verts));
     char *work = nullptr;
-    cudaError_t e = cudaMalloc(&work, 4 * words + 2 * align(n) + align(2 * n) + align(sizeof(Totals)));
+    cudaError_t e = cudaMalloc(&work, 4 * words + 2 * align(n) + align(2 * n) + met + align(sizeof(Totals)));
     if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // no room for the conversion: two-wide
     if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
     char *p = work;
@@ -357,18 +365,18 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
     };
     b.parent = reinterpret_cast<uint32_t *>(take(words));
     b.arrived = reinterpret_cast<uint32_t *>(take(words));
+    b.met = reinterpret_cast<uint32_t *>(take(met));  // (cleared together with arrived and tot)
+    b.tot = reinterpret_cast<Totals *>(take(align(sizeof(Totals))));
     b.cost = reinterpret_cast<float *>(take(words));
     b.index = reinterpret_cast<uint32_t *>(take(words));
     b.take = reinterpret_cast<uint8_t *>(take(align(n)));
     b.depth = reinterpret_cast<uint8_t *>(take(align(n)));
     b.need = reinterpret_cast<uint16_t *>(take(align(2 * n)));
-    b.tot = reinterpret_cast<Totals *>(take(align(sizeof(Totals))));
     const unsigned grid = (unsigned)std::min<size_t>((n + kBuildBlock - 1) / kBuildBlock, (size_t)num_sms * 2048 / kBuildBlock);
     Totals t;
     auto run = [&]() -> cudaError_t {
         cudaError_t c = cudaMemsetAsync(b.parent, 0xff, words, nullptr);
-        if (c == cudaSuccess) c = cudaMemsetAsync(b.arrived, 0, words, nullptr);
-        if (c == cudaSuccess) c = cudaMemsetAsync(b.tot, 0, sizeof(Totals), nullptr);
+        if (c == cudaSuccess) c = cudaMemsetAsync(b.arrived, 0, words + met + align(sizeof(Totals)), nullptr);
         if (c != cudaSuccess) return c;
         k_wide_parents<<<grid, kBuildBlock>>>(b);
         k_wide_costs<<<grid, kBuildBlock>>>(b);
@@ -376,7 +384,7 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
         c = cudaMemcpy(&t, b.tot, sizeof t, cudaMemcpyDeviceToHost);
         if (c != cudaSuccess) return c;
         if (!convertible(t, b.count)) return cudaSuccess;  // stays two-wide
-        // shared leaves could multiply the triangles
+        // (pairs: at most one per vertex slot, with every triangle in one leaf)
         if (t.pairs > num_verts || t.pairs > kWideIndex || t.depth[kDepths - 1]) return cudaSuccess;
         const size_t top_nodes = std::max<size_t>(1, top_bytes / kWideNodeBytes);
         Buckets k;

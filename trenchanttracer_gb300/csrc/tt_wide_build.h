@@ -21,9 +21,9 @@ struct WideBVH {
 // Makes the four-wide form of the device arrays of `two` (num_nodes and num_verts float4s). out.nodes
 // stays nullptr when the tree must stay two-wide: not a tree with every node reachable from the root, a
 // box or vertex outside the bounds of tt_wide.h, an inverted box, a child's box that sticks out
-// of its parent's, a leaf that is not closed, a stack need above kWideStack, or
-// no device memory for it. Works on the legacy
-// stream and waits for it.
+// of its parent's, a leaf that is not closed, shares a triangle with another or is longer than
+// kLeafTriangles, a stack need above kWideStack, or no device memory for it. Works on the legacy stream
+// and waits for it.
 cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_verts, size_t top_bytes, int num_sms,
                        WideBVH &out);
 
