@@ -219,7 +219,9 @@ tt_status tt_dbvh_autotune(tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_hit
 
 /* intersect(ray, bvh, needClosestHit) (include/geometry/IntersectKernel.cuh:78-296) over n
  * rays in device memory; hits are written to device memory. closest = 1 is the closest hit,
- * 0 the any hit (first accepted triangle in traversal order). */
+ * 0 the any hit (first accepted triangle in traversal order). Calls on one `bvh` may be issued to any
+ * streams in any order, but must not run at the same time: they share a work counter and the
+ * ordering's scratch (tt_trace_host has its own). */
 tt_status tt_trace(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_hit *d_hits,
                    int32_t closest, void *stream);
 /* as tt_trace, writing the full hit record (material index and interpolated normal). */

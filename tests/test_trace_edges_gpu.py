@@ -42,3 +42,36 @@ def test_file_with_a_node_that_no_node_refers_to(tmp_path):
     ref, got = DeviceBVH(bvh), DeviceBVH(odd)
     for closest in (True, False):
         assert np.array_equal(trace(got, rays, closest), trace(ref, rays, closest))
+
+
+@pytest.mark.parametrize("n", [1000, 40000, (1 << 20) + 1])
+def test_calls_whose_streams_run_in_another_order_than_they_were_issued(n):
+    """A call that waits in its stream while later calls on another stream come and go: each traces all its rays. The
+    small set needs no counter; the larger ones' calls do not run at the same time."""
+    bvh, extent = tree("spheres")
+    dbvh = DeviceBVH(bvh)
+    rays = torch.from_numpy(rays_for(extent, 6, n)).cuda()
+    h_rays, h_hits = torch.empty(n, 8).pin_memory().numpy(), torch.empty(n, 2, dtype=torch.int32).pin_memory().numpy()
+    h_rays[:] = rays.cpu().numpy()
+    ref = trace(dbvh, rays)
+    late, early = torch.cuda.Stream(), torch.cuda.Stream()
+    waiting = torch.full((n, 2), -7, dtype=torch.int32, device="cuda")
+    others = [torch.full((n, 2), -7, dtype=torch.int32, device="cuda") for _ in range(7)]
+    for _ in range(5):
+        trace(dbvh, rays)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(late):
+        torch.cuda._sleep(400_000_000)  # a fifth of a second
+    dbvh.intersect(rays, waiting, stream=late.cuda_stream)
+    for h in others:
+        dbvh.intersect(rays, h, stream=early.cuda_stream)
+    early.synchronize()
+    h_hits[:] = -7
+    dbvh.intersect_host(h_rays, h_hits, stream=early.cuda_stream)
+    assert not late.query()  # (else the call came first and shows nothing)
+    for h in others:
+        assert np.array_equal(h.cpu().numpy(), ref)
+    assert np.array_equal(h_hits, ref)
+    late.synchronize()
+    assert np.array_equal(waiting.cpu().numpy(), ref)
+    dbvh.check()

@@ -21,10 +21,12 @@ static void trace(int kernel, unsigned blocks, const TraceArgs &a) {
 extern "C" {
 // Traces n rays by a kernel (0: the default, 1: without shared stack, 2: over host rays, 3: two-wide in the
 // default's place, 4: two-wide with per-lane claims) in a grid of `blocks` warps, over a two-wide tree and,
-// unless wide_nodes is null, its four-wide form. order: the ray in each place, or null. Returns the error word.
+// unless wide_nodes is null, its four-wide form. order: the ray in each place, or null. share: the places dealt
+// to each warp (0: claimed from a counter). Returns the error word.
 __attribute__((visibility("default"))) unsigned trace_kernel_host(
     int kernel, unsigned blocks, const float *nodes, const float *verts, const int *tri_idx, const char *wide_nodes,
-    const char *wide_pairs, unsigned wide_flags, const float *rays, long long n, int closest, const int *order, int *hits) {
+    const char *wide_pairs, unsigned wide_flags, const float *rays, long long n, int closest, const int *order, unsigned share,
+    int *hits) {
     unsigned err = 0;
     unsigned long long counter = 0, state[4] = {0, 0, 0, 1};
     TraceArgs a{};
@@ -38,6 +40,7 @@ __attribute__((visibility("default"))) unsigned trace_kernel_host(
     a.n = n;
     a.hits = hits;
     a.counter = &counter;
+    a.share = share;
     a.err = &err;
     a.order_src = order;
     a.order_state = order ? state : nullptr;

@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(kBlock) k_extend(NativeArgs a, int cur) {
     const int n_sorted = ordered ? (kPrefix ? *a.order.n_sorted : n) : 0;
     trace_queue<true, kQueueInner>(
         stack, rays, a.bvh, (unsigned)n, err,
-        [&](int count) {
+        [&](bool, unsigned &count) {
             int base = 0;
-            if (lane == 0) base = atomicAdd(a.ps.counts + 3, count);
+            if (lane == 0) base = atomicAdd(a.ps.counts + 3, (int)count);
             return (unsigned)__shfl_sync(0xffffffffu, base, 0);
         },
         [&](unsigned place) {
@@ -89,9 +89,9 @@ __global__ void __launch_bounds__(kBlock) k_shadow(NativeArgs a) {
     const bool ordered = a.shadow_order.src && order_built(a.shadow_order.state);
     trace_queue<false, kQueueInner>(
         stack, rays, a.bvh, (unsigned)n, err,
-        [&](int count) {
+        [&](bool, unsigned &count) {
             int base = 0;
-            if (lane == 0) base = atomicAdd(a.ps.counts + 4, count);
+            if (lane == 0) base = atomicAdd(a.ps.counts + 4, (int)count);
             return (unsigned)__shfl_sync(0xffffffffu, base, 0);
         },
         [&](unsigned place) {

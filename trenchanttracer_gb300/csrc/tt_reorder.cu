@@ -56,6 +56,7 @@ struct OrderArgs {
     int64_t min_rays;
     unsigned long long *state;
     unsigned *err;
+    unsigned long long *clear;  // a word to set to 0, or nullptr
 };
 
 __device__ __forceinline__ int64_t order_rays(const OrderArgs &a) {
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
     const int64_t tid = (int64_t)blockIdx.x * kOrderBlock + threadIdx.x;
     const int64_t nthreads = (int64_t)gridDim.x * kOrderBlock;
     const int64_t n = order_rays(a);
+    if (a.clear && tid == 0) *a.clear = 0ull;
     if (n < a.min_rays) {  // nothing to look at
         if (tid == 0) a.state[3] = 0ull;
         return;
@@ -285,7 +287,7 @@ static std::atomic<int> g_order_sms[64];  // SMs per device (0 = not yet known)
 
 tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const float lo[3], const float hi[3],
                        void *scratch, size_t state_at, int64_t min_rays, unsigned *err, cudaStream_t s, OrderOut *out,
-                       bool with_pos) {
+                       bool with_pos, unsigned long long *clear) {
     if (n <= 0 || n >= ((int64_t)1 << 31)) return fail(TT_ERR_INVALID, "ray ordering: n must be in 1..2^31-1");
     if (state_at < reorder_state_offset(n) || (state_at & 255))
         return fail(TT_ERR_INVALID, "ray ordering: scratch too small for this many rays");
@@ -321,6 +323,7 @@ tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const fl
     a.sums = reinterpret_cast<unsigned *>(p);
     a.state = reinterpret_cast<unsigned long long *>(static_cast<char *>(scratch) + state_at);
     a.err = err;
+    a.clear = clear;
     const int64_t want = (n + kOrderBlock - 1) / kOrderBlock;
     const unsigned grid = (unsigned)(want < (int64_t)sms * 8 ? want : (int64_t)sms * 8);
     e = launch_chained(k_order_probe, (unsigned)sms * 4, kOrderBlock, 0, s, a);

@@ -101,15 +101,15 @@ struct OrderOut {
 // scratch was made and fixed for its life (reorder_state_offset of the size it was made for).
 // Calls on one scratch must be ordered (one stream). Launches only, no allocation, so a call can
 // be captured in a CUDA graph. Fewer than min_rays rays keep their own order. Device-side errors go
-// to *err as kErrOrder. with_pos: also the
-// inverse permutation.
+// to *err as kErrOrder. with_pos: also the inverse permutation. clear: a word that the first pass sets to 0 (the work
+// counter of the kernel that follows).
 //
 // The rays themselves stay where they are and a trace kernel reads them through src. A copy in
 // sorted order, undone for the hits by a last pass, cost more than the scattered sectors do in a trace
 // that takes 3 % of the memory bandwidth: 4M terrain bounces 840 us with the copy, 790 without.
 tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const float lo[3], const float hi[3],
                        void *scratch, size_t state_at, int64_t min_rays, unsigned *err, cudaStream_t s, OrderOut *out,
-                       bool with_pos = false);
+                       bool with_pos = false, unsigned long long *clear = nullptr);
 
 // Whether this call's rays were ordered: false when more than half of the sampled warps held 32
 // equal keys (the rays are coherent already: camera rays share one origin cell and neighbouring

@@ -75,7 +75,6 @@ struct DeviceBVH {
     size_t bytes = 0;
     uint32_t num_nodes = 0, num_verts = 0;
     unsigned long long *scratch = nullptr;  // work counters and the error word (kScratch...)
-    unsigned turn[4] = {0, 0, 0, 0};        // of the four-wide launches' counters, per work-counter slot
     int device = 0;
     int num_sms = 0;
     int blocks_per_sm[kNumKernels] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
@@ -102,14 +101,11 @@ struct DeviceBVH {
 };
 
 // Scratch words (64-bit) of a DeviceBVH: [0] work counter of the caller-stream launches,
-// [1] error word shared by all launches, [2..4] work counters of the three pipeline streams: each set to 0
-// in front of the launch that uses it. The four-wide launches outside stream capture do without that
-// operation (1.6 us of a small call): every work-counter slot has kTurns counters from kScratchTurns on, a
-// launch takes the next one and sets to 0 the one whose turn comes two launches later.
+// [1] error word shared by all launches, [2..4] work counters of the three pipeline streams. A launch that
+// uses a counter sets it to 0 in its own stream first, so calls may be issued in any order on any streams as long as
+// they do not run at the same time on one slot. (That operation is 1.6 us of a call; small sets have no counter.)
 constexpr int kScratchErr = 1;
 constexpr int kScratchPipe = 2;
-constexpr int kScratchTurns = 8;
-constexpr unsigned kTurns = 4;
 
 struct TraceArgs {
     BvhView bvh;
@@ -117,7 +113,7 @@ struct TraceArgs {
     int64_t n;
     void *hits;
     unsigned long long *counter;
-    unsigned long long *clear;  // a counter to set to 0 for a later launch, or nullptr
+    unsigned share;  // four-wide: places of every warp, first warp first; 0: the warps claim from the counter
     unsigned int *err;
     // TT_VARIANT_SORTED, when order_built(order_state): the ray in each place of the order
     const int *order_src;
@@ -163,12 +159,15 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
     rays.sh = sh_rays + (kHost ? threadIdx.x : 0);
     const bool use_perm = kPerm && a.order_state && order_built(a.order_state);
     unsigned *queue = reinterpret_cast<unsigned *>(a.counter);  // the next ray
-    if (a.clear && blockIdx.x == 0 && threadIdx.x == 0) *a.clear = 0ull;
     trace_queue<kClosest, kWideInner>(
         stack, rays, a.bvh, (unsigned)a.n, err,
-        [&](int count) {
+        [&](bool first, unsigned &count) {
+            if (a.share) {
+                count = a.share;  // (trace_queue asks for no less: a share is n / warps or one more)
+                return first ? (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * a.share : (unsigned)a.n;
+            }
             unsigned b = 0;
-            if (lane == 0) b = atomicAdd(queue, (unsigned)count);
+            if (lane == 0) b = atomicAdd(queue, count);
             return __shfl_sync(0xffffffffu, b, 0);
         },
         [&](unsigned place) { return use_perm ? ordered_slot(a.order_src, place, (unsigned)a.n, err) : place; },
@@ -430,7 +429,7 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     a.n = n;
     a.hits = d_hits;
     a.counter = d.scratch + counter_slot;
-    a.clear = nullptr;
+    a.share = 0;
     a.err = reinterpret_cast<unsigned int *>(d.scratch + kScratchErr);
     a.order_src = nullptr;
     a.order_state = nullptr;
@@ -441,10 +440,26 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
         (variant == VARIANT_SORTED || variant == VARIANT_SORTED_OCC) && !host_rays && n >= kOrderMinRays;
     if (host_rays) variant = VARIANT_HOST;
     if (!d.view.wide_nodes && variant != VARIANT_DYNAMIC && variant != VARIANT_WARP_VOTE) variant = VARIANT_TWO_WIDE;
-    // per work-counter slot: the ordering scratch, so the pipeline streams never share one, and the turns
-    const int k = counter_slot == 0 ? 0 : 1 + (counter_slot - kScratchPipe) % 3;
-    DeviceBVH &dm = const_cast<DeviceBVH &>(d);
+    // Four rays a warp before a second warp is left out: a small set is bound by its longest chain of
+    // node steps, which lanes of one warp lengthen for each other (1,000 surface rays on a
+    // 524,288-triangle terrain: 33 us, with 32 a warp 37; 1,000 camera rays 33 against 45; from 20,000
+    // rays on level).
+    const int64_t max_useful = (n + 4 * (kTraceBlock / 32) - 1) / (4 * (kTraceBlock / 32));
+    const bool two_wide = variant == VARIANT_TWO_WIDE || variant == VARIANT_DYNAMIC || variant == VARIANT_WARP_VOTE;
+    int64_t blocks = (int64_t)d.num_sms * d.blocks_per_sm[variant];
+    if (!two_wide && blocks >= max_useful) {
+        // the warps' first claims would take all the rays: they are dealt out, without a counter
+        const int64_t warps = max_useful * (kTraceBlock / 32);
+        a.share = (unsigned)((n + warps - 1) / warps);
+    } else if (!order_rays) {  // (the ordering's first pass does it)
+        TT_CUDA(cudaMemsetAsync(a.counter, 0, 8, stream));
+    }
+    if (blocks > max_useful) blocks = max_useful;
+    if (blocks < 1) blocks = 1;
     if (order_rays) {
+        // one scratch per work-counter slot, so the pipeline streams never share one
+        const int k = counter_slot == 0 ? 0 : 1 + (counter_slot - kScratchPipe) % 3;
+        DeviceBVH &dm = const_cast<DeviceBVH &>(d);
         const size_t need = reorder_scratch_bytes(n);
         if (dm.order_bytes[k] < need) {
             if (dm.order[k]) cudaFree(dm.order[k]);
@@ -459,40 +474,18 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
         }
         const tt_status st =
             reorder_rays(a.rays, n, nullptr, d.lo, d.hi, dm.order[k], dm.order_state_at[k], kOrderMinRays, a.err, stream,
-                         &order);
+                         &order, false, a.counter);
         if (st != TT_OK) return st;
         a.order_src = order.src;
         a.order_state = order.state;
     }
-    // Four rays a warp before a second warp is left out: a small set is bound by its longest chain of
-    // node steps, which lanes of one warp lengthen for each other (1,000 surface rays on a
-    // 524,288-triangle terrain: 33 us, with 32 a warp 37; 1,000 camera rays 33 against 45; from 20,000
-    // rays on level).
-    const int64_t max_useful = (n + 4 * (kTraceBlock / 32) - 1) / (4 * (kTraceBlock / 32));
-    int64_t blocks = (int64_t)d.num_sms * d.blocks_per_sm[variant];
-    if (blocks > max_useful) blocks = max_useful;
-    if (blocks < 1) blocks = 1;
-    const bool two_wide = variant == VARIANT_TWO_WIDE || variant == VARIANT_DYNAMIC || variant == VARIANT_WARP_VOTE;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (!two_wide && stream && stream != cudaStreamLegacy && cudaStreamIsCapturing(stream, &capture) != cudaSuccess)
-        cudaGetLastError();  // (the legacy stream cannot be captured)
-    // a captured launch runs again without the launches around it, so its counter is set to 0 with it
-    const bool turns = !two_wide && capture == cudaStreamCaptureStatusNone;
-    if (turns) {
-        unsigned long long *c = d.scratch + kScratchTurns + kTurns * k;
-        a.counter = c + dm.turn[k] % kTurns;
-        a.clear = c + (dm.turn[k] + 2) % kTurns;
-    } else {
-        TT_CUDA(cudaMemsetAsync(d.scratch + counter_slot, 0, 8, stream));
-    }
     cudaError_t le;
-    const bool chained = order_rays && turns;
+    const bool chained = order_rays && !two_wide;  // behind the ordering's last pass
     if (closest) le = ext ? launch_variant<true, true>(d, variant, (unsigned)blocks, chained, stream, a)
                           : launch_variant<true, false>(d, variant, (unsigned)blocks, chained, stream, a);
     else le = ext ? launch_variant<false, true>(d, variant, (unsigned)blocks, chained, stream, a)
                   : launch_variant<false, false>(d, variant, (unsigned)blocks, chained, stream, a);
     TT_CUDA(le);
-    if (turns) dm.turn[k]++;
     return TT_OK;
 }
 
@@ -715,7 +708,8 @@ tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_
     if (dr_mapped && dh_mapped && !(reinterpret_cast<uintptr_t>(dr_mapped) & 15) &&
         !(reinterpret_cast<uintptr_t>(dh_mapped) & 7) && d.view.wide_nodes && d.variant != VARIANT_DYNAMIC &&
         d.variant != VARIANT_WARP_VOTE) {
-        tt_status st = launch_trace(d, dr_mapped, n, const_cast<void *>(dh_mapped), closest != 0, false, s, 0, true);
+        tt_status st =
+            launch_trace(d, dr_mapped, n, const_cast<void *>(dh_mapped), closest != 0, false, s, kScratchPipe, true);
         if (st != TT_OK) return st;
         TT_CUDA(cudaStreamSynchronize(s));
         return read_error_word(d, s);

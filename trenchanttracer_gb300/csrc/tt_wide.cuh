@@ -484,8 +484,9 @@ constexpr int kWideInner = 8;
 // stand at inner nodes they step on; then the lanes that wait at leaves test their triangles
 // together, and where none does, the lanes whose rays are finished store them and take the queue's
 // next ones (one claim; consecutive slots, so an ordered queue's neighbours start together).
-// claim(count): the first of `count` queue places, all lanes taking part (places from n on do not
-// exist); at(place): the slot in that place; fetch(slot, r0, r1): a slot's ray; store(lanes, slot,
+// claim(first, count): the first of the `count` queue places that come to the warp (it may take fewer off them,
+// by lowering count), all lanes taking part; places from n on do not exist; first: the warp's first
+// claim. at(place): the slot in that place; fetch(slot, r0, r1): a slot's ray; store(lanes, slot,
 // result): the lanes of `lanes` store together.
 //
 // Measured on 4M rays over a 2,097,152-triangle terrain against one warp-wide loop per 32 rays (each
@@ -497,8 +498,7 @@ __device__ __forceinline__ void trace_queue(Stack &stack, Rays &rays, const BvhV
     WideState s;
     s.ref = kWideIdle;
     unsigned slot = 0;
-    bool more = true;  // the queue may have rays left
-    unsigned base = 0;
+    unsigned left = n;  // rays that the queue may still have
     const unsigned warps = gridDim.x * blockDim.x / 32, few = min(n / warps, 3u);
     for (;;) {
         const unsigned inner = __ballot_sync(0xffffffffu, s.ref < kWideMark);
@@ -518,12 +518,12 @@ __device__ __forceinline__ void trace_queue(Stack &stack, Rays &rays, const BvhV
                 s.ref = kWideIdle;
             }
             __syncwarp();
-            if (more) {
+            if (left) {
                 // no more than the warp's share of what is left, but a few
                 const unsigned want = ~inner;
-                const unsigned count = min((unsigned)__popc(want), max((n - base) / warps, few) + 1u);
-                base = claim((int)count);
-                more = base < n && n - base > count;
+                unsigned count = min((unsigned)__popc(want), max(left / warps, few) + 1u);
+                const unsigned base = claim(left == n, count);
+                left = base < n && n - base > count ? n - base - count : 0;
                 if (s.ref == kWideIdle) {
                     const unsigned off = __popc(want & ((1u << (threadIdx.x & 31)) - 1u));
                     if (off < count && base < n && off < n - base) {
