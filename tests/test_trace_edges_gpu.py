@@ -75,3 +75,21 @@ def test_calls_whose_streams_run_in_another_order_than_they_were_issued(n):
     late.synchronize()
     assert np.array_equal(waiting.cpu().numpy(), ref)
     dbvh.check()
+
+
+@pytest.mark.parametrize("at", [0, 24])
+@pytest.mark.parametrize("n", [100, 300000])
+def test_host_hits_over_the_rays(n, at):
+    """Hits written where the (page-locked) rays are, from their first byte or from the fourth part on: every ray is
+    read before the first hit is written."""
+    bvh, extent = tree("spheres")
+    dbvh = DeviceBVH(bvh)
+    rays = rays_for(extent, 9, n)
+    ref = trace(dbvh, torch.from_numpy(rays).cuda())
+    buf = torch.empty(8 * n).pin_memory().numpy()
+    h_rays = buf.reshape(n, 8)
+    h_rays[:] = rays
+    first = at * n // 4 // 2 * 2
+    h_hits = buf[first:first + 2 * n].view(np.int32).reshape(n, 2)
+    dbvh.intersect_host(h_rays, h_hits)
+    assert np.array_equal(h_hits, ref)

@@ -704,8 +704,11 @@ tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_
     // too), so the transfer overlaps traversal with no staging. Staged chunks that overlap their copies
     // take longer for every set: 2M / 4M cosine bounces on a 524,288-triangle terrain 0.65 / 1.15 ms
     // against 0.50 / 0.85, 4M camera rays 0.85 against 0.72, 1,000 rays 73 us against 61.
+    // Hits that are to lie over the rays want every ray read before the first is written: staged.
+    const uintptr_t r0 = reinterpret_cast<uintptr_t>(h_rays), h0 = reinterpret_cast<uintptr_t>(h_hits);
+    const bool apart = r0 + 32ull * n <= h0 || h0 + 8ull * n <= r0;
     const void *dr_mapped = mapped_host_range(h_rays, 32ull * n), *dh_mapped = mapped_host_range(h_hits, 8ull * n);
-    if (dr_mapped && dh_mapped && !(reinterpret_cast<uintptr_t>(dr_mapped) & 15) &&
+    if (apart && dr_mapped && dh_mapped && !(reinterpret_cast<uintptr_t>(dr_mapped) & 15) &&
         !(reinterpret_cast<uintptr_t>(dh_mapped) & 7) && d.view.wide_nodes && d.variant != VARIANT_DYNAMIC &&
         d.variant != VARIANT_WARP_VOTE) {
         tt_status st =
