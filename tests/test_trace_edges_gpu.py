@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from tests.test_wide_bvh import SCENES, rays_for
-from trenchanttracer_gb300 import BVHCompact, DeviceBVH
+from trenchanttracer_gb300 import BVHCompact, DeviceBVH, TTError
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -93,3 +93,23 @@ def test_host_hits_over_the_rays(n, at):
     h_hits = buf[first:first + 2 * n].view(np.int32).reshape(n, 2)
     dbvh.intersect_host(h_rays, h_hits)
     assert np.array_equal(h_hits, ref)
+
+
+def test_upload_after_a_refused_call():
+    """A call that fails leaves its error behind in the thread; the next upload is none of its business."""
+    bvh, extent = tree("spheres")
+    dbvh = DeviceBVH(bvh)
+    n, runtime = 1000, torch.cuda.cudart()
+    room = np.empty(8 * n + 2048, np.float32)
+    h_rays = room[-room.ctypes.data % 4096 // 4:][:8 * n].reshape(n, 8)
+    h_rays[:] = rays_for(extent, 12, n)
+    h_hits = np.empty((n, 2), np.int32)
+    assert int(runtime.cudaHostRegister(h_rays.ctypes.data, 16384, 0)) == 0
+    try:
+        with pytest.raises(TTError):  # half of the rays page-locked: no valid range to copy
+            dbvh.intersect_host(h_rays, h_hits)
+        again = DeviceBVH(bvh)
+    finally:
+        runtime.cudaHostUnregister(h_rays.ctypes.data)
+    rays = torch.from_numpy(h_rays.copy()).cuda()
+    assert np.array_equal(trace(again, rays), trace(dbvh, rays))

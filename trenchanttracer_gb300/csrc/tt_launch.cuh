@@ -36,4 +36,16 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int block, si
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// A plain launch that returns its own error (cudaGetLastError would also return what an earlier call of the
+// caller's thread had left there).
+template <class... P, class... A>
+inline cudaError_t launch_plain(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace tt

@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <string>
 
+#include "tt_launch.cuh"
 #include "tt_wide.cuh"
 #include "tt_wide_build.h"
 
@@ -377,11 +378,10 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
     auto run = [&]() -> cudaError_t {
         cudaError_t c = cudaMemsetAsync(b.parent, 0xff, words, nullptr);
         if (c == cudaSuccess) c = cudaMemsetAsync(b.arrived, 0, words + met + align(sizeof(Totals)), nullptr);
-        if (c != cudaSuccess) return c;
-        k_wide_parents<<<grid, kBuildBlock>>>(b);
-        k_wide_costs<<<grid, kBuildBlock>>>(b);
-        k_wide_roots<<<grid, kBuildBlock>>>(b);
-        c = cudaMemcpy(&t, b.tot, sizeof t, cudaMemcpyDeviceToHost);
+        if (c == cudaSuccess) c = launch_plain(k_wide_parents, grid, kBuildBlock, 0, nullptr, b);
+        if (c == cudaSuccess) c = launch_plain(k_wide_costs, grid, kBuildBlock, 0, nullptr, b);
+        if (c == cudaSuccess) c = launch_plain(k_wide_roots, grid, kBuildBlock, 0, nullptr, b);
+        if (c == cudaSuccess) c = cudaMemcpy(&t, b.tot, sizeof t, cudaMemcpyDeviceToHost);
         if (c != cudaSuccess) return c;
         if (!convertible(t, b.count)) return cudaSuccess;  // stays two-wide
         // (pairs: at most one per vertex slot, with every triangle in one leaf)
@@ -393,9 +393,9 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
         c = cudaMalloc(&out.base, nb + pb);
         if (c != cudaSuccess) return c;
         char *nodes = static_cast<char *>(out.base), *pairs = nodes + nb;
-        k_wide_places<<<grid, kBuildBlock>>>(b, k);
-        k_wide_records<<<grid, kBuildBlock>>>(b, nodes, (uint32_t)wide, pairs, (uint32_t)t.pairs);
-        c = cudaGetLastError();
+        c = launch_plain(k_wide_places, grid, kBuildBlock, 0, nullptr, b, k);
+        if (c == cudaSuccess)
+            c = launch_plain(k_wide_records, grid, kBuildBlock, 0, nullptr, b, nodes, wide, pairs, t.pairs);
         if (c == cudaSuccess) c = cudaStreamSynchronize(nullptr);
         if (c != cudaSuccess) return c;
         out.nodes = nodes;
@@ -406,13 +406,13 @@ cudaError_t build_wide(const BvhView &two, uint32_t num_nodes, uint32_t num_vert
     };
     e = run();
     cudaFree(work);
-    if (e == cudaErrorMemoryAllocation) {  // no room for a second form: two-wide, as before
-        cudaGetLastError();
-        e = cudaSuccess;
-    }
     if (e != cudaSuccess && out.base) {
         cudaFree(out.base);
         out = WideBVH();
+    }
+    if (e == cudaErrorMemoryAllocation) {  // no room for a second form: two-wide, as before
+        cudaGetLastError();
+        e = cudaSuccess;
     }
     return e;
 }
