@@ -113,3 +113,34 @@ def test_upload_after_a_refused_call():
         runtime.cudaHostUnregister(h_rays.ctypes.data)
     rays = torch.from_numpy(h_rays.copy()).cuda()
     assert np.array_equal(trace(again, rays), trace(dbvh, rays))
+
+
+def test_host_rays_in_two_registrations():
+    """Rays that span two page-locked registrations next to each other are traced; with one of the two gone, the call
+    is refused (a copy of such a range is no valid one) and writes no hits."""
+    bvh, extent = tree("spheres")
+    dbvh = DeviceBVH(bvh)
+    n = 100000
+    room = np.empty(8 * n + 2048, np.float32)
+    h_rays = room[-room.ctypes.data % 4096 // 4:][:8 * n].reshape(n, 8)
+    h_rays[:] = rays_for(extent, 12, n)
+    h_hits = torch.empty(n, 2, dtype=torch.int32).pin_memory().numpy()
+    ref = trace(dbvh, torch.from_numpy(h_rays.copy()).cuda())
+    first, half, runtime = h_rays.ctypes.data, 16 * n // 4096 * 4096, torch.cuda.cudart()
+    assert int(runtime.cudaHostRegister(first, half, 0)) == 0
+    try:
+        assert int(runtime.cudaHostRegister(first + half, 32 * n - half, 0)) == 0
+        h_hits[:] = -7
+        try:
+            dbvh.intersect_host(h_rays, h_hits)
+        finally:
+            runtime.cudaHostUnregister(first + half)
+        assert np.array_equal(h_hits, ref)
+        h_hits[:] = -7
+        with pytest.raises(TTError):
+            dbvh.intersect_host(h_rays, h_hits)
+        assert (h_hits == -7).all()
+    finally:
+        runtime.cudaHostUnregister(first)
+    dbvh.intersect_host(h_rays, h_hits)
+    assert np.array_equal(h_hits, ref)

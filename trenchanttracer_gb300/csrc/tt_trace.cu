@@ -662,9 +662,9 @@ tt_status tt_trace_ext(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_h
 }
 
 // The device address of a range of page-locked host memory mapped into the device's address space, or
-// nullptr: pageable memory, device memory, a range that is not all of one page-locked allocation
-// (its ends alone do not tell: two registered ranges may have pageable memory between them), or
-// an error, which is cleared.
+// nullptr: pageable memory, device memory, a range with a part that is not page-locked or not mapped (its
+// ends alone do not tell: two registered ranges may have pageable memory between them), or an
+// error, which is cleared. The range may span registrations that adjoin.
 static const void *mapped_host_range(const void *p, size_t bytes) {
     using GetAttribute = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
     static const GetAttribute get = [] {
@@ -678,19 +678,25 @@ static const void *mapped_host_range(const void *p, size_t bytes) {
         }
         return reinterpret_cast<GetAttribute>(fn);
     }();
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
+    const char *mapped = nullptr;
+    for (size_t done = 0; done < bytes;) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, static_cast<const char *>(p) + done) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (at.type != cudaMemoryTypeHost || !at.devicePointer || !get) return nullptr;
+        if (done == 0) mapped = static_cast<const char *>(at.devicePointer);
+        if (at.devicePointer != mapped + done) return nullptr;
+        const CUdeviceptr here = reinterpret_cast<CUdeviceptr>(at.devicePointer);
+        CUdeviceptr start = 0;
+        size_t size = 0;
+        if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, here) != CUDA_SUCCESS ||
+            get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, here) != CUDA_SUCCESS || here < start || here - start >= size)
+            return nullptr;
+        done += size - (here - start);
     }
-    if (at.type != cudaMemoryTypeHost || !at.devicePointer || !get) return nullptr;
-    const CUdeviceptr first = reinterpret_cast<CUdeviceptr>(at.devicePointer);
-    CUdeviceptr start = 0;
-    size_t size = 0;
-    if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, first) != CUDA_SUCCESS ||
-        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, first) != CUDA_SUCCESS)
-        return nullptr;
-    return first >= start && first - start <= size && bytes <= size - (first - start) ? at.devicePointer : nullptr;
+    return mapped;
 }
 
 tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_hit *h_hits, int32_t closest,
