@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from tests.test_wide_bvh import SCENES, rays_for
-from trenchanttracer_gb300 import BVHCompact, DeviceBVH, TTError
+from trenchanttracer_gb300 import BVHCompact, DeviceBVH, TTError, scenes
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -144,3 +144,26 @@ def test_host_rays_in_two_registrations():
         runtime.cudaHostUnregister(first)
     dbvh.intersect_host(h_rays, h_hits)
     assert np.array_equal(h_hits, ref)
+
+
+@pytest.mark.parametrize("share", [0.0, 0.01, 0.05, 0.5, 1.0])
+@pytest.mark.parametrize("closest", [True, False])
+def test_coherent_sets_with_rays_that_the_four_wide_loop_does_not_serve(share, closest):
+    """Camera rays of which some start at a negative tmin: the probe sends a set with too many of them to the two-wide
+    loop as a whole, and its decision must not outlast the call."""
+    sc, alpha, leaf, _ = SCENES["spheres"]()
+    dbvh = DeviceBVH(BVHCompact.build(sc, alpha, 1, leaf))
+    side = 1100
+    rays = torch.from_numpy(scenes.pinhole_rays(side, side, [0.0, 14.0, 34.0], [0.0, 2.0, 0.0], 0.45)).cuda()
+    g = torch.Generator("cuda").manual_seed(3)
+    rays[torch.rand(side * side, generator=g, device="cuda") < share, 6] = -1e-3
+    dbvh.set_variant(DeviceBVH.VARIANT_DYNAMIC)
+    ref = trace(dbvh, rays, closest)
+    plain = rays.clone()
+    plain[:, 6] = 1e-3
+    ref_plain = trace(dbvh, plain, closest)
+    for variant in (DeviceBVH.VARIANT_SORTED, DeviceBVH.VARIANT_SORTED_OCC):
+        dbvh.set_variant(variant)
+        assert np.array_equal(trace(dbvh, rays, closest), ref)
+        assert np.array_equal(trace(dbvh, plain, closest), ref_plain)
+        assert np.array_equal(trace(dbvh, rays[:40001].contiguous(), closest), ref[:40001])

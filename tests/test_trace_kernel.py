@@ -51,14 +51,14 @@ def kernels(tmp_path_factory):
     return lib, passes
 
 
-def trace(lib, tree, kernel, rays, closest, order=None, wide=True, blocks=2, spare=0, share=0):
+def trace(lib, tree, kernel, rays, closest, order=None, wide=True, blocks=2, spare=0, share=0, decision=0):
     """Hits of the first len(rays) - spare rays; the spare ones and their hits lie behind the buffers' ends."""
     n = rays.shape[0] - spare
     hits = np.full((rays.shape[0], 2), -7, np.int32)
     nodes, pairs = tree.wide if wide else (None, None)
     err = lib.trace_kernel_host(kernel, blocks, ptr(tree.nodes), ptr(tree.verts), ptr(tree.tri), ptr(nodes), ptr(pairs),
                                 tree.flags if wide else 0, ptr(rays), C.c_longlong(n), int(closest), ptr(order),
-                                C.c_uint(share), ptr(hits))
+                                C.c_uint(share), decision or int(order is not None), ptr(hits))
     return hits, err
 
 
@@ -78,6 +78,19 @@ def test_queue_kernels_give_the_two_wide_hits(kernels, name, closest):
     for n in (1, 2, 31, 32, 33, 63, 65):
         got, err = trace(lib, tree, ORDERED, rays[:n], closest)
         assert err == 0 and np.array_equal(got, ref[:n]), n
+
+
+@pytest.mark.parametrize("name", ["spheres", "zero_planes", "needles"])
+def test_the_probe_may_send_a_set_to_the_two_wide_loop(kernels, name):
+    """The default kernel over a set of which the probe found too many rays that the four-wide loop does not serve."""
+    lib, passes = kernels
+    tree = Tree(passes, name)
+    for n in (1, 33, 1000):
+        rays = rays_for(tree.extent, 37, n)
+        for closest in (1, 0):
+            ref, _ = trace(lib, tree, DYNAMIC, rays, closest)
+            got, err = trace(lib, tree, ORDERED, rays, closest, decision=2)
+            assert err == 0 and np.array_equal(got, ref), (n, closest)
 
 
 @pytest.mark.parametrize("n,warps", [(1, 4), (3, 4), (4, 4), (5, 4), (13, 4), (16, 4), (253, 64), (256, 64)])

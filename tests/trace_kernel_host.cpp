@@ -22,13 +22,14 @@ extern "C" {
 // Traces n rays by a kernel (0: the default, 1: without shared stack, 2: over host rays, 3: two-wide in the
 // default's place, 4: two-wide with per-lane claims) in a grid of `blocks` warps, over a two-wide tree and,
 // unless wide_nodes is null, its four-wide form. order: the ray in each place, or null. share: the places dealt
-// to each warp (0: claimed from a counter). Returns the error word.
+// to each warp (0: claimed from a counter). decision: of the ordering's probe (1 with an order, 2: two-wide).
+// Returns the error word.
 __attribute__((visibility("default"))) unsigned trace_kernel_host(
     int kernel, unsigned blocks, const float *nodes, const float *verts, const int *tri_idx, const char *wide_nodes,
     const char *wide_pairs, unsigned wide_flags, const float *rays, long long n, int closest, const int *order, unsigned share,
-    int *hits) {
+    int decision, int *hits) {
     unsigned err = 0;
-    unsigned long long counter = 0, state[4] = {0, 0, 0, 1};
+    unsigned long long counter = 0, state[5] = {0, 0, 0, (unsigned long long)decision, 0};
     TraceArgs a{};
     a.bvh.nodes = reinterpret_cast<const float4 *>(nodes);
     a.bvh.verts = reinterpret_cast<const float4 *>(verts);
@@ -43,7 +44,7 @@ __attribute__((visibility("default"))) unsigned trace_kernel_host(
     a.share = share;
     a.err = &err;
     a.order_src = order;
-    a.order_state = order ? state : nullptr;
+    a.order_state = decision ? state : nullptr;
     if (closest) trace<true>(kernel, blocks, a);
     else trace<false>(kernel, blocks, a);
     return err;

@@ -29,6 +29,7 @@
 #include "tt_internal.h"
 #include "tt_launch.cuh"
 #include "tt_reorder.h"
+#include "tt_wide.cuh"
 
 namespace tt {
 
@@ -40,8 +41,9 @@ static_assert(kScanChunk == 8 * kOrderBlock && kNumChunks == 4 * kOrderBlock, "s
 static_assert(((1 << (kOrderDirBits + kOrderMinOriginBits)) / kScanChunk) % 4 == 0, "whole uint4 of chunk totals");
 
 // State block (64-bit words): [0] sampled uniform warps, [1] sampled full warps, [2] probe blocks
-// done, [3] the decision (1: ordered). The probe's last block to finish writes the decision and
-// clears [0..2] for the next call, so calls need no other bookkeeping (and replay in a graph).
+// done, [3] the decision (1: ordered, 2: two-wide in their own order), [4] rays of the full warps that the
+// four-wide loop does not serve. The probe's last block to finish writes the decision and clears
+// [0..2] and [4] for the next call, so calls need no other bookkeeping (and replay in a graph).
 struct OrderArgs {
     const float4 *rays;
     int64_t n;         // rays, or the capacity when n_dev is set
@@ -57,6 +59,7 @@ struct OrderArgs {
     unsigned long long *state;
     unsigned *err;
     unsigned long long *clear;  // a word to set to 0, or nullptr
+    int64_t wide_flags;         // of the tree, or -1: its form does not matter
 };
 
 __device__ __forceinline__ int64_t order_rays(const OrderArgs &a) {
@@ -97,7 +100,7 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned x, unsigned *s
 // (1) clear the counts; probe; the last block decides
 __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
     chain_begin();
-    __shared__ unsigned s_probe[2];
+    __shared__ unsigned s_probe[3];
     const int lane = threadIdx.x & 31;
     const int64_t tid = (int64_t)blockIdx.x * kOrderBlock + threadIdx.x;
     const int64_t nthreads = (int64_t)gridDim.x * kOrderBlock;
@@ -109,10 +112,10 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
     }
     for (int64_t j = tid; j < (1 << a.key_bits) / 4; j += nthreads)
         reinterpret_cast<uint4 *>(a.counts)[j] = make_uint4(0u, 0u, 0u, 0u);
-    if (threadIdx.x < 2) s_probe[threadIdx.x] = 0u;
+    if (threadIdx.x < 3) s_probe[threadIdx.x] = 0u;
     __syncthreads();
     const int64_t warps = (n + 31) / 32;
-    unsigned uniform = 0, full = 0;
+    unsigned uniform = 0, full = 0, unserved = 0;
     for (int64_t j = tid >> 5; j * kProbeStride < warps; j += nthreads >> 5) {
         // one warp of every kProbeStride, each time another one: a fixed one meets the same columns in every
         // row of an image (1,024 wide: two, the centre's among them, where directions change their
@@ -120,25 +123,31 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
         const int64_t w = j * kProbeStride + (((unsigned)j * 0x9e3779b1u) >> 28) % kProbeStride;
         if (w * 32 + 32 > n) continue;  // only full warps count; w is the same in every lane
         const int64_t i = w * 32 + lane;
-        const unsigned key = order_key(a.rays[2 * i], a.rays[2 * i + 1], a.g);
+        const float4 r0 = a.rays[2 * i], r1 = a.rays[2 * i + 1];
+        const unsigned key = order_key(r0, r1, a.g);
         full++;
         if (__match_any_sync(0xffffffffu, key) == 0xffffffffu) uniform++;
+        if (a.wide_flags >= 0) unserved += !wide_serves(r0, r1, (uint32_t)a.wide_flags);
     }
     if (lane == 0 && full) {
         atomicAdd(&s_probe[0], uniform);
         atomicAdd(&s_probe[1], full);
     }
+    if (unserved) atomicAdd(&s_probe[2], unserved);
     __syncthreads();
     if (threadIdx.x == 0) {
         if (s_probe[1]) {
             atomicAdd(a.state + 0, (unsigned long long)s_probe[0]);
             atomicAdd(a.state + 1, (unsigned long long)s_probe[1]);
+            if (s_probe[2]) atomicAdd(a.state + 4, (unsigned long long)s_probe[2]);
         }
         __threadfence();
         if (atomicAdd(a.state + 2, 1ull) == (unsigned long long)gridDim.x - 1) {  // every block's counts are in
             const unsigned long long u = atomicAdd(a.state + 0, 0ull), f = atomicAdd(a.state + 1, 0ull);
+            const unsigned long long w = atomicAdd(a.state + 4, 0ull);
             // ordered unless mostly uniform
-            a.state[3] = (f > 0 && 2 * u <= f) ? 1ull : 0ull;
+            a.state[3] = (f > 0 && 2 * u <= f) ? 1ull : (64 * w > 32 * f ? 2ull : 0ull);
+            a.state[4] = 0ull;
             a.state[0] = 0ull;
             a.state[1] = 0ull;
             a.state[2] = 0ull;
@@ -287,7 +296,7 @@ static std::atomic<int> g_order_sms[64];  // SMs per device (0 = not yet known)
 
 tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const float lo[3], const float hi[3],
                        void *scratch, size_t state_at, int64_t min_rays, unsigned *err, cudaStream_t s, OrderOut *out,
-                       bool with_pos, unsigned long long *clear) {
+                       bool with_pos, unsigned long long *clear, int64_t wide_flags) {
     if (n <= 0 || n >= ((int64_t)1 << 31)) return fail(TT_ERR_INVALID, "ray ordering: n must be in 1..2^31-1");
     if (state_at < reorder_state_offset(n) || (state_at & 255))
         return fail(TT_ERR_INVALID, "ray ordering: scratch too small for this many rays");
@@ -324,6 +333,7 @@ tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const fl
     a.state = reinterpret_cast<unsigned long long *>(static_cast<char *>(scratch) + state_at);
     a.err = err;
     a.clear = clear;
+    a.wide_flags = wide_flags;
     const int64_t want = (n + kOrderBlock - 1) / kOrderBlock;
     const unsigned grid = (unsigned)(want < (int64_t)sms * 8 ? want : (int64_t)sms * 8);
     e = launch_chained(k_order_probe, (unsigned)sms * 4, kOrderBlock, 0, s, a);

@@ -102,19 +102,27 @@ struct OrderOut {
 // Calls on one scratch must be ordered (one stream). Launches only, no allocation, so a call can
 // be captured in a CUDA graph. Fewer than min_rays rays keep their own order. Device-side errors go
 // to *err as kErrOrder. with_pos: also the inverse permutation. clear: a word that the first pass sets to 0 (the work
-// counter of the kernel that follows).
+// counter of the kernel that follows). wide_flags >= 0, a tree's BvhView::wide_flags: coherent rays are also looked
+// at for those that its four-wide form does not serve (order_two_wide).
 //
 // The rays themselves stay where they are and a trace kernel reads them through src. A copy in
 // sorted order, undone for the hits by a last pass, cost more than the scattered sectors do in a trace
 // that takes 3 % of the memory bandwidth: 4M terrain bounces 840 us with the copy, 790 without.
 tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const float lo[3], const float hi[3],
                        void *scratch, size_t state_at, int64_t min_rays, unsigned *err, cudaStream_t s, OrderOut *out,
-                       bool with_pos = false, unsigned long long *clear = nullptr);
+                       bool with_pos = false, unsigned long long *clear = nullptr, int64_t wide_flags = -1);
 
 // Whether this call's rays were ordered: false when more than half of the sampled warps held 32
 // equal keys (the rays are coherent already: camera rays share one origin cell and neighbouring
 // pixels one direction cell) or too few rays came; they are then traced in their own order.
 __device__ __forceinline__ bool order_built(const unsigned long long *state) { return state[3] == 1ull; }
+
+// Whether this call's rays are coherent and hold so many that the four-wide loop does not serve that the two-wide
+// one takes less for all: more than a 64th of the sampled ones. Each such ray holds up its warp while one lane
+// runs the two-wide loop. 4M camera rays on the 2,097,152-triangle terrain, two-wide 658 us: with none
+// such 489, a thousandth 503, a twentieth 815, half 1,203. Incoherent sets are faster four-wide whatever the share
+// (4M bounces, two-wide 1,165 us: 891 with a twentieth, 898 with half).
+__device__ __forceinline__ bool order_two_wide(const unsigned long long *state) { return state[3] == 2ull; }
 
 // The ray in a place of the order of rays 0 .. n - 1, for the kernels that take their rays through it. An order
 // that is no permutation (two calls that overlap on one scratch make one, and places that the scatter left out

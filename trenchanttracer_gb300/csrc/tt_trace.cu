@@ -159,23 +159,28 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) trace_wide_kernel(Tra
     rays.sh = sh_rays + (kHost ? threadIdx.x : 0);
     const bool use_perm = kPerm && a.order_state && order_built(a.order_state);
     unsigned *queue = reinterpret_cast<unsigned *>(a.counter);  // the next ray
-    trace_queue<kClosest, kWideInner>(
-        stack, rays, a.bvh, (unsigned)a.n, err,
-        [&](bool first, unsigned &count) {
-            if (a.share) {
-                count = a.share;  // (trace_queue asks for no less: a share is n / warps or one more)
-                return first ? (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * a.share : (unsigned)a.n;
-            }
-            unsigned b = 0;
-            if (lane == 0) b = atomicAdd(queue, count);
-            return __shfl_sync(0xffffffffu, b, 0);
-        },
-        [&](unsigned place) { return use_perm ? ordered_slot(a.order_src, place, (unsigned)a.n, err) : place; },
-        [&](unsigned i, float4 &r0, float4 &r1) {
-            r0 = __ldg(a.rays + 2 * (size_t)i);
-            r1 = __ldg(a.rays + 2 * (size_t)i + 1);
-        },
-        [&](unsigned, unsigned i, const TraceResult &tr) { store_hit<kExt>(a, a.hits, i, tr); });
+    const auto claim = [&](bool first, unsigned &count) {
+        if (a.share) {
+            count = a.share;  // (trace_queue asks for no less: a share is n / warps or one more)
+            return first ? (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * a.share : (unsigned)a.n;
+        }
+        unsigned b = 0;
+        if (lane == 0) b = atomicAdd(queue, count);
+        return __shfl_sync(0xffffffffu, b, 0);
+    };
+    const auto at = [&](unsigned place) {
+        return use_perm ? ordered_slot(a.order_src, place, (unsigned)a.n, err) : place;
+    };
+    const auto fetch = [&](unsigned i, float4 &r0, float4 &r1) {
+        r0 = __ldg(a.rays + 2 * (size_t)i);
+        r1 = __ldg(a.rays + 2 * (size_t)i + 1);
+    };
+    const auto store = [&](unsigned, unsigned i, const TraceResult &tr) { store_hit<kExt>(a, a.hits, i, tr); };
+    if (kPerm && a.order_state && order_two_wide(a.order_state))
+        two_wide_queue<kClosest, kSh * (kClosest ? 2 : 1), kTraceBlock>(
+            reinterpret_cast<int *>(sh_stack) + threadIdx.x, a.bvh, (unsigned)a.n, err, claim, at, fetch, store);
+    else
+        trace_queue<kClosest, kWideInner>(stack, rays, a.bvh, (unsigned)a.n, err, claim, at, fetch, store);
     if (err) atomicOr(a.err, err);
 }
 
@@ -474,7 +479,7 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
         }
         const tt_status st =
             reorder_rays(a.rays, n, nullptr, d.lo, d.hi, dm.order[k], dm.order_state_at[k], kOrderMinRays, a.err, stream,
-                         &order, false, a.counter);
+                         &order, false, a.counter, two_wide ? -1 : (int64_t)d.view.wide_flags);
         if (st != TT_OK) return st;
         a.order_src = order.src;
         a.order_state = order.state;
