@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 from tests.test_wide_bvh import SCENES, rays_for
-from trenchanttracer_gb300 import BVHCompact, DeviceBVH, TTError, scenes
+from trenchanttracer_gb300 import (BVHCompact, DeviceBVH, Renderer, Scene, TTError, make_camera_meta, render_meta,
+                                   render_params, scenes)
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -167,3 +168,33 @@ def test_coherent_sets_with_rays_that_the_four_wide_loop_does_not_serve(share, c
         assert np.array_equal(trace(dbvh, rays, closest), ref)
         assert np.array_equal(trace(dbvh, plain, closest), ref_plain)
         assert np.array_equal(trace(dbvh, rays[:40001].contiguous(), closest), ref[:40001])
+
+
+def without_a_four_wide_form(bvh, path):
+    """The same tree with one box plane of its last node far away: its two-wide hits are the same (the box only grows),
+    and it has no four-wide form."""
+    def grow(nodes):
+        nodes.view(F)[-4, 1] = 1e15
+        return nodes
+    return edited(bvh, path, grow)
+
+
+@pytest.mark.parametrize("streamed", [0, 1])
+@pytest.mark.parametrize("shape", [(64, 0), (128, 8), (256, 16)])
+def test_renders_on_a_tree_without_a_four_wide_form(tmp_path, shape, streamed):
+    """Extension and shadow queues of a tree that stays two-wide, at every stack depth: the image of the four-wide
+    tree."""
+    sc = Scene.from_mesh(scenes.multi_material(6, 3))
+    sc.set_env(scenes.sky_env(64, 32, sun_radiance=5e2, sun_diameter_deg=10.0))
+    sc.set_geometries([{"type": "Sphere", "position": [0.0, 3.0, 9.0], "radius": 2.0, "material": 0}])
+    bvh = BVHCompact.build(sc, 1e-5, 1, 8)
+    images = []
+    for b in (bvh, without_a_four_wide_form(bvh, tmp_path / "bvh.cache")):
+        r = Renderer(DeviceBVH(b), sc)
+        r.set_launch(*shape, 3001, 1, streamed)
+        acc = torch.zeros(3 * 97 * 61, device="cuda")
+        cam = make_camera_meta(97, 61, [0.0, 14.0, 34.0], [0.0, -12.0, -34.0], fov=(60.0, 40.0))
+        r.render_native(cam, render_params(spp=3, max_depth=6, rr_depth=3, seed=3), acc)
+        r.check()
+        images.append(acc.cpu().numpy())
+    assert images[0].any() and np.array_equal(*(i.view(np.uint32) for i in images))
