@@ -198,3 +198,19 @@ def test_renders_on_a_tree_without_a_four_wide_form(tmp_path, shape, streamed):
         r.check()
         images.append(acc.cpu().numpy())
     assert images[0].any() and np.array_equal(*(i.view(np.uint32) for i in images))
+
+
+@pytest.mark.parametrize("w,h,samples", [(16, 16, 1), (200, 133, 3)])
+def test_compat_frames_on_a_tree_without_a_four_wide_form(tmp_path, w, h, samples):
+    sc = Scene.from_mesh(scenes.cornell(3))
+    sc.set_env(np.ones((8, 16, 3), F))
+    bvh = BVHCompact.build(sc, 1e-5, 1, 8)
+    images = []
+    for b in (bvh, without_a_four_wide_form(bvh, tmp_path / "bvh.cache")):
+        r = Renderer(DeviceBVH(b), sc)
+        acc = torch.zeros(3 * w * h, device="cuda")
+        cam = make_camera_meta(w, h, [0.0, 0.0, 1.55], [0.0, 0.0, -1.0], fov=(45.0, 45.0))
+        r.render_compat(cam, render_meta(7, samples), acc)
+        r.check()
+        images.append(acc.cpu().numpy())
+    assert images[0].any() and np.array_equal(*(i.view(np.uint32) for i in images))

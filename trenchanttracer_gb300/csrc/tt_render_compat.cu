@@ -402,7 +402,39 @@ __device__ __forceinline__ RRay camera_ray(const CompatArgs &a, int pixel_x, int
     return ray;
 }
 
+__device__ __forceinline__ void add_pixel(const CompatArgs &a, int x, int y, const V3 &c) {
+    const int i = (int)((unsigned)(a.cam.height - y - 1) * (unsigned)a.cam.width + (unsigned)x);
+    float *px = a.accum + 3ll * i;
+    px[0] = __fadd_rn(px[0], c.x);
+    px[1] = __fadd_rn(px[1], c.y);
+    px[2] = __fadd_rn(px[2], c.z);
+}
+
 constexpr int kCompatBounces = 10;  // the reference's bounce loop (src/core/RenderKernel.cu:33)
+// pathTracingKernel (src/core/RenderKernel.cu:97-206) on a tree without a four-wide form: one thread per pixel
+// in 16 x 16 blocks, as in the reference. (The Cornell box at 512 x 512 x 4 on its two-wide tree: 3.59 ms, compiled
+// for three blocks per SM 4.10; the kernel below, which keeps fewer threads and gains nothing from its steps then, 4.41.)
+__global__ void __launch_bounds__(256, 4) render_compat_two_wide_kernel(CompatArgs a) {
+    const int x = (int)(blockIdx.x * 16 + threadIdx.x), y = (int)(blockIdx.y * 16 + threadIdx.y);
+    const unsigned id = (blockIdx.x + blockIdx.y * gridDim.x) * 256u + threadIdx.y * 16u + threadIdx.x;
+    uint32_t err = 0;
+    curandState rs;
+    curand_init((unsigned long long)(a.meta.hashed_frame + id), 0, 0, &rs);
+    V3 final_color(0.0f, 0.0f, 0.0f);
+    for (int s = 0; s < a.meta.samples; s++) {
+        RRay ray = camera_ray(a, x, a.cam.height - y - 1, &rs);
+        V3 mask(1.0f, 1.0f, 1.0f), acc(0.0f, 0.0f, 0.0f);
+        for (int depth = 0; depth < kCompatBounces; depth++) {
+            const TraceResult tr = traverse<true>(a.bvh, make_float4(ray.o.x, ray.o.y, ray.o.z, ray.d.x),
+                                                  make_float4(ray.d.y, ray.d.z, ray.tmin, ray.tmax), err);
+            if (bounce(a, &rs, ray, tr, mask, acc)) break;
+        }
+        final_color = r_madd(acc, __fdiv_rn(1.0f, (float)a.meta.samples), final_color);
+    }
+    add_pixel(a, x, y, final_color);
+    if (err) atomicOr(a.err, err);
+}
+
 constexpr int kCompatBlock = 128;
 constexpr unsigned kCompatChunk = 4;
 constexpr int kCompatBlocks = 5;  // resident blocks per SM it is compiled for (4: +5 %, 6: +2 %, 8: +7 %)
@@ -454,13 +486,7 @@ __global__ void __launch_bounds__(kCompatBlock, kCompatBlocks) render_compat_ker
                 if (bounce(a, &rs, ray, wide_result(s), mask, acc) || depth == kCompatBounces) {
                     final_color = r_madd(acc, __fdiv_rn(1.0f, (float)a.meta.samples), final_color);
                     fresh = true;
-                    if (--left == 0) {
-                        const int i = (int)((unsigned)(a.cam.height - y - 1) * (unsigned)a.cam.width + (unsigned)x);
-                        float *px = a.accum + 3ll * i;
-                        px[0] = __fadd_rn(px[0], final_color.x);
-                        px[1] = __fadd_rn(px[1], final_color.y);
-                        px[2] = __fadd_rn(px[2], final_color.z);
-                    }
+                    if (--left == 0) add_pixel(a, x, y, final_color);
                 }
             }
             __syncwarp();
@@ -667,6 +693,11 @@ tt_status tt_render_compat(tt_renderer *r, const tt_camera_meta *cam, const tt_r
     a.meta = *meta;
     a.accum = d_accum;
     a.err = r->err;
+    if (!r->bvh.wide_nodes) {
+        render_compat_two_wide_kernel<<<dim3(cam->width / 16, cam->height / 16), dim3(16, 16), 0, (cudaStream_t)stream>>>(a);
+        TT_CUDA_R(cudaGetLastError());
+        return TT_OK;
+    }
     const long long pixels = (long long)(cam->width / 16) * (cam->height / 16) * 256;
     const long long blocks = std::min<long long>((pixels + kCompatBlock - 1) / kCompatBlock,
                                                  (long long)r->num_sms * kCompatBlocks);
