@@ -448,9 +448,10 @@ static tt_status launch_trace(const DeviceBVH &d, const void *d_rays, int64_t n,
     // Four rays a warp before a second warp is left out: a small set is bound by its longest chain of
     // node steps, which lanes of one warp lengthen for each other (1,000 surface rays on a
     // 524,288-triangle terrain: 33 us, with 32 a warp 37; 1,000 camera rays 33 against 45; from 20,000
-    // rays on level).
-    const int64_t max_useful = (n + 4 * (kTraceBlock / 32) - 1) / (4 * (kTraceBlock / 32));
+    // rays on level). The two-wide kernels' warps take 32 at a time.
     const bool two_wide = variant == VARIANT_TWO_WIDE || variant == VARIANT_DYNAMIC || variant == VARIANT_WARP_VOTE;
+    const int64_t per_block = (two_wide ? 32 : 4) * (kTraceBlock / 32);
+    const int64_t max_useful = (n + per_block - 1) / per_block;
     int64_t blocks = (int64_t)d.num_sms * d.blocks_per_sm[variant];
     if (!two_wide && blocks >= max_useful) {
         // the warps' first claims would take all the rays: they are dealt out, without a counter
