@@ -23,7 +23,8 @@ class Tree:
         size, flags = (C.c_longlong * 2)(), C.c_uint(0)
         raw = (C.c_void_p * 2)()
         wide = passes.wide_passes_form(ptr(self.nodes), C.c_longlong(len(self.nodes)), ptr(self.verts),
-                                       C.c_longlong(len(self.verts)), C.c_longlong(50), raw, size, C.byref(flags))
+                                       C.c_longlong(len(self.verts)), C.c_longlong(50), raw, size, C.byref(flags),
+                                       C.byref(C.c_uint(0)))
         assert wide > 0
         # 32-byte aligned copies, as the kernels' loads want them
         self.wide = [aligned(np.frombuffer(C.string_at(raw[k], size[k]), np.uint8)) for k in (0, 1)]

@@ -122,3 +122,23 @@ def test_a_leaf_of_very_many_triangles_stays_two_wide(host, triangles, accepted)
     assert (wide > 0 and stage == 0) if accepted else (wide == 0 and stage == 3)
     *_, a, b, c = convert(host, base, rays, 1, 1)
     assert np.array_equal(got[0], a) and np.array_equal(got[1], b) and got[2] == c
+
+
+def test_the_walk_up_a_chain_of_nodes_is_bounded(host):
+    """A file may hold one long chain of nodes, which one thread walks up. A tree that deep needs more stack than the
+    four-wide loop has, so the walk ends where that is certain."""
+    base = BVHCompact.build(soup(2, 4, 1.0, 3.0), 1e-5, 1, 1).arrays()
+    n = 5000
+    nodes = np.tile(base["nodes"][:4], (n, 1))
+    lo, hi = F(-9.0), F(9.0)
+    nodes.view(F)[0::4] = nodes.view(F)[1::4] = nodes.view(F)[2::4] = [lo, hi, lo, hi]
+    leaf = int(base["nodes"][3, 0])
+    nodes[3::4, 0] = leaf
+    nodes[3::4, 1] = 4 * np.arange(1, n + 1)
+    nodes[-1, 1] = int(base["nodes"][3, 1])
+    verts = np.ascontiguousarray(base["vertices"])
+    out, size, flags, done = (C.c_void_p * 2)(), (C.c_longlong * 2)(), C.c_uint(0), C.c_uint(0)
+    host.wide_passes_form.restype = C.c_longlong
+    wide = host.wide_passes_form(C.c_void_p(nodes.ctypes.data), C.c_longlong(len(nodes)), C.c_void_p(verts.ctypes.data),
+                                 C.c_longlong(len(verts)), C.c_longlong(50), out, size, C.byref(flags), C.byref(done))
+    assert wide == 0 and done.value <= 150

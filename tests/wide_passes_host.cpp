@@ -86,6 +86,7 @@ struct Form {
     uint32_t flags = 0;
     long long wide = 0;  // nodes; 0: refused after pass `stage`; -1: see below
     int stage = 0;
+    uint32_t done = 0;  // nodes whose cost the second pass knows
 };
 
 static Form convert(const float *nodes, long long num_nodes, const float *verts, long long num_verts,
@@ -117,6 +118,7 @@ static Form convert(const float *nodes, long long num_nodes, const float *verts,
     if (t.bad) return f;
     run(blocks, [&] { k_wide_costs(b); });
     f.stage = 2;
+    f.done = t.done;
     if (!convertible(t, b.count)) return f;
     for (uint32_t k = 1; k < b.count; k++)  // the third pass follows every node's links up to the root
         if (parent[k] / 2 >= b.count) {
@@ -162,9 +164,10 @@ long long wide_passes_trace(const float *nodes, long long num_nodes, const float
     return f.wide;
 }
 
-// The four-wide form alone; out[0] nodes, out[1] pairs (kept until the next call), sizes in bytes, flags.
+// The four-wide form alone; out[0] nodes, out[1] pairs (kept until the next call), sizes in bytes, flags; done: the
+// nodes whose cost the second pass found.
 long long wide_passes_form(const float *nodes, long long num_nodes, const float *verts, long long num_verts,
-                           long long top_nodes, const char **out, long long *bytes, unsigned *flags) {
+                           long long top_nodes, const char **out, long long *bytes, unsigned *flags, unsigned *done) {
     static Form f;
     f = convert(nodes, num_nodes, verts, num_verts, top_nodes);
     out[0] = f.nodes.data();
@@ -172,6 +175,7 @@ long long wide_passes_form(const float *nodes, long long num_nodes, const float 
     bytes[0] = (long long)f.nodes.size();
     bytes[1] = (long long)f.pairs.size();
     *flags = f.flags;
+    *done = f.done;
     return f.wide;
 }
 }

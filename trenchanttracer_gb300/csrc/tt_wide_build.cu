@@ -121,7 +121,13 @@ __global__ void __launch_bounds__(kBuildBlock) k_wide_costs(Build b) {
         int32_t ch[2];
         load_node(b.nodes + 4 * (size_t)n, box, ch);
         if (ch[0] >= 0 || ch[1] >= 0) continue;
-        for (;;) {  // every node is reached once: each pass goes one level up a finite tree
+        // Every node is reached once: each pass goes one level up a finite tree. A node of 2 h levels needs h stack
+        // entries at least (a wide node holds two levels and keeps one or more of its slots for later).
+        for (int level = 0;; level++) {
+            if (level > 2 * kWideStack) {
+                b.tot->bad = 1;
+                break;
+            }
             float total = area(box[0], box[1]);
             uint8_t taken = 0;
             uint32_t slots = 2, below = 0;
