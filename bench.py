@@ -473,7 +473,10 @@ def run_ours(args) -> None:
                                          "source": "ncu smsp__thread_inst_executed_per_inst_executed, incoherent "
                                                    "trace launch (profiles/trace_kernel_terrain_closest.md)"},
                      "bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                     "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": TRACE_DRAM_BYTES_PER_LAUNCH,
+                     "frac": round(achieved / peaks["hbm_gbs"], 4),
+                     "frac_note": "algorithmic bytes of the two-wide algorithm over the HBM rate; most are served from "
+                                  "L1 and L2, so no share of a bound (see binding)",
+                     "traffic": TRACE_DRAM_BYTES_PER_LAUNCH,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per trace launch of this "
                                        "workload (mean of the primary and incoherent launches)",
                      "peak_source": f"{peaks['source']} hbm_gbs (MEASURED_PEAKS.json)" if peaks["source"] == "measured"

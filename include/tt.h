@@ -205,9 +205,10 @@ void tt_dbvh_free(tt_dbvh *dbvh);
 #define TT_NUM_VARIANTS 8
 tt_status tt_dbvh_set_variant(tt_dbvh *bvh, int32_t variant);
 /* How many bytes of the node array's top levels the trace launches keep persisting in L2 (an
- * access-policy window over the start of the array, where tt_bvh_upload lays the tree's top
+ * access-policy window over the start of the four-wide nodes, where tt_bvh_upload lays the tree's top
  * levels out breadth first; the persisting set-aside is a limit of the calling process's
- * context). 0 = no window. No counterpart in the reference. */
+ * context). 0 = no window. Launches over the two-wide tree (variants 3 and 4, trees without a four-wide
+ * form) have none. No counterpart in the reference. */
 tt_status tt_dbvh_set_l2_window(tt_dbvh *bvh, int64_t bytes);
 tt_status tt_dbvh_get_variant(const tt_dbvh *bvh, int32_t *variant);
 /* Autotuner: traces the n device rays with every variant (the warp-vote one only when
@@ -228,9 +229,9 @@ tt_status tt_trace(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_hit *
 tt_status tt_trace_ext(const tt_dbvh *bvh, const tt_ray *d_rays, int64_t n, tt_hit_ext *d_hits,
                        int32_t closest, void *stream);
 /* as tt_trace with HOST buffers; synchronises the stream before returning. Page-locked, device-mapped
- * buffers (rays 16-byte, hits 8-byte aligned) are read and written by the trace itself across the
- * host link; others are copied through a device staging area owned by `bvh`. Returns the device
- * error word like tt_dbvh_check. */
+ * buffers (rays 16-byte, hits 8-byte aligned, not overlapping) are read and written by the trace itself
+ * across the host link; others are copied through a device staging area owned by `bvh`. Returns the
+ * device error word like tt_dbvh_check. */
 tt_status tt_trace_host(const tt_dbvh *bvh, const tt_ray *h_rays, int64_t n, tt_hit *h_hits,
                         int32_t closest, void *stream);
 /* Synchronises `stream`, then reads and clears the device error word that tt_trace /
@@ -404,8 +405,9 @@ typedef struct tt_launch_shape {
     int32_t block;        /* threads per block: 64, 128 or 256 */
     int32_t stack_shared; /* traversal stack entries per thread kept in shared memory: 0, 8 or 16 */
     int32_t wave_paths;   /* paths in flight per wave (queue capacity): 1 .. 2^26 */
-    int32_t ordered;      /* 1: order each extension queue by origin and direction cell before
-                             tracing it (coherent queues, e.g. camera rays, are left alone) */
+    int32_t ordered;      /* 1: order each extension and shadow queue of 2^22 rays or more by origin
+                             and direction cell before tracing it (coherent queues, e.g. camera
+                             rays, are left alone) */
     int32_t streamed;     /* 1: a render of more paths than one wave streams them through a pool
                              of wave_paths slots that is refilled with new camera paths as paths
                              end (no refill for cached renders, or when max_depth * wave_paths

@@ -19,8 +19,8 @@ using namespace pt;
 // 512 x 512 x 16 takes 3.39 ms with 8, 3.33 with 10, 3.30 with 12; 12 views of a terrain 2.59, 2.58 and 2.65.
 constexpr int kQueueInner = 10;
 
-// Compiled for 1,024 threads per SM (64 registers): with both loops in the kernel the compiler takes 70, and with
-// one block less the queues of the Cornell box take 4 % longer. A tree without a four-wide form goes through
+// Compiled for 1,024 threads per SM (64 registers): with both loops in the kernel the compiler takes 70, which
+// leaves one block less (the Cornell box 3.35 ms instead of 3.24 with another way to hold both loops). A tree without a four-wide form goes through
 // two_wide_queue: tracing each ray where trace_queue meets it, the box took 6.91 ms, so 5.35.
 // kPrefix: the ordering covers only the queue's first *n_sorted slots (a streamed render's
 // survivors); the rest is traced in place. Without it an ordered queue is ordered whole.

@@ -12,13 +12,14 @@
 // Kernels, in stream order: (1) clear the key counts and probe a 16th of the warps of rays (a
 // warp is uniform when its 32 keys are equal); when more than half of the sampled warps are
 // uniform the rays are already coherent and every later kernel returns at once, leaving the rays
-// in their own order. (2) Keys, and for each ray its rank among the rays of its key, from one
+// in their own order (two-wide when too many of them are such, order_two_wide). (2) Keys, and for each ray its rank among the rays of its key, from one
 // atomic per group of equal keys in a warp (__match_any_sync). (3) Exclusive scan of the counts in
 // 2048-entry chunks, chunk totals aside. (4) Every block scans the 1024 chunk totals in shared
 // memory; each ray's slot is chunk offset + count offset + rank, where the kernel writes the ray's
 // index; the trace kernel reads each ray, one 32-byte sector, through that index. Slots are
-// bounds-checked. The order inside a key is whatever the atomics give; only the grouping matters.
-// Plain launches on the caller's stream, so copies on other streams keep overlapping them.
+// bounds-checked where they are written and where they are read (ordered_slot). The order inside a key is
+// whatever the atomics give; only the grouping matters. Chained launches (tt_launch.cuh) on the caller's
+// stream; copies on other streams overlap them.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -19,16 +19,20 @@ constexpr int kOrderOriginBits = 13;
 constexpr int kOrderMinOriginBits = 6;
 constexpr int kOrderBits = kOrderDirBits + kOrderOriginBits;  // the largest key
 static_assert(kOrderDirBits % 2 == 0 && kOrderBits <= 21, "direction cells square; counts for 2^21 keys at most");
-// Fewer rays than this are traced in their own order: ordering them does not pay for its passes.
-// Measured on hashed cosine bounces and shadow rays, ordered against not, in us: on a
+// Fewer rays than this are traced in their own order. One line for closest and any hit, between the counts where
+// ordering starts to pay for either: at 1M it still costs cosine bounces up to 7 % or gains 3 %, and gains
+// shadow rays 3 to 8 %. Measured on hashed cosine bounces and shadow rays, ordered against not, in us: on a
 // 2,097,152-triangle terrain 287 / 269 at 1M, 451 / 457 at 2M, 790 / 835 at 4M (shadow rays 371 / 382
 // and 1,166 / 1,310 at 1M and 4M); on 400 spheres of 5,120 triangles 201 / 179 at 300K, 395 / 407 at 1M,
 // 1,215 / 1,398 at 4M (shadow rays 342 / 370 and 1,092 / 1,284).
 constexpr int64_t kOrderMinRays = 1 << 20;
 // The same for the queues of a render. They follow the image, so neighbours start close together
 // and go less far astray: with queues from 1M rays on ordered, 12 uneven views of a terrain (4M-slot
-// pool) take 3.35 ms, from 2M on 2.88, from 4M on 2.65; 960 x 540 x 16 samples of 400 spheres 15.5, 15.2
-// and 15.2 ms.
+// pool, whose queues never reach 4M) take 3.35 ms, from 2M on 2.88, with none 2.65; 960 x 540 x 16 samples of 400
+// spheres 15.5, 15.2 and 15.2 ms. Above the line it depends on the scene: in pools of 16M and 64M slots the
+// 8.2M-triangle multi-material view takes 164.8 and 163.7 ms unordered, 161.5 and 159.9 ordered, 16 views of
+// the terrain from 16M slots 32.7 unordered, 35.0 ordered. In a pool that cannot reach the line `ordered` only costs
+// its passes' launches (4M slots: 178.5 ms unordered, 185.0 ordered).
 constexpr int64_t kOrderMinQueue = 1 << 22;
 // Error-word bit: a slot of the order came out of range (see ordered_slot, and k_order_scatter).
 constexpr uint32_t kErrOrder = 4u;

@@ -464,7 +464,8 @@ __device__ __forceinline__ TraceResult wide_result(const WideState &s) {
     return res;
 }
 
-// One ray through the tree, start to finish, on the given stack.
+// One ray through the tree, start to finish, on the given stack: the steps without the queue, which the CPU tests compare
+// with the two-wide loop ray by ray (the kernels use trace_queue).
 template <bool kClosest, class Stack>
 __device__ __forceinline__ TraceResult traverse_wide(Stack &stack, const BvhView &bvh, float4 r0, float4 r1,
                                                      uint32_t &err) {
