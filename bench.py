@@ -63,16 +63,16 @@ METRIC = "Mrays/s closest-hit; time to relMSE 0.01, cached vs plain tracer, 1 GB
 UNIT = "Mrays/s"
 L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of the trace kernel of
-# this workload (the default, ray-ordered variant), the mean of a launch of 4M camera rays (318.2
-# MB) and one of 4M cosine rays (897.9 MB: rays read through an index, hits written to their own
+# this workload (the default, ray-ordered variant), the mean of a launch of 4M camera rays (317.1
+# MB) and one of 4M cosine rays (886.4 MB: rays read through an index, hits written to their own
 # places) that ncu captured on a GB300 on this terrain; the ordering kernels around them add 8 MB
 # (camera rays: the probe only) and 215 MB (probe, keys, scan, index). bench.py cannot run ncu itself.
-TRACE_DRAM_BYTES_PER_LAUNCH = 608_000_000
+TRACE_DRAM_BYTES_PER_LAUNCH = 602_000_000
 # L2 of the same GB300 from one ncu capture of an incoherent trace launch (1M rays): 132.0 sectors/ns
 # were 11.67 % of the sustained peak, i.e. 1,131 sectors/ns x 32 B (an earlier capture: 1,136, kept);
-# the launch's own L2 traffic was that 11.7 % of it
+# the launch's own L2 traffic is 11.2 % of it
 TRACE_L2_PEAK_GBS = 36_370.0
-TRACE_L2_TRAFFIC_PCT = 11.7
+TRACE_L2_TRAFFIC_PCT = 11.2
 
 
 def load_peaks() -> dict:
@@ -85,7 +85,7 @@ def load_peaks() -> dict:
 
 # the SIMD efficiency and the L2 figures of the trace kernel from the same committed ncu capture
 # (profiles/trace_kernel_terrain_closest.md, incoherent launch): threads per executed instruction
-TRACE_THREADS_PER_INST = 16.89
+TRACE_THREADS_PER_INST = 16.7
 
 
 def terrain_config(n_rays: int) -> dict:
@@ -462,7 +462,7 @@ def run_ours(args) -> None:
         "e2e": {"value": round(e2e_val, 2), "unit": UNIT, "h2d_bytes_per_step": int(n_rays * 32),
                 "d2h_bytes_per_step": int(n_rays * 8)},
         "roofline": {"binding": "latency and issue of divergent traversal: DRAM at 10 % of its peak, real L2 traffic "
-                                f"at {TRACE_L2_TRAFFIC_PCT} % of its peak, issue on 49 % of cycles with "
+                                f"at {TRACE_L2_TRAFFIC_PCT} % of its peak, issue on 53 % of cycles with "
                                 f"{TRACE_THREADS_PER_INST} of 32 lanes per instruction (ncu, incoherent launch)",
                      "l2": {"frac": round(achieved / TRACE_L2_PEAK_GBS, 4), "achieved": round(achieved, 1),
                             "peak": TRACE_L2_PEAK_GBS, "unit": "GB/s", "l2_traffic_pct_of_peak": TRACE_L2_TRAFFIC_PCT,
