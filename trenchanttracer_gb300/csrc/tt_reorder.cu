@@ -146,8 +146,8 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_probe(OrderArgs a) {
         if (atomicAdd(a.state + 2, 1ull) == (unsigned long long)gridDim.x - 1) {  // every block's counts are in
             const unsigned long long u = atomicAdd(a.state + 0, 0ull), f = atomicAdd(a.state + 1, 0ull);
             const unsigned long long w = atomicAdd(a.state + 4, 0ull);
-            // ordered unless mostly uniform
-            a.state[3] = (f > 0 && 2 * u <= f) ? 1ull : (64 * w > 32 * f ? 2ull : 0ull);
+            // ordered unless mostly uniform; two-wide from one such ray a warp on
+            a.state[3] = (f > 0 && 2 * u <= f) ? 1ull : (w > f ? 2ull : 0ull);
             a.state[4] = 0ull;
             a.state[0] = 0ull;
             a.state[1] = 0ull;

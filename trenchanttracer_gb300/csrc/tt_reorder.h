@@ -122,10 +122,12 @@ tt_status reorder_rays(const float4 *rays, int64_t n, const int *n_dev, const fl
 __device__ __forceinline__ bool order_built(const unsigned long long *state) { return state[3] == 1ull; }
 
 // Whether this call's rays are coherent and hold so many that the four-wide loop does not serve that the two-wide
-// one takes less for all: more than a 64th of the sampled ones. Each such ray holds up its warp while one lane
-// runs the two-wide loop. 4M camera rays on the 2,097,152-triangle terrain, two-wide 658 us: with none
-// such 489, a thousandth 503, a twentieth 815, half 1,203. Incoherent sets are faster four-wide whatever the share
-// (4M bounces, two-wide 1,165 us: 891 with a twentieth, 898 with half).
+// one takes less for all: more than one of a sampled warp's 32. Each such ray holds up its warp while one lane
+// runs the two-wide loop. 4M camera rays on the 2,097,152-triangle terrain, two-wide 660 us: with none
+// such 489, a hundredth 604, a fiftieth 670, a twentieth 814, half 1,203. On terrains, spheres and the Cornell box, 1M
+// and 4M camera rays, closest and any hit, two-wide takes 0.84 to 1.13 of the time with a fiftieth of them, 0.69
+// to 0.99 with a twentieth. Incoherent sets are faster four-wide whatever the share (4M bounces, two-wide
+// 1,165 us: 891 with a twentieth, 898 with half).
 __device__ __forceinline__ bool order_two_wide(const unsigned long long *state) { return state[3] == 2ull; }
 
 // The ray in a place of the order of rays 0 .. n - 1, for the kernels that take their rays through it. An order
